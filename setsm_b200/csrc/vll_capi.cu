@@ -88,7 +88,7 @@ struct vll_context {
     Buf img[VLL_MAX_IMAGES][6];
     Buf wgs, pts, gp3, ncc, vox, voxoff, gsum, gcnt;
     Buf ocd[VLL_MAX_IMAGES], ocdn[VLL_MAX_IMAGES], ocdptr;
-    Buf pre_tmp, pre_wt, pre_img, pre_mag, pre_ori;
+    Buf pre_tmp, pre_img, pre_mag, pre_ori;
     Buf sumcost;                       // SGM aggregation (float per voxel slot)
     Buf sgm_lr;                        // SGM: the 8 directions' costs per slot
     Buf tin_pts, tin_tris, tin_scratch;  // Ortho_blunder: points, triangles, work arrays
@@ -793,7 +793,6 @@ void vll_destroy(vll_context *ctx) {
     for (auto &b : ctx->ocdn) release(b);
     release(ctx->ocdptr);
     release(ctx->pre_tmp);
-    release(ctx->pre_wt);
     release(ctx->pre_img);
     release(ctx->pre_mag);
     release(ctx->pre_ori);
@@ -1986,13 +1985,10 @@ int vll_preprocess_level_device(vll_context *ctx, const uint16_t *d_image, uint3
     for (int r = -half + 1; r <= half - 1; ++r)
         for (int c = -half + 1; c <= half - 1; ++c)
             wt[(size_t)(half - 1 + r) * sz + (half - 1 + c)] = exp(-(double)(r * r + c * c) / 4.5);
-    VLL_CUDA(ctx, ensure(ctx->pre_wt, wt.size() * sizeof(double)));
-    VLL_CUDA(ctx, cudaMemcpyAsync(ctx->pre_wt.p, wt.data(), wt.size() * sizeof(double),
-                                  cudaMemcpyHostToDevice, ctx->stream));
     VLL_CUDA(ctx, vll::launch_sobel(d_image, width, height, d_mag, (uint8_t *)ctx->pre_tmp.p,
                                     ctx->stream));
     VLL_CUDA(ctx, vll::launch_orientation(d_mag, (const uint8_t *)ctx->pre_tmp.p, width, height,
-                                          half, (const double *)ctx->pre_wt.p, d_ori, ctx->stream));
+                                          wt.data(), d_ori, ctx->stream));
     VLL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return VLL_OK;
 }
@@ -2037,10 +2033,7 @@ int vll_pyramid_down_device(vll_context *ctx, const uint16_t *d_image, uint32_t 
             sum += val;
         }
     for (double &v : f) v /= sum;
-    VLL_CUDA(ctx, ensure(ctx->pre_wt, sizeof(f)));
-    VLL_CUDA(ctx, cudaMemcpyAsync(ctx->pre_wt.p, f, sizeof(f), cudaMemcpyHostToDevice, ctx->stream));
-    VLL_CUDA(ctx, vll::launch_pyramid(d_image, width, height, (const double *)ctx->pre_wt.p, d_out,
-                                      ctx->stream));
+    VLL_CUDA(ctx, vll::launch_pyramid(d_image, width, height, f, d_out, ctx->stream));
     VLL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return VLL_OK;
 }

@@ -157,8 +157,9 @@ cudaError_t run_ortho_blunder(const DevLevel *dP, const DevLevel &hP, double mpp
 // vll_preprocess.cu
 cudaError_t launch_sobel(const uint16_t *src, uint32_t w, uint32_t h, uint16_t *mag, uint8_t *bin,
                          cudaStream_t s);
+// wt: the 13x13 window weights, f: the 9x9 filter (host arrays, passed by value)
 cudaError_t launch_orientation(const uint16_t *mag, const uint8_t *bin, uint32_t w, uint32_t h,
-                               int half, const double *wt, uint8_t *ori, cudaStream_t s);
+                               const double *wt, uint8_t *ori, cudaStream_t s);
 cudaError_t launch_pyramid(const uint16_t *src, uint32_t w, uint32_t h, const double *f,
                            uint16_t *out, cudaStream_t s);
 
