@@ -11,20 +11,29 @@
 // the triangles depend on that exact order of decisions, and the list's
 // order on where each half-edge lives in memory (the edge allocator's stack,
 // split and merged with the recursion; a point's triangles are listed from
-// the edge of it stored last).  This file replays the same recursion level
-// by level: every node of a depth sorts its range at once (segmented radix
-// sort), then, deepest first, every node of a depth triangulates its base
-// case or merges its children in one thread, each on its own slice of the
-// shared half-edge pool and allocator stack.  Then one thread per point walks
-// its triangles in the reference's order.  Integer predicates are 64-bit with
-// the reference's wrap-around arithmetic.
+// the edge of it stored last).  This file replays the same recursion: both
+// sorted orders are made once and split down the tree by stable partitions
+// (no node is sorted again), every subtree of fewer than 100 points is
+// triangulated by one thread, and then, deepest first, every node of a depth
+// merges its halves in one thread, each on its own slice of the shared
+// half-edge pool and allocator stack.  Then one thread per point walks its
+// triangles in the reference's order.  The tree's shape follows from the
+// number of points alone, so the host only counts depths.  Integer predicates
+// are 64-bit with the reference's wrap-around arithmetic.
+//
+// What bounds it: the merges near the root, one thread each, a chain of some
+// hundred steps per cut (vll_tin_core.cuh).  Threads that walk alone have a
+// warp to themselves, so the warps' chains neither diverge nor share an L1
+// slice with 31 others.  224 k points of a 700 x 640 grid: 5.0 ms, of which
+// the merges are 4.1, the root's alone 1.4 (42.4 ms with a record per field,
+// 32 nodes to a warp, a segmented sort per depth and the tree on the host).
 #include <algorithm>
 #include <cstdio>
 #include <string>
 #include <vector>
+#include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_segmented_sort.cuh>
 
 #include "vll_internal.h"
 #include "vll_tin_core.cuh"
@@ -34,22 +43,33 @@ namespace {
 
 using namespace tin;
 
+// THREADED_CUTOFF (basic_topology_types.hpp:15): nodes below it recurse
+// serially on one edge list.
+constexpr int kThreadedCutoff = 100;
+// Nodes of at most this many points are partitioned down to the leaves by one
+// block in shared memory; larger ones a depth at a time over all points.
+constexpr int kBlockPoints = 1024;
+
 // ---------------------------------------------------------------------------
-// kernels
+// points and their two orders
 // ---------------------------------------------------------------------------
 // Grid coordinates of the points (SubFunctions.cpp:2793-2798: 0.5 plus the
-// offset in grid cells, truncated to int) and their grid index.
+// offset in grid cells, truncated to int), their grid index and the keys of
+// the orders (col, row) and (row, -col), non-negative in biased 32-bit halves.
 __global__ void tin_coords_kernel(const vll_point3 *__restrict__ pts, int n, double minx,
-                                  double miny, double res, int width, int *__restrict__ row,
-                                  int *__restrict__ col, unsigned long long *__restrict__ gkey,
-                                  int *__restrict__ ids) {
+                                  double miny, double res, int width, int2 *__restrict__ xy,
+                                  unsigned long long *__restrict__ gkey,
+                                  unsigned long long *__restrict__ kx,
+                                  unsigned long long *__restrict__ ky, int *__restrict__ ids) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int c = (int)(0.5 + __ddiv_rn(__dadd_rn(pts[i].x, -minx), res));
         const int r = (int)(0.5 + __ddiv_rn(__dadd_rn(pts[i].y, -miny), res));
-        col[i] = c;
-        row[i] = r;
+        xy[i] = make_int2(c, r);
         // grid index row * width + col, biased so that any int pair sorts
         gkey[i] = (unsigned long long)((long long)r * width + c + (1ll << 62));
+        const unsigned int br = (unsigned int)r ^ 0x80000000u, bc = (unsigned int)c ^ 0x80000000u;
+        kx[i] = ((unsigned long long)bc << 32) | br;
+        ky[i] = ((unsigned long long)br << 32) | (0xFFFFFFFFu - bc);
         ids[i] = i;
     }
 }
@@ -61,18 +81,127 @@ __global__ void tin_dup_kernel(const unsigned long long *__restrict__ sorted, in
         if (sorted[i] == sorted[i - 1]) atomicExch(err + 1, 1u);
 }
 
-// Sort keys of the positions inside this depth's ranges: (col, row) or
-// (row, -col), both non-negative in the biased 32-bit halves.
-__global__ void tin_keys_kernel(const int *__restrict__ perm, int n, int horiz,
-                                const int *__restrict__ row, const int *__restrict__ col,
-                                unsigned long long *__restrict__ keys) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int p = perm[i];
-        const unsigned int r = (unsigned int)row[p] ^ 0x80000000u;
-        const unsigned int c = (unsigned int)col[p] ^ 0x80000000u;
-        keys[i] = horiz ? (((unsigned long long)c << 32) | r)
-                        : (((unsigned long long)r << 32) | (0xFFFFFFFFu - c));
+// The depth-d node holding position i.
+__device__ __forceinline__ void node_at(int n, int d, int i, int &lo, int &cnt) {
+    lo = 0;
+    cnt = n;
+    for (int b = 0; b < d; ++b) {
+        const int mid = cnt / 2;
+        if (i < lo + mid) {
+            cnt = mid;
+        } else {
+            lo += mid;
+            cnt -= mid;
+        }
     }
+}
+
+// One depth: `a` is the order the depth's nodes are cut in.  Which half each
+// point falls in ...
+__global__ void tin_side_kernel(const int *__restrict__ a, int n, int d,
+                                unsigned char *__restrict__ left) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int lo, cnt;
+        node_at(n, d, i, lo, cnt);
+        left[a[i]] = i < lo + cnt / 2;
+    }
+}
+__global__ void tin_flag_kernel(const int *__restrict__ b, int n,
+                                const unsigned char *__restrict__ left, int *__restrict__ flag) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        flag[i] = left[b[i]];
+}
+// ... and the other order `b` stably split by it (sum: exclusive sums of the
+// left flags along b).
+__global__ void tin_split_kernel(const int *__restrict__ b, int n, int d,
+                                 const int *__restrict__ flag, const int *__restrict__ sum,
+                                 int *__restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int lo, cnt;
+        node_at(n, d, i, lo, cnt);
+        const int s = sum[i] - sum[lo];
+        out[flag[i] ? lo + s : lo + cnt / 2 + (i - lo - s)] = b[i];
+    }
+}
+
+// The same for all remaining depths of one node per block (at most
+// kBlockPoints points): px, py its points in both orders.  Writes the points'
+// coordinates in the order their leaves take them: the order their parent cut.
+__global__ void __launch_bounds__(256) tin_leaves_kernel(const int *__restrict__ px,
+                                                         const int *__restrict__ py, int n, int d0,
+                                                         int *__restrict__ inv,
+                                                         const int2 *__restrict__ xy,
+                                                         int2 *__restrict__ out) {
+    constexpr int kItems = kBlockPoints / 256;
+    typedef cub::BlockScan<int, 256> Scan;
+    __shared__ typename Scan::TempStorage scan_tmp;
+    __shared__ int gid[kBlockPoints];
+    __shared__ unsigned short order[2][kBlockPoints], next[kBlockPoints], leaf[kBlockPoints];
+    __shared__ unsigned short sum[kBlockPoints];
+    __shared__ unsigned char left[kBlockPoints];
+    int lo0, cnt0;
+    node_range(n, d0, blockIdx.x, lo0, cnt0);
+    // local ids: the position in the (col, row) order
+    for (int i = threadIdx.x; i < cnt0; i += 256) {
+        gid[i] = px[lo0 + i];
+        inv[gid[i]] = i;
+        order[0][i] = leaf[i] = (unsigned short)i;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt0; i += 256) order[1][i] = (unsigned short)inv[py[lo0 + i]];
+    __syncthreads();
+    int widest = cnt0;
+    for (int d = d0; widest >= 4; ++d, widest = (widest + 1) / 2) {
+        unsigned short *a = order[d & 1], *b = order[(d & 1) ^ 1];
+        for (int i = threadIdx.x; i < cnt0; i += 256) {
+            int lo = 0, cnt = cnt0;
+            for (int k = d0; k < d && cnt >= 4; ++k) {
+                const int mid = cnt / 2;
+                if (i < lo + mid) {
+                    cnt = mid;
+                } else {
+                    lo += mid;
+                    cnt -= mid;
+                }
+            }
+            if (cnt < 4) continue;   // a leaf of an earlier depth
+            leaf[i] = a[i];
+            left[a[i]] = i < lo + cnt / 2;
+        }
+        __syncthreads();
+        int f[kItems], s[kItems];
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int i = threadIdx.x * kItems + k;
+            f[k] = i < cnt0 ? left[b[i]] : 0;
+        }
+        Scan(scan_tmp).ExclusiveSum(f, s);
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) sum[threadIdx.x * kItems + k] = (unsigned short)s[k];
+        __syncthreads();
+        for (int i = threadIdx.x; i < cnt0; i += 256) {
+            int lo = 0, cnt = cnt0;
+            for (int k = d0; k < d && cnt >= 4; ++k) {
+                const int mid = cnt / 2;
+                if (i < lo + mid) {
+                    cnt = mid;
+                } else {
+                    lo += mid;
+                    cnt -= mid;
+                }
+            }
+            int to = i;
+            if (cnt >= 4) {
+                const int before = sum[i] - sum[lo];
+                to = left[b[i]] ? lo + before : lo + cnt / 2 + (i - lo - before);
+            }
+            next[to] = b[i];
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < cnt0; i += 256) b[i] = next[i];
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < cnt0; i += 256) out[lo0 + i] = xy[gid[leaf[i]]];
 }
 
 __global__ void tin_iota_kernel(int *__restrict__ a, long long n) {
@@ -81,85 +210,125 @@ __global__ void tin_iota_kernel(int *__restrict__ a, long long n) {
         a[i] = (int)i;
 }
 
-// One thread per subtree of fewer than 100 points, over its post-order list
-// (order[start[i] .. start[i + 1])).
-__global__ void tin_serial_kernel(TinGraph G, TinNode *nodes, const int *__restrict__ order,
-                                  const int *__restrict__ start, int m, const int *__restrict__ perm,
-                                  long long bound) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-        serial_subtree(G, nodes, order + start[i], start[i + 1] - start[i], perm, bound);
+// ---------------------------------------------------------------------------
+// triangulation
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ TinNode *node_of(TinNode *nodes, int d, unsigned j) {
+    return nodes + ((1ll << d) - 1 + j);
 }
 
-// EdgeList::MergeEdgeLists (edge_list.cpp:96-106): the right (top) child's
-// free stack moves down onto the left (bottom) child's.  One warp per node;
-// the destination precedes the source, so copying 32 entries at a time in
-// increasing order (each group read before written) is safe.
-__global__ void tin_concat_kernel(TinGraph G, const TinNode *nodes, const int *__restrict__ list,
-                                  int m) {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < m; w += warps) {
-        const TinNode &N = nodes[list[w]];
-        const TinNode &L = nodes[N.left];
-        const TinNode &R = nodes[N.right];
-        const int src = 6 * R.lo, dst = 6 * N.lo + L.idx;
-        for (int k0 = 0; k0 < R.idx; k0 += 32) {
-            const int k = k0 + lane;
-            int v = 0;
-            if (k < R.idx) v = G.unused[src + k];
-            __syncwarp();
-            if (k < R.idx) G.unused[dst + k] = v;
-            __syncwarp();
-        }
+// A warp per node of depth d that is the root of a subtree of fewer than 100
+// points (and not inside one): lane 0 triangulates it.
+__global__ void __launch_bounds__(32) tin_serial_kernel(TinGraph G, TinNode *nodes,
+                                                        const int2 *__restrict__ pts, int n, int d,
+                                                        long long bound) {
+    if (threadIdx.x != 0 || G.err[1]) return;
+    int lo, cnt;
+    if (d > 0) {
+        node_range(n, d - 1, blockIdx.x >> 1, lo, cnt);
+        if (cnt < kThreadedCutoff) return;
     }
+    node_range(n, d, blockIdx.x, lo, cnt);
+    if (cnt >= kThreadedCutoff) return;
+    Alloc a = alloc_at(G, 6 * lo, 6 * cnt);
+    TinNode *N = node_of(nodes, d, blockIdx.x);
+    N->ex = serial_subtree(G, pts, lo, cnt, (d & 1) == 0, a, bound);
+    N->idx = a.idx;
 }
 
-__global__ void tin_merge_kernel(TinGraph G, TinNode *nodes, const int *__restrict__ list, int m,
-                                 long long bound) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-        threaded_merge(G, nodes, list[i], bound);
+// A warp per node of depth d of 100 points or more
+// (TriangulateHorizontalThreaded / TriangulateVerticalThreaded): its halves
+// drew from split slices of its stack, which are concatenated
+// (EdgeList::MergeEdgeLists, edge_list.cpp:96-106: the right (top) child's
+// free stack moves down onto the left (bottom) child's; the destination
+// precedes the source, so copying 32 entries at a time in increasing order,
+// each group read before written, is safe); then lane 0 merges the halves.
+__global__ void __launch_bounds__(32) tin_merge_kernel(TinGraph G, TinNode *nodes, int n, int d,
+                                                       long long bound) {
+    if (G.err[1]) return;
+    int lo, cnt;
+    node_range(n, d, blockIdx.x, lo, cnt);
+    if (cnt < kThreadedCutoff) return;
+    const TinNode L = *node_of(nodes, d + 1, 2 * blockIdx.x);
+    const TinNode R = *node_of(nodes, d + 1, 2 * blockIdx.x + 1);
+    const int lane = threadIdx.x;
+    const int src = 6 * (lo + cnt / 2), dst = 6 * lo + L.idx;
+    for (int k0 = 0; k0 < R.idx; k0 += 32) {
+        const int k = k0 + lane;
+        int v = 0;
+        if (k < R.idx) v = G.unused[src + k];
+        __syncwarp();
+        if (k < R.idx) G.unused[dst + k] = v;
+        __syncwarp();
+    }
+    if (lane != 0) return;
+    Alloc a = alloc_at(G, 6 * lo, L.idx + R.idx);
+    TinNode *N = node_of(nodes, d, blockIdx.x);
+    N->ex = merge_halves(G, (d & 1) == 0, L.ex, R.ex, a, bound);
+    N->idx = a.idx;
+}
+
+// ---------------------------------------------------------------------------
+// the triangle list
+// ---------------------------------------------------------------------------
+// Free edges take dnext -1.
+__global__ void tin_free_kernel(TinGraph G, const TinNode *__restrict__ root) {
+    const int n = root->idx;
+    if (G.err[1]) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        G.edge[G.unused[i]].x = -1;
 }
 
 // EdgeList::SetGrid (basic_topology_types.hpp:157-202): a point keeps the
-// in-use edge out of it that is last in the pool.
-__global__ void tin_invalid_kernel(const int *__restrict__ unused, int n_free,
-                                   unsigned char *__restrict__ invalid) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_free; i += gridDim.x * blockDim.x)
-        invalid[unused[i]] = 1;
-}
-
-__global__ void tin_store_kernel(const int *__restrict__ orig, const unsigned char *__restrict__ invalid,
-                                 long long n_edges, int *__restrict__ stored) {
+// in-use edge out of it that is last in the pool.  The edges' points, as
+// positions in grid order, are found by their grid index.
+__global__ void tin_store_kernel(TinGraph G, const unsigned long long *__restrict__ gkey, int n,
+                                 int width, long long n_edges, int *__restrict__ pos,
+                                 int *__restrict__ stored) {
+    if (G.err[1]) return;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n_edges;
-         t += (long long)gridDim.x * blockDim.x)
-        if (!invalid[t]) atomicMax(stored + orig[t], (int)t);
+         t += (long long)gridDim.x * blockDim.x) {
+        const int4 E = G.edge[t];
+        if (E.x < 0) continue;
+        const unsigned long long key =
+            (unsigned long long)((long long)E.w * width + E.z + (1ll << 62));
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(gkey + mid) < key)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        pos[t] = lo;
+        atomicMax(stored + lo, (int)t);
+    }
 }
 
 // Grid::GetAllTris (grid.cpp:16-51): the points in grid order, each listing
 // the triangles around it (AdjTriIter, counter-clockwise from its stored
 // edge) of which it is the (col, row)-smallest vertex.  Pass 0 counts, pass 1
-// writes the vertices' input indices at the exclusive prefix `off`.
+// writes the vertices' input indices at the exclusive prefix `off` (off[n]:
+// the total; nothing is written when it exceeds cap or the input was refused).
 template <bool WRITE>
 __global__ void tin_tris_kernel(TinGraph G, const int *__restrict__ order, int n,
-                                const int *__restrict__ stored, long long *__restrict__ cnt,
-                                const long long *__restrict__ off, vll_tri *__restrict__ out,
-                                long long cap, long long bound) {
+                                const int *__restrict__ pos, const int *__restrict__ stored,
+                                long long *__restrict__ cnt, const long long *__restrict__ off,
+                                vll_tri *__restrict__ out, long long cap, long long bound) {
+    if (G.err[1] || (WRITE && (G.err[0] || off[n] > cap))) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int p = order[i];
         long long c = 0;
         long long o = WRITE ? off[i] : 0;
-        point_tris(G, stored[p], bound, [&](int q0, int q1, int q2) {
-            if (WRITE && o < cap) out[o] = vll_tri{(uint32_t)q0, (uint32_t)q1, (uint32_t)q2};
+        point_tris(G, stored[i], bound, [&](int e0, int e1, int e2) {
+            if (WRITE && o < cap)
+                out[o] = vll_tri{(uint32_t)order[pos[e0]], (uint32_t)order[pos[e1]],
+                                 (uint32_t)order[pos[e2]]};
             ++o;
             ++c;
         });
         if (!WRITE) cnt[i] = c;
     }
 }
-
-// THREADED_CUTOFF (basic_topology_types.hpp:15): nodes below it recurse
-// serially on one edge list.
-constexpr int kThreadedCutoff = 100;
 
 inline int grid1(long long n, int threads, int cap = 148 * 32) {
     const long long b = (n + threads - 1) / threads;
@@ -226,120 +395,51 @@ int run_tin_create(TinWork &w, const vll_point3 *d_pts, int64_t n64, const doubl
         *err = m;
         return VLL_ERR_INVALID;
     }
-    // ---- the recursion tree (it depends on n only) ----
-    std::vector<TinNode> nodes;
-    std::vector<int> depth;
-    nodes.reserve((size_t)n);
-    {
-        struct Item {
-            int lo, cnt, horiz, depth, parent, side;
-        };
-        std::vector<Item> stack{{0, n, 1, 0, -1, 0}};
-        while (!stack.empty()) {
-            const Item it = stack.back();
-            stack.pop_back();
-            const int id = (int)nodes.size();
-            TinNode N{};
-            N.lo = it.lo;
-            N.cnt = it.cnt;
-            N.left = N.right = -1;
-            N.horiz = it.horiz;
-            nodes.push_back(N);
-            depth.push_back(it.depth);
-            if (it.parent >= 0) (it.side ? nodes[it.parent].right : nodes[it.parent].left) = id;
-            if (it.cnt >= 4) {
-                const int mid = it.cnt / 2;
-                stack.push_back({it.lo + mid, it.cnt - mid, !it.horiz, it.depth + 1, id, 1});
-                stack.push_back({it.lo, mid, !it.horiz, it.depth + 1, id, 0});
-            }
-        }
-    }
-    const int n_nodes = (int)nodes.size();
-    const int max_depth = *std::max_element(depth.begin(), depth.end());
-    // per depth: the ranges sorted there (every internal node) and the
-    // merges of nodes of 100 points or more; and the post-order lists of the
-    // subtrees below 100 points, each triangulated by one thread
-    std::vector<std::vector<int>> inner(max_depth + 1), threaded(max_depth + 1);
-    std::vector<int> parent((size_t)n_nodes, -1);
-    for (int i = 0; i < n_nodes; ++i) {
-        if (nodes[i].left < 0) continue;
-        inner[depth[i]].push_back(i);
-        if (nodes[i].cnt >= kThreadedCutoff) threaded[depth[i]].push_back(i);
-        parent[nodes[i].left] = parent[nodes[i].right] = i;
-    }
-    std::vector<int> lists, serial_start{0};
-    std::vector<size_t> threaded_at(max_depth + 1);
-    for (int d = 0; d <= max_depth; ++d) {
-        threaded_at[d] = lists.size();
-        lists.insert(lists.end(), threaded[d].begin(), threaded[d].end());
-    }
-    const size_t serial_at = lists.size();
-    {
-        std::vector<std::pair<int, int>> stk;
-        for (int r = 0; r < n_nodes; ++r) {
-            if (nodes[r].cnt >= kThreadedCutoff) continue;
-            if (parent[r] >= 0 && nodes[parent[r]].cnt < kThreadedCutoff) continue;
-            stk.assign(1, {r, 0});
-            while (!stk.empty()) {
-                auto &t = stk.back();
-                const int v = t.first;
-                if (nodes[v].left < 0 || t.second == 2) {
-                    lists.push_back(v);
-                    stk.pop_back();
-                    continue;
-                }
-                const int c = t.second++ == 0 ? nodes[v].left : nodes[v].right;
-                stk.push_back({c, 0});
-            }
-            serial_start.push_back((int)(lists.size() - serial_at));
-        }
-    }
-    const int n_serial = (int)serial_start.size() - 1;
-    // begin / end of every depth's sorted ranges, uploaded once
-    std::vector<int> seg_begin, seg_end;
-    std::vector<size_t> seg_at(max_depth + 1);
-    for (int d = 0; d <= max_depth; ++d) {
-        seg_at[d] = seg_begin.size();
-        for (int id : inner[d]) {
-            seg_begin.push_back(nodes[id].lo);
-            seg_end.push_back(nodes[id].lo + nodes[id].cnt);
-        }
-    }
+    // ---- the recursion tree's depths (its nodes of a depth differ by one point) ----
+    auto smallest = [n](int d) { return n >> d; };
+    auto largest = [n](int d) { return (int)(((long long)n + (1ll << d) - 1) >> d); };
+    int d_block = 0;    // first depth whose nodes a block can partition
+    while (largest(d_block) > kBlockPoints) ++d_block;
+    int d_serial = 0;   // first depth with a node of fewer than 100 points
+    while (smallest(d_serial) >= kThreadedCutoff) ++d_serial;
+    // at that depth the larger nodes may still be of 100 points: their halves
+    // are then the subtrees
+    const bool mixed = largest(d_serial) >= kThreadedCutoff;
     // ---- device buffers ----
     const long long n_edges = 6ll * n;
-    int *row, *col, *ids, *ids_sorted, *perm, *perm2, *unused, *stored, *dlist, *sb, *se, *dstart;
-    int *dnext, *oprev, *twin, *orig;
-    unsigned long long *gkey, *gkey_sorted, *keys, *keys2;
+    int *ids, *ids_sorted, *px, *py, *p2, *flag, *sum, *inv, *unused, *stored, *pos;
+    unsigned long long *gkey, *gkey_sorted, *kx, *ky, *ktmp;
     unsigned int *flags;
-    unsigned char *invalid;
+    unsigned char *left;
     long long *tcnt, *toff;
-    TinNode *dnodes;
+    int2 *xy, *leaf_xy;
+    int4 *edge;
+    TinNode *nodes;
     size_t slot = 0;
-    TIN_CUDA(tin_buf(w, slot++, n, &row));
-    TIN_CUDA(tin_buf(w, slot++, n, &col));
     TIN_CUDA(tin_buf(w, slot++, n, &ids));
     TIN_CUDA(tin_buf(w, slot++, n, &ids_sorted));
-    TIN_CUDA(tin_buf(w, slot++, n, &perm));
-    TIN_CUDA(tin_buf(w, slot++, n, &perm2));
+    TIN_CUDA(tin_buf(w, slot++, n, &px));
+    TIN_CUDA(tin_buf(w, slot++, n, &py));
+    TIN_CUDA(tin_buf(w, slot++, n, &p2));
+    TIN_CUDA(tin_buf(w, slot++, n, &flag));
+    TIN_CUDA(tin_buf(w, slot++, n, &sum));
+    TIN_CUDA(tin_buf(w, slot++, n, &inv));
     TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &unused));
     TIN_CUDA(tin_buf(w, slot++, n, &stored));
-    TIN_CUDA(tin_buf(w, slot++, lists.size(), &dlist));
-    TIN_CUDA(tin_buf(w, slot++, serial_start.size(), &dstart));
-    TIN_CUDA(tin_buf(w, slot++, seg_begin.size(), &sb));
-    TIN_CUDA(tin_buf(w, slot++, seg_end.size(), &se));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &dnext));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &oprev));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &twin));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &orig));
+    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &pos));
+    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &edge));
     TIN_CUDA(tin_buf(w, slot++, n, &gkey));
     TIN_CUDA(tin_buf(w, slot++, n, &gkey_sorted));
-    TIN_CUDA(tin_buf(w, slot++, n, &keys));
-    TIN_CUDA(tin_buf(w, slot++, n, &keys2));
+    TIN_CUDA(tin_buf(w, slot++, n, &kx));
+    TIN_CUDA(tin_buf(w, slot++, n, &ky));
+    TIN_CUDA(tin_buf(w, slot++, n, &ktmp));
     TIN_CUDA(tin_buf(w, slot++, 4, &flags));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_edges, &invalid));
+    TIN_CUDA(tin_buf(w, slot++, n, &left));
     TIN_CUDA(tin_buf(w, slot++, (size_t)n + 1, &tcnt));
     TIN_CUDA(tin_buf(w, slot++, (size_t)n + 1, &toff));
-    TIN_CUDA(tin_buf(w, slot++, (size_t)n_nodes, &dnodes));
+    TIN_CUDA(tin_buf(w, slot++, n, &xy));
+    TIN_CUDA(tin_buf(w, slot++, n, &leaf_xy));
+    TIN_CUDA(tin_buf(w, slot++, (size_t)2 << (d_serial + 1), &nodes));
     // temporary storage of the library sorts and scans
     size_t tmp_bytes = 0, t1 = 0;
     TIN_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, gkey, gkey_sorted, ids, ids_sorted, n, 0,
@@ -347,29 +447,14 @@ int run_tin_create(TinWork &w, const vll_point3 *d_pts, int64_t n64, const doubl
     tmp_bytes = std::max(tmp_bytes, t1);
     TIN_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, tcnt, toff, n + 1, s));
     tmp_bytes = std::max(tmp_bytes, t1);
-    int max_segs = 1;
-    for (int d = 0; d <= max_depth; ++d) max_segs = std::max(max_segs, (int)inner[d].size());
-    TIN_CUDA(cub::DeviceSegmentedSort::SortPairs(nullptr, t1, keys, keys2, perm, perm2, n, max_segs,
-                                                 sb, se, s));
+    TIN_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, flag, sum, n, s));
     tmp_bytes = std::max(tmp_bytes, t1);
     void *tmp;
     TIN_CUDA(tin_buf(w, slot++, tmp_bytes, (unsigned char **)&tmp));
 
     TIN_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(unsigned int), s));
-    TIN_CUDA(cudaMemcpyAsync(dnodes, nodes.data(), nodes.size() * sizeof(TinNode),
-                             cudaMemcpyHostToDevice, s));
-    TIN_CUDA(cudaMemcpyAsync(dlist, lists.data(), lists.size() * sizeof(int),
-                             cudaMemcpyHostToDevice, s));
-    TIN_CUDA(cudaMemcpyAsync(dstart, serial_start.data(), serial_start.size() * sizeof(int),
-                             cudaMemcpyHostToDevice, s));
-    if (!seg_begin.empty()) {
-        TIN_CUDA(cudaMemcpyAsync(sb, seg_begin.data(), seg_begin.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice, s));
-        TIN_CUDA(cudaMemcpyAsync(se, seg_end.data(), seg_end.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice, s));
-    }
     tin_coords_kernel<<<grid1(n, 256), 256, 0, s>>>(d_pts, n, min_max[0], min_max[1], resolution,
-                                                    width, row, col, gkey, ids);
+                                                    width, xy, gkey, kx, ky, ids);
     TIN_CUDA(cudaGetLastError());
     // grid order of the points (GetAllTris walks it) and the distinctness check
     t1 = tmp_bytes;
@@ -377,56 +462,54 @@ int run_tin_create(TinWork &w, const vll_point3 *d_pts, int64_t n64, const doubl
                                              s));
     tin_dup_kernel<<<grid1(n, 256), 256, 0, s>>>(gkey_sorted, n, flags);
     TIN_CUDA(cudaGetLastError());
-    // ---- ranges sorted top-down, depth by depth ----
-    tin_iota_kernel<<<grid1(n, 256), 256, 0, s>>>(perm, n);
-    TIN_CUDA(cudaGetLastError());
-    for (int d = 0; d <= max_depth; ++d) {
-        if (inner[d].empty()) continue;
-        // positions outside this depth's ranges keep their place
-        TIN_CUDA(cudaMemcpyAsync(perm2, perm, (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, s));
-        tin_keys_kernel<<<grid1(n, 256), 256, 0, s>>>(perm, n, nodes[inner[d][0]].horiz, row, col,
-                                                      keys);
-        TIN_CUDA(cudaGetLastError());
+    // ---- both orders, split down the tree ----
+    t1 = tmp_bytes;
+    TIN_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t1, kx, ktmp, ids, px, n, 0, 64, s));
+    t1 = tmp_bytes;
+    TIN_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t1, ky, ktmp, ids, py, n, 0, 64, s));
+    for (int d = 0; d < d_block; ++d) {
+        const bool horiz = (d & 1) == 0;
+        const int *a = horiz ? px : py;
+        int *&b = horiz ? py : px;
+        tin_side_kernel<<<grid1(n, 256), 256, 0, s>>>(a, n, d, left);
+        tin_flag_kernel<<<grid1(n, 256), 256, 0, s>>>(b, n, left, flag);
         t1 = tmp_bytes;
-        TIN_CUDA(cub::DeviceSegmentedSort::SortPairs(tmp, t1, keys, keys2, perm, perm2, n,
-                                                     (int)inner[d].size(), sb + seg_at[d],
-                                                     se + seg_at[d], s));
-        std::swap(perm, perm2);
+        TIN_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t1, flag, sum, n, s));
+        tin_split_kernel<<<grid1(n, 256), 256, 0, s>>>(b, n, d, flag, sum, p2);
+        TIN_CUDA(cudaGetLastError());
+        std::swap(b, p2);
     }
+    tin_leaves_kernel<<<1u << d_block, 256, 0, s>>>(px, py, n, d_block, inv, xy, leaf_xy);
+    TIN_CUDA(cudaGetLastError());
     // ---- triangulation bottom-up ----
-    TinGraph G{dnext, oprev, twin, orig, row, col, unused, flags};
+    TinGraph G{edge, unused, flags};
     tin_iota_kernel<<<grid1(n_edges, 256), 256, 0, s>>>(unused, n_edges);
     TIN_CUDA(cudaGetLastError());
     const long long bound = 64ll * n + 1024;
-    tin_serial_kernel<<<grid1(n_serial, 32), 32, 0, s>>>(G, dnodes, dlist + serial_at, dstart,
-                                                         n_serial, perm, bound);
-    TIN_CUDA(cudaGetLastError());
-    for (int d = max_depth; d >= 0; --d) {
-        const int ni = (int)threaded[d].size();
-        if (!ni) continue;
-        tin_concat_kernel<<<grid1(32ll * ni, 128), 128, 0, s>>>(G, dnodes, dlist + threaded_at[d], ni);
+    for (int d = d_serial; d <= d_serial + (mixed ? 1 : 0); ++d) {
+        tin_serial_kernel<<<1u << d, 32, 0, s>>>(G, nodes, leaf_xy, n, d, bound);
         TIN_CUDA(cudaGetLastError());
-        tin_merge_kernel<<<grid1(ni, 32), 32, 0, s>>>(G, dnodes, dlist + threaded_at[d], ni, bound);
+    }
+    for (int d = d_serial - (mixed ? 0 : 1); d >= 0; --d) {
+        tin_merge_kernel<<<1u << d, 32, 0, s>>>(G, nodes, n, d, bound);
         TIN_CUDA(cudaGetLastError());
     }
     // ---- stored edge per point, then the triangle list ----
-    TinNode root;
-    TIN_CUDA(cudaMemcpyAsync(&root, dnodes, sizeof(TinNode), cudaMemcpyDeviceToHost, s));
-    TIN_CUDA(cudaStreamSynchronize(s));
-    TIN_CUDA(cudaMemsetAsync(invalid, 0, (size_t)n_edges, s));
     TIN_CUDA(cudaMemsetAsync(stored, 0xff, (size_t)n * sizeof(int), s));
-    if (root.idx > 0) {
-        tin_invalid_kernel<<<grid1(root.idx, 256), 256, 0, s>>>(unused, root.idx, invalid);
-        TIN_CUDA(cudaGetLastError());
-    }
-    tin_store_kernel<<<grid1(n_edges, 256), 256, 0, s>>>(orig, invalid, n_edges, stored);
+    tin_free_kernel<<<grid1(n, 256), 256, 0, s>>>(G, nodes);
     TIN_CUDA(cudaGetLastError());
-    tin_tris_kernel<false><<<grid1(n, 128), 128, 0, s>>>(G, ids_sorted, n, stored, tcnt, nullptr,
-                                                         nullptr, 0, bound);
+    tin_store_kernel<<<grid1(n_edges, 256), 256, 0, s>>>(G, gkey_sorted, n, width, n_edges, pos,
+                                                         stored);
     TIN_CUDA(cudaGetLastError());
-    TIN_CUDA(cudaMemsetAsync(tcnt + n, 0, sizeof(long long), s));
+    TIN_CUDA(cudaMemsetAsync(tcnt, 0, ((size_t)n + 1) * sizeof(long long), s));
+    tin_tris_kernel<false><<<grid1(n, 128), 128, 0, s>>>(G, ids_sorted, n, pos, stored, tcnt,
+                                                         nullptr, nullptr, 0, bound);
+    TIN_CUDA(cudaGetLastError());
     t1 = tmp_bytes;
     TIN_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t1, tcnt, toff, n + 1, s));
+    tin_tris_kernel<true><<<grid1(n, 128), 128, 0, s>>>(G, ids_sorted, n, pos, stored, nullptr,
+                                                        toff, d_tris, capacity, bound);
+    TIN_CUDA(cudaGetLastError());
     long long total = 0;
     unsigned int hflags[4];
     TIN_CUDA(cudaMemcpyAsync(&total, toff + n, sizeof(total), cudaMemcpyDeviceToHost, s));
@@ -444,15 +527,6 @@ int run_tin_create(TinWork &w, const vll_point3 *d_pts, int64_t n64, const doubl
     if (total > capacity) {
         *err = "triangle list longer than the output capacity";
         return VLL_ERR_CAPACITY;
-    }
-    tin_tris_kernel<true><<<grid1(n, 128), 128, 0, s>>>(G, ids_sorted, n, stored, nullptr, toff,
-                                                        d_tris, capacity, bound);
-    TIN_CUDA(cudaGetLastError());
-    TIN_CUDA(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
-    TIN_CUDA(cudaStreamSynchronize(s));
-    if (hflags[0]) {
-        *err = "triangulation walk exceeded its bound (malformed input)";
-        return VLL_ERR_INVALID;
     }
 #undef TIN_CUDA
     return VLL_OK;

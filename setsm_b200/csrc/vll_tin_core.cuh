@@ -1,389 +1,520 @@
 // vll_tin_core.cuh -- the triangulation steps of TINCreate_list
 // (grid_triangulation.cpp): half-edge pool, the reference's edge allocator,
-// integer predicates, base cases and the merge of two halves.  Compiled for
-// the device by vll_tin.cu; the functions are host-callable too, so the same
-// steps can run serially on the CPU.
+// integer predicates, base cases and the merge of two halves.
 #pragma once
 
 #include <cstdint>
-
-#ifdef __CUDACC__
-#define VLL_TIN_HD __host__ __device__
-#else
-#define VLL_TIN_HD
-#endif
+#include <cuda_runtime.h>
 
 namespace vll {
 namespace tin {
 
-// Half-edges (struct Edge, basic_topology_types.hpp:73-79) as arrays of
-// indices into the pool; orig is a point id (the points are distinct, so a
-// point's id stands for its grid coordinates).
+// Half-edges (struct Edge, basic_topology_types.hpp:73-79).  An edge is one
+// 16-byte record {dnext, oprev, origin column, origin row}: dnext is the next
+// edge out of the destination and oprev the previous edge into the origin,
+// both counter-clockwise.  The points are distinct, so coordinates stand for
+// the point, and a predicate needs no further access.  Edges are allocated
+// and freed in pairs from a stack that starts as 0, 1, 2, ..., so an edge's
+// twin is always e ^ 1 and the pair is one 32-byte sector: a merge, which is a
+// chain of dependent accesses by one thread, waits once per pair.
 struct TinGraph {
-    int *dnext;    // next edge out of the destination, counter-clockwise
-    int *oprev;    // previous edge into the origin, counter-clockwise
-    int *twin;
-    int *orig;
-    const int *row, *col;   // grid coordinates by point id
+    int4 *edge;
     int *unused;            // the allocator's stack of free edges
-    unsigned int *err;      // [0] set when a walk exceeds its bound
+    unsigned int *err;      // [0] set when a walk exceeds its bound, [1] equal points
 };
 
-// A node of the recursion: points [lo, lo + cnt) of the permutation.
+struct Pt {
+    int c, r;
+};
+__device__ __forceinline__ Pt pt_of(const int4 &e) { return Pt{e.z, e.w}; }
+__device__ __forceinline__ bool same(Pt a, Pt b) { return a.c == b.c && a.r == b.r; }
+
+__device__ __forceinline__ int4 rec(const TinGraph &G, int e) { return G.edge[e]; }
+__device__ __forceinline__ int dnext(const TinGraph &G, int e) { return G.edge[e].x; }
+__device__ __forceinline__ int oprev(const TinGraph &G, int e) { return G.edge[e].y; }
+__device__ __forceinline__ Pt orig(const TinGraph &G, int e) { return pt_of(G.edge[e]); }
+__device__ __forceinline__ Pt dest(const TinGraph &G, int e) { return pt_of(G.edge[e ^ 1]); }
+
+// A node's hull extremes: left ccw, right cw, bottom ccw, top cw.
+struct Ext {
+    int l, r, b, t;
+};
+// A node of 100 points or more, or the root of a smaller subtree.
 struct TinNode {
-    int lo, cnt;
-    int left, right;   // children (-1 for a base case of 2 or 3 points)
-    int horiz;         // sorted by (col, row) and cut into left / right halves
-    int idx;           // height of the node's free-edge stack (base 6 lo)
-    int ex[4];         // hull extremes: left ccw, right cw, bottom ccw, top cw
+    int idx;   // height of the node's free-edge stack (base 6 lo)
+    Ext ex;
 };
-enum { EX_L = 0, EX_R = 1, EX_B = 2, EX_T = 3 };
 
-VLL_TIN_HD inline bool less_xy(const TinGraph &G, int a, int b) {
-    const int ac = G.col[a], bc = G.col[b];
-    return ac < bc || (ac == bc && G.row[a] < G.row[b]);
+// Points [lo, lo + cnt) of node j at depth d (its path's bits, the topmost
+// first): every node is cut at half its points.
+__device__ __forceinline__ void node_range(int n, int d, unsigned j, int &lo, int &cnt) {
+    lo = 0;
+    cnt = n;
+    for (int b = d - 1; b >= 0; --b) {
+        const int mid = cnt / 2;
+        if ((j >> b) & 1u) {
+            lo += mid;
+            cnt -= mid;
+        } else {
+            cnt = mid;
+        }
+    }
 }
-VLL_TIN_HD inline bool less_yx(const TinGraph &G, int a, int b) {
-    const int ar = G.row[a], br = G.row[b];
-    return ar < br || (ar == br && G.col[a] > G.col[b]);
-}
+
+__device__ __forceinline__ bool less_xy(Pt a, Pt b) { return a.c < b.c || (a.c == b.c && a.r < b.r); }
+__device__ __forceinline__ bool less_yx(Pt a, Pt b) { return a.r < b.r || (a.r == b.r && a.c > b.c); }
 
 // Orientation / InCircle (grid_triangulation.cpp:29-61) in 64-bit integers;
 // the products wrap like the reference's (its 128-bit type is an alias of
-// int64_t), computed unsigned to keep the wrap-around defined.
-VLL_TIN_HD inline long long orient(const TinGraph &G, int a, int b, int c) {
-    const unsigned long long d11 = (unsigned long long)(long long)(G.col[a] - G.col[c]);
-    const unsigned long long d21 = (unsigned long long)(long long)(G.col[b] - G.col[c]);
-    const unsigned long long d12 = (unsigned long long)(long long)(G.row[a] - G.row[c]);
-    const unsigned long long d22 = (unsigned long long)(long long)(G.row[b] - G.row[c]);
-    return (long long)(d11 * d22 - d12 * d21);
+// int64_t), computed unsigned to keep the wrap-around defined.  Differences
+// within +-2^14 -- any grid up to 16384 cells a side -- need no wide
+// products: the same values from 32-bit terms and 32 x 32 -> 64 products.
+constexpr int kNear = 1 << 14;
+__device__ __forceinline__ bool near14(int d) { return (unsigned)(d + kNear) <= 2u * kNear; }
+
+__device__ __forceinline__ long long orient(Pt a, Pt b, Pt c) {
+    const int d11 = a.c - c.c, d21 = b.c - c.c, d12 = a.r - c.r, d22 = b.r - c.r;
+    if (near14(d11) && near14(d21) && near14(d12) && near14(d22))
+        return (long long)(d11 * d22 - d12 * d21);
+    typedef unsigned long long U;
+    return (long long)((U)(long long)d11 * (U)(long long)d22 -
+                       (U)(long long)d12 * (U)(long long)d21);
 }
 
-VLL_TIN_HD inline long long incircle(const TinGraph &G, int a, int b, int c, int d) {
-    const long long d11 = (long long)(G.col[a] - G.col[d]), d12 = (long long)(G.row[a] - G.row[d]);
-    const long long d21 = (long long)(G.col[b] - G.col[d]), d22 = (long long)(G.row[b] - G.row[d]);
-    const long long d31 = (long long)(G.col[c] - G.col[d]), d32 = (long long)(G.row[c] - G.row[d]);
+__device__ __forceinline__ long long incircle(Pt a, Pt b, Pt c, Pt d) {
+    const int d11 = a.c - d.c, d12 = a.r - d.r, d21 = b.c - d.c, d22 = b.r - d.r;
+    const int d31 = c.c - d.c, d32 = c.r - d.r;
+    if (near14(d11) && near14(d12) && near14(d21) && near14(d22) && near14(d31) && near14(d32)) {
+        const int s1 = d11 * d11 + d12 * d12, s2 = d21 * d21 + d22 * d22, s3 = d31 * d31 + d32 * d32;
+        const int bc = d21 * d32 - d31 * d22, ac = d11 * d32 - d31 * d12, ab = d11 * d22 - d21 * d12;
+        return (long long)s1 * bc - (long long)s2 * ac + (long long)s3 * ab;
+    }
     typedef unsigned long long U;
-    const U d13 = (U)d11 * (U)d11 + (U)d12 * (U)d12;
-    const U d23 = (U)d21 * (U)d21 + (U)d22 * (U)d22;
-    const U d33 = (U)d31 * (U)d31 + (U)d32 * (U)d32;
-    const U bc = (U)d21 * (U)d32 - (U)d31 * (U)d22;
-    const U ac = (U)d11 * (U)d32 - (U)d31 * (U)d12;
-    const U ab = (U)d11 * (U)d22 - (U)d21 * (U)d12;
-    return (long long)(d13 * bc - d23 * ac + d33 * ab);
+    const U e11 = (U)(long long)d11, e12 = (U)(long long)d12, e21 = (U)(long long)d21,
+            e22 = (U)(long long)d22, e31 = (U)(long long)d31, e32 = (U)(long long)d32;
+    const U s1 = e11 * e11 + e12 * e12, s2 = e21 * e21 + e22 * e22, s3 = e31 * e31 + e32 * e32;
+    const U bc = e21 * e32 - e31 * e22, ac = e11 * e32 - e31 * e12, ab = e11 * e22 - e21 * e12;
+    return (long long)(s1 * bc - s2 * ac + s3 * ab);
 }
 
 // The node's slice of the allocator (EdgeList::GetNewEdge / RemoveEdge,
 // edge_list.cpp:62-83): a stack of free edge indices at unused[base ...).
+// `top` is the stack's top entry, held ahead of its use.
 struct Alloc {
-    int base, idx;
+    int base, idx, top;
 };
-
-VLL_TIN_HD inline int new_edge(const TinGraph &G, Alloc &a) {
-    a.idx--;
-    return G.unused[a.base + a.idx];
+__device__ __forceinline__ Alloc alloc_at(const TinGraph &G, int base, int idx) {
+    return Alloc{base, idx, idx > 0 ? G.unused[base + idx - 1] : -1};
 }
-VLL_TIN_HD inline void free_edge(const TinGraph &G, Alloc &a, int e) {
+// The next pair of edges: the first popped is the new edge, its twin follows.
+// (A stack never runs out on distinct points; should it, the slice's first
+// pair is reused and the error flag raised.)
+__device__ __forceinline__ int new_pair(const TinGraph &G, Alloc &a) {
+    int e = a.top;
+    if (a.idx < 2) {
+        atomicExch(G.err, 1u);
+        a.idx = 2;
+        e = a.base;
+    }
+    a.idx -= 2;
+    a.top = a.idx > 0 ? G.unused[a.base + a.idx - 1] : -1;
+    return e;
+}
+__device__ __forceinline__ void free_pair(const TinGraph &G, Alloc &a, int e) {
     G.unused[a.base + a.idx] = e;
-    a.idx++;
+    G.unused[a.base + a.idx + 1] = e ^ 1;
+    a.idx += 2;
+    a.top = e ^ 1;
 }
 
-// AddEdgeAndTwin, RemoveEdgeAndTwin, Weld, Bridge (grid_triangulation.cpp:
-// 95-177), in the reference's statement order.
-VLL_TIN_HD inline int add_edge_twin(const TinGraph &G, Alloc &a, int o, int d) {
-    const int e = new_edge(G, a);
-    const int et = new_edge(G, a);
-    G.dnext[e] = et;
-    G.oprev[e] = et;
-    G.twin[e] = et;
-    G.dnext[et] = e;
-    G.oprev[et] = e;
-    G.twin[et] = e;
-    G.orig[e] = o;
-    G.orig[et] = d;
+// AddEdgeAndTwin, RemoveEdgeAndTwin, Bridge (grid_triangulation.cpp:95-177).
+__device__ __forceinline__ int add_edge_twin(const TinGraph &G, Alloc &a, Pt o, Pt d) {
+    const int e = new_pair(G, a), et = e ^ 1;
+    G.edge[e] = make_int4(et, et, o.c, o.r);
+    G.edge[et] = make_int4(e, e, d.c, d.r);
     return e;
 }
 
-VLL_TIN_HD inline void remove_edge_twin(const TinGraph &G, Alloc &a, int e) {
-    const int et = G.twin[e];
-    G.dnext[G.oprev[e]] = G.dnext[et];
-    G.oprev[G.dnext[e]] = G.oprev[et];
-    G.dnext[G.oprev[et]] = G.dnext[e];
-    G.oprev[G.dnext[et]] = G.oprev[e];
-    free_edge(G, a, e);
-    free_edge(G, a, et);
+__device__ __forceinline__ void remove_edge_twin(const TinGraph &G, Alloc &a, int e) {
+    const int4 E = rec(G, e), T = rec(G, e ^ 1);
+    G.edge[E.y].x = T.x;
+    G.edge[E.x].y = T.y;
+    G.edge[T.y].x = E.x;
+    G.edge[T.x].y = E.y;
+    free_pair(G, a, e);
 }
 
-VLL_TIN_HD inline void weld(const TinGraph &G, int in, int out) {
-    const int prev = G.oprev[out];
-    G.oprev[out] = in;
-    G.dnext[in] = out;
-    G.oprev[G.twin[in]] = prev;
-    G.dnext[prev] = G.twin[in];
+// Weld (grid_triangulation.cpp:127-140) of edge `in` before edge `out`.
+__device__ __forceinline__ void weld(const TinGraph &G, int in, int out) {
+    const int prev = oprev(G, out);
+    G.edge[out].y = in;
+    G.edge[in].x = out;
+    G.edge[in ^ 1].y = prev;
+    G.edge[prev].x = in ^ 1;
 }
 
-VLL_TIN_HD inline int bridge(const TinGraph &G, Alloc &a, int start, int end) {
-    const int o = G.orig[G.twin[start]];
-    const int d = G.orig[end];
-    const int e = add_edge_twin(G, a, o, d);
-    const int et = G.twin[e];
-    weld(G, et, G.dnext[start]);
+__device__ __forceinline__ int bridge(const TinGraph &G, Alloc &a, int start, int end) {
+    const int e = add_edge_twin(G, a, dest(G, start), orig(G, end));
+    weld(G, e ^ 1, dnext(G, start));
     weld(G, e, end);
     return e;
 }
 
 // Walks in this file stop after this many steps (a well-formed structure
 // never needs that many) and raise the error flag.
-VLL_TIN_HD inline bool step_ok(const TinGraph &G, long long &steps, long long bound) {
+__device__ __forceinline__ bool step_ok(const TinGraph &G, long long &steps, long long bound) {
     if (++steps <= bound) return true;
-#ifdef __CUDA_ARCH__
     atomicExch(G.err, 1u);
-#else
-    *G.err = 1u;
-#endif
     return false;
 }
 
-// NextCrossEdge (grid_triangulation.cpp:1287-1335): the next bridge of the
-// merge zipper above `base`, or -1 at the upper common tangent.
-VLL_TIN_HD inline int next_cross_edge(const TinGraph &G, Alloc &a, int base, long long &steps,
-                               long long bound) {
-    int l_cand = G.dnext[base];
-    const bool valid_l = orient(G, G.orig[base], G.orig[l_cand], G.orig[G.twin[l_cand]]) < 0;
-    if (valid_l) {
-        int next_cand = G.dnext[G.twin[l_cand]];
-        while (incircle(G, G.orig[l_cand], G.orig[base], G.orig[G.twin[l_cand]],
-                        G.orig[G.twin[next_cand]]) > 0) {
-            if (!step_ok(G, steps, bound)) return -1;
-            remove_edge_twin(G, a, l_cand);
-            l_cand = next_cand;
-            next_cand = G.dnext[G.twin[l_cand]];
+// One side's candidate of the merge zipper and what follows it: the edge and
+// its twin, the destination of the next edge around the candidate's origin
+// (the one whose circle test decides whether the candidate stays), and the
+// pair that becomes the candidate when the zipper advances on this side.
+struct Cand {
+    int e;
+    int4 a, b;      // records of e and e ^ 1
+    Pt next;        // destination of the next edge around the origin
+    int adv;        // the candidate after an advance on this side
+    int4 va, vb;    // its records
+};
+
+// kLeft: the next edge around the origin is dnext(twin), and the advance goes
+// to dnext; else they are twin(oprev) and twin(oprev(twin)).
+template <bool kLeft>
+__device__ __forceinline__ void cand_follow(const TinGraph &G, Cand &c) {
+    c.adv = kLeft ? c.a.x : (c.b.y ^ 1);
+    const int4 nx = rec(G, kLeft ? (c.b.x ^ 1) : c.a.y);
+    c.va = rec(G, c.adv);
+    c.vb = rec(G, c.adv ^ 1);
+    c.next = pt_of(nx);
+}
+template <bool kLeft>
+__device__ __forceinline__ void cand_load(const TinGraph &G, int e, Cand &c) {
+    c.e = e;
+    c.a = rec(G, e);
+    c.b = rec(G, e ^ 1);
+    cand_follow<kLeft>(G, c);
+}
+
+// The merge zipper (NextCrossEdge, grid_triangulation.cpp:1287-1335, from the
+// lower common tangent up): bridges from `base` until neither side has a
+// candidate above; returns the last bridge.  The reference's steps in its
+// order.  It is a chain of dependent accesses, so the base edge and both
+// candidates with what follows them stay in registers: an advance on one
+// side finds its candidate already loaded and waits only for the records
+// after it, and a bridge's stores are applied to the held records; where
+// they touch others than the usual ones, or an edge was removed, the records
+// are loaded again.
+__device__ int zipper(const TinGraph &G, Alloc &al, int base, long long &steps, long long bound) {
+    int4 Ba = rec(G, base), Bb = rec(G, base ^ 1);
+    Cand L, R;
+    cand_load<true>(G, Ba.x, L);
+    cand_load<false>(G, Ba.y ^ 1, R);
+    for (;;) {
+        if (!step_ok(G, steps, bound)) return base;
+        const Pt bo = pt_of(Ba), bd = pt_of(Bb);
+        const bool valid_l = orient(bo, pt_of(L.a), pt_of(L.b)) < 0;
+        bool removed = false;
+        if (valid_l && incircle(pt_of(L.a), bo, pt_of(L.b), L.next) > 0) {
+            removed = true;
+            int l = L.e, next = dnext(G, l ^ 1);
+            do {
+                if (!step_ok(G, steps, bound)) return base;
+                remove_edge_twin(G, al, l);
+                l = next;
+                next = dnext(G, l ^ 1);
+            } while (incircle(orig(G, l), bo, dest(G, l), dest(G, next)) > 0);
+            cand_load<false>(G, R.e, R);
+            L.e = l;
+        }
+        const bool valid_r = orient(bd, bo, pt_of(R.b)) > 0;
+        if (valid_r && incircle(bd, bo, pt_of(R.b), R.next) > 0) {
+            removed = true;
+            int r = R.e, next = oprev(G, r) ^ 1;
+            do {
+                if (!step_ok(G, steps, bound)) return base;
+                remove_edge_twin(G, al, r);
+                r = next;
+                next = oprev(G, r) ^ 1;
+            } while (incircle(bd, bo, dest(G, r), dest(G, next)) > 0);
+            R.e = r;
+        }
+        if (removed) {
+            Ba = rec(G, base);
+            Bb = rec(G, base ^ 1);
+            cand_load<true>(G, L.e, L);
+            cand_load<false>(G, R.e, R);
+        }
+        if (!valid_l && !valid_r) return base;
+        const int e = new_pair(G, al), et = e ^ 1;
+        if (!valid_l || (valid_r && incircle(pt_of(L.b), pt_of(L.a), pt_of(R.a), pt_of(R.b)) > 0)) {
+            // bridge(base, twin(r)): advance on the right
+            const int end = R.e ^ 1, X = L.e, prev = L.a.y;
+            const int prev2 = end == X ? et : R.b.y;
+            const Pt d = pt_of(R.b);
+            G.edge[e] = make_int4(end, prev, bd.c, bd.r);
+            G.edge[et] = make_int4(X, prev2, d.c, d.r);
+            G.edge[X].y = et;
+            G.edge[prev].x = e;
+            G.edge[end].y = e;
+            G.edge[prev2].x = et;
+            // (pairs of the stores against the pairs held: unusual)
+            const int pl = L.e >> 1, pa = L.adv >> 1, pr = R.adv >> 1;
+            const int s1 = prev >> 1, s2 = end >> 1, s3 = prev2 >> 1;
+            const bool odd = s1 == pl || s1 == pa || s1 == pr || s2 == pl || s2 == pa || s2 == pr ||
+                             s3 == pl || s3 == pa || pa == pl || prev2 == et;
+            base = et;
+            if (odd) {
+                Ba = rec(G, base);
+                Bb = rec(G, base ^ 1);
+                cand_load<true>(G, Ba.x, L);
+                cand_load<false>(G, Ba.y ^ 1, R);
+            } else {
+                Ba = make_int4(X, prev2, d.c, d.r);
+                Bb = make_int4(end, prev, bd.c, bd.r);
+                L.a.y = et;
+                R.e = R.adv;          // prev2 ^ 1
+                R.a = R.va;
+                R.b = R.vb;
+                R.b.x = et;
+                cand_follow<false>(G, R);
+            }
+        } else {
+            // bridge(l, base): advance on the left
+            const int end = base, X = L.a.x, prev = L.va.y;
+            const int prev2 = end == X ? et : Ba.y;
+            const Pt o = pt_of(L.b);
+            G.edge[e] = make_int4(end, prev, o.c, o.r);
+            G.edge[et] = make_int4(X, prev2, bo.c, bo.r);
+            G.edge[X].y = et;
+            G.edge[prev].x = e;
+            G.edge[end].y = e;
+            G.edge[prev2].x = et;
+            const int pa = L.adv >> 1, pr = R.e >> 1, pv = R.adv >> 1;
+            const int s1 = prev >> 1, s2 = end >> 1, s3 = prev2 >> 1;
+            const bool odd = s1 == pa || s1 == pr || s1 == pv || s2 == pa || s2 == pr || s2 == pv ||
+                             s3 == pa || s3 == pv || pa == pr || pa == pv || prev2 == et;
+            base = et;
+            if (odd) {
+                Ba = rec(G, base);
+                Bb = rec(G, base ^ 1);
+                cand_load<true>(G, Ba.x, L);
+                cand_load<false>(G, Ba.y ^ 1, R);
+            } else {
+                Ba = make_int4(X, prev2, bo.c, bo.r);
+                Bb = make_int4(end, prev, o.c, o.r);
+                R.b.x = et;           // prev2 is twin(r)
+                L.e = X;
+                L.a = L.va;
+                L.b = L.vb;
+                L.a.y = et;
+                cand_follow<true>(G, L);
+            }
         }
     }
-    int r_cand = G.twin[G.oprev[base]];
-    const bool valid_r = orient(G, G.orig[G.twin[base]], G.orig[base], G.orig[G.twin[r_cand]]) > 0;
-    if (valid_r) {
-        int next_cand = G.twin[G.oprev[r_cand]];
-        while (incircle(G, G.orig[G.twin[base]], G.orig[base], G.orig[G.twin[r_cand]],
-                        G.orig[G.twin[next_cand]]) > 0) {
-            if (!step_ok(G, steps, bound)) return -1;
-            remove_edge_twin(G, a, r_cand);
-            r_cand = next_cand;
-            next_cand = G.twin[G.oprev[r_cand]];
-        }
-    }
-    if (!valid_l && !valid_r) return -1;
-    if (!valid_l || (valid_r && incircle(G, G.orig[G.twin[l_cand]], G.orig[l_cand],
-                                         G.orig[r_cand], G.orig[G.twin[r_cand]]) > 0))
-        return G.twin[bridge(G, a, base, G.twin[r_cand])];
-    return G.twin[bridge(G, a, l_cand, base)];
 }
 
 // Triangulate2 / Triangulate3 (grid_triangulation.cpp:580-699) on the node's
 // points in the order its parent sorted them.
-VLL_TIN_HD inline void base_case(const TinGraph &G, TinNode &N, const int *perm, Alloc &a) {
-    if (N.cnt == 2) {
-        const int pa = perm[N.lo], pb = perm[N.lo + 1];
+__device__ inline Ext base_case(const TinGraph &G, const int2 *pts, int cnt, Alloc &a) {
+    Ext x;
+    if (cnt == 2) {
+        const Pt pa{pts[0].x, pts[0].y}, pb{pts[1].x, pts[1].y};
         const int e = add_edge_twin(G, a, pa, pb);
-        if (less_xy(G, pa, pb)) {
-            N.ex[EX_L] = e;
-            N.ex[EX_R] = G.twin[e];
-        } else {
-            N.ex[EX_L] = G.twin[e];
-            N.ex[EX_R] = e;
-        }
-        if (less_yx(G, pa, pb)) {
-            N.ex[EX_B] = e;
-            N.ex[EX_T] = G.twin[e];
-        } else {
-            N.ex[EX_B] = G.twin[e];
-            N.ex[EX_T] = e;
-        }
-        return;
+        const bool xy = less_xy(pa, pb), yx = less_yx(pa, pb);
+        x.l = xy ? e : e ^ 1;
+        x.r = xy ? e ^ 1 : e;
+        x.b = yx ? e : e ^ 1;
+        x.t = yx ? e ^ 1 : e;
+        return x;
     }
-    int p[3] = {perm[N.lo], perm[N.lo + 1], perm[N.lo + 2]};
-    // sort the three by (col, row)
-    for (int i = 1; i < 3; ++i)
-        for (int j = i; j > 0 && less_xy(G, p[j], p[j - 1]); --j) {
-            const int t = p[j];
-            p[j] = p[j - 1];
-            p[j - 1] = t;
+    Pt A{pts[0].x, pts[0].y}, B{pts[1].x, pts[1].y}, C{pts[2].x, pts[2].y};
+    auto order = [](Pt &p, Pt &q, bool swap) {
+        if (swap) {
+            const Pt t = p;
+            p = q;
+            q = t;
         }
-    int A = p[0], B = p[1], C = p[2];
+    };
+    // sort the three by (col, row)
+    order(A, B, less_xy(B, A));
+    order(B, C, less_xy(C, B));
+    order(A, B, less_xy(B, A));
     int e1 = add_edge_twin(G, a, A, B);
     int e2 = add_edge_twin(G, a, B, C);
     weld(G, e1, e2);
     int e3;
-    long long s = orient(G, A, B, C);
+    long long s = orient(A, B, C);
     if (s > 0) {
         e3 = bridge(G, a, e2, e1);
-        N.ex[EX_L] = e1;
-        N.ex[EX_R] = G.twin[e2];
+        x.l = e1;
+        x.r = e2 ^ 1;
     } else if (s < 0) {
         e3 = bridge(G, a, e2, e1);
-        N.ex[EX_L] = G.twin[e3];
-        N.ex[EX_R] = e3;
+        x.l = e3 ^ 1;
+        x.r = e3;
     } else {
-        N.ex[EX_L] = e1;
-        N.ex[EX_R] = G.twin[e2];
+        x.l = e1;
+        x.r = e2 ^ 1;
     }
     // the same three by (row, -col)
-    for (int i = 1; i < 3; ++i)
-        for (int j = i; j > 0 && less_yx(G, p[j], p[j - 1]); --j) {
-            const int t = p[j];
-            p[j] = p[j - 1];
-            p[j - 1] = t;
-        }
-    A = p[0];
-    B = p[1];
-    C = p[2];
-    const int e = (G.orig[e1] == A) ? e1 : (G.orig[e2] == A ? e2 : G.twin[e2]);
-    e1 = (G.orig[G.twin[e]] == B) ? e : G.dnext[G.twin[e]];
-    e2 = G.dnext[e1];
-    e3 = G.dnext[e2];
-    s = orient(G, A, B, C);
+    order(A, B, less_yx(B, A));
+    order(B, C, less_yx(C, B));
+    order(A, B, less_yx(B, A));
+    const int e = same(orig(G, e1), A) ? e1 : (same(orig(G, e2), A) ? e2 : e2 ^ 1);
+    e1 = same(dest(G, e), B) ? e : dnext(G, e ^ 1);
+    e2 = dnext(G, e1);
+    e3 = dnext(G, e2);
+    s = orient(A, B, C);
     if (s >= 0) {
-        N.ex[EX_B] = e1;
-        N.ex[EX_T] = G.twin[e2];
+        x.b = e1;
+        x.t = e2 ^ 1;
     } else {
-        N.ex[EX_B] = G.twin[e3];
-        N.ex[EX_T] = e3;
+        x.b = e3 ^ 1;
+        x.t = e3;
     }
+    return x;
 }
 
 // The merge of a node's two triangulated halves
 // (TriangulateHorizontalSerial / TriangulateVerticalSerial,
 // grid_triangulation.cpp:417-578): common tangent, zipper, new extremes.
-VLL_TIN_HD inline void merge_node(const TinGraph &G, TinNode *nodes, int ni, Alloc &a,
-                                  long long bound) {
-    TinNode &N = nodes[ni];
-    TinNode &L = nodes[N.left];
-    TinNode &R = nodes[N.right];
+__device__ inline Ext merge_halves(const TinGraph &G, bool horiz, Ext L, Ext R, Alloc &a,
+                                   long long bound) {
     long long steps = 0;
-    if (N.horiz) {
-        int le = L.ex[EX_R], re = R.ex[EX_L];
+    // the tangent walk from the facing extremes: p on the left (bottom) half,
+    // q on the right (top) one
+    int p = horiz ? L.r : L.t, q = horiz ? R.l : R.b;
+    {
+        int4 P = rec(G, p), Pt_ = rec(G, p ^ 1), Q = rec(G, q), Qt = rec(G, q ^ 1);
         for (;;) {
-            if (!step_ok(G, steps, bound)) return;
-            if (orient(G, G.orig[le], G.orig[G.twin[le]], G.orig[re]) > 0)
-                le = G.twin[G.oprev[G.twin[le]]];
-            else if (orient(G, G.orig[re], G.orig[G.twin[re]], G.orig[le]) < 0)
-                re = G.dnext[re];
-            else
+            if (!step_ok(G, steps, bound)) return L;
+            if (orient(pt_of(P), pt_of(Pt_), pt_of(Q)) > 0) {
+                p = Pt_.y ^ 1;       // twin(oprev(twin(p)))
+                P = rec(G, p);
+                Pt_ = rec(G, p ^ 1);
+            } else if (orient(pt_of(Q), pt_of(Qt), pt_of(P)) < 0) {
+                q = Q.x;             // dnext(q)
+                Q = rec(G, q);
+                Qt = rec(G, q ^ 1);
+            } else {
                 break;
+            }
         }
-        const int lct = bridge(G, a, G.oprev[re], G.dnext[G.twin[le]]);
-        if (G.orig[le] == G.orig[L.ex[EX_L]]) L.ex[EX_L] = G.twin[lct];
-        if (G.orig[re] == G.orig[R.ex[EX_R]]) R.ex[EX_R] = lct;
-        int nb = lct, uct = -1;
-        while (nb != -1) {
-            if (!step_ok(G, steps, bound)) return;
-            uct = nb;
-            nb = next_cross_edge(G, a, uct, steps, bound);
-        }
-        N.ex[EX_L] = L.ex[EX_L];
-        N.ex[EX_R] = R.ex[EX_R];
-        int t = G.twin[lct];
-        while (less_yx(G, G.orig[t], G.orig[G.twin[t]]) && step_ok(G, steps, bound)) t = G.oprev[t];
-        t = G.dnext[t];
-        while (less_yx(G, G.orig[G.twin[t]], G.orig[t]) && step_ok(G, steps, bound)) t = G.dnext[t];
-        N.ex[EX_B] = t;
-        t = G.twin[uct];
-        while (less_yx(G, G.orig[G.twin[t]], G.orig[t]) && step_ok(G, steps, bound))
-            t = G.twin[G.dnext[G.twin[t]]];
-        t = G.twin[G.oprev[G.twin[t]]];
-        while (less_yx(G, G.orig[t], G.orig[G.twin[t]]) && step_ok(G, steps, bound))
-            t = G.twin[G.oprev[G.twin[t]]];
-        N.ex[EX_T] = t;
-    } else {
-        int be = L.ex[EX_T], te = R.ex[EX_B];
-        for (;;) {
-            if (!step_ok(G, steps, bound)) return;
-            if (orient(G, G.orig[be], G.orig[G.twin[be]], G.orig[te]) > 0)
-                be = G.twin[G.oprev[G.twin[be]]];
-            else if (orient(G, G.orig[te], G.orig[G.twin[te]], G.orig[be]) < 0)
-                te = G.dnext[te];
-            else
-                break;
-        }
-        const int rct = bridge(G, a, G.oprev[te], G.dnext[G.twin[be]]);
-        if (G.orig[be] == G.orig[L.ex[EX_B]]) L.ex[EX_B] = G.twin[rct];
-        if (G.orig[te] == G.orig[R.ex[EX_T]]) R.ex[EX_T] = rct;
-        int nb = rct, lct = -1;
-        while (nb != -1) {
-            if (!step_ok(G, steps, bound)) return;
-            lct = nb;
-            nb = next_cross_edge(G, a, lct, steps, bound);
-        }
-        N.ex[EX_B] = L.ex[EX_B];
-        N.ex[EX_T] = R.ex[EX_T];
-        int t = rct;
-        while (less_xy(G, G.orig[G.twin[t]], G.orig[t]) && step_ok(G, steps, bound))
-            t = G.twin[G.dnext[G.twin[t]]];
-        t = G.twin[G.oprev[G.twin[t]]];
-        while (less_xy(G, G.orig[t], G.orig[G.twin[t]]) && step_ok(G, steps, bound))
-            t = G.twin[G.oprev[G.twin[t]]];
-        N.ex[EX_R] = t;
-        t = lct;
-        while (less_xy(G, G.orig[t], G.orig[G.twin[t]]) && step_ok(G, steps, bound)) t = G.oprev[t];
-        t = G.dnext[t];
-        while (less_xy(G, G.orig[G.twin[t]], G.orig[t]) && step_ok(G, steps, bound)) t = G.dnext[t];
-        N.ex[EX_L] = t;
     }
+    const int first = bridge(G, a, oprev(G, q), dnext(G, p ^ 1));
+    Ext x;
+    if (horiz) {
+        if (same(orig(G, p), orig(G, L.l))) L.l = first ^ 1;
+        if (same(orig(G, q), orig(G, R.r))) R.r = first;
+        const int last = zipper(G, a, first, steps, bound);
+        x.l = L.l;
+        x.r = R.r;
+        int t = first ^ 1;
+        while (less_yx(orig(G, t), dest(G, t)) && step_ok(G, steps, bound)) t = oprev(G, t);
+        t = dnext(G, t);
+        while (less_yx(dest(G, t), orig(G, t)) && step_ok(G, steps, bound)) t = dnext(G, t);
+        x.b = t;
+        t = last ^ 1;
+        while (less_yx(dest(G, t), orig(G, t)) && step_ok(G, steps, bound)) t = dnext(G, t ^ 1) ^ 1;
+        t = oprev(G, t ^ 1) ^ 1;
+        while (less_yx(orig(G, t), dest(G, t)) && step_ok(G, steps, bound)) t = oprev(G, t ^ 1) ^ 1;
+        x.t = t;
+    } else {
+        if (same(orig(G, p), orig(G, L.b))) L.b = first ^ 1;
+        if (same(orig(G, q), orig(G, R.t))) R.t = first;
+        const int last = zipper(G, a, first, steps, bound);
+        x.b = L.b;
+        x.t = R.t;
+        int t = first;
+        while (less_xy(dest(G, t), orig(G, t)) && step_ok(G, steps, bound)) t = dnext(G, t ^ 1) ^ 1;
+        t = oprev(G, t ^ 1) ^ 1;
+        while (less_xy(orig(G, t), dest(G, t)) && step_ok(G, steps, bound)) t = oprev(G, t ^ 1) ^ 1;
+        x.r = t;
+        t = last;
+        while (less_xy(orig(G, t), dest(G, t)) && step_ok(G, steps, bound)) t = oprev(G, t);
+        t = dnext(G, t);
+        while (less_xy(dest(G, t), orig(G, t)) && step_ok(G, steps, bound)) t = dnext(G, t);
+        x.l = t;
+    }
+    return x;
 }
 
 // A subtree of fewer than 100 points (TriangulateHorizontalSerial /
 // TriangulateVerticalSerial): the reference recurses without splitting its
 // edge list, so the whole subtree draws from one allocator stack, children
-// before parents, left before right.  `order` lists the subtree's nodes in
-// that post-order; the stack is the subtree root's slice, fresh.
-VLL_TIN_HD inline void serial_subtree(const TinGraph &G, TinNode *nodes, const int *order, int m,
-                                      const int *perm, long long bound) {
-    TinNode &root = nodes[order[m - 1]];
-    Alloc a{6 * root.lo, 6 * root.cnt};
-    for (int i = 0; i < m; ++i) {
-        TinNode &N = nodes[order[i]];
-        if (N.left < 0)
-            base_case(G, N, perm, a);
-        else
-            merge_node(G, nodes, order[i], a, bound);
+// before parents, left before right.
+__device__ inline Ext serial_subtree(const TinGraph &G, const int2 *pts, int lo, int cnt, bool horiz,
+                                     Alloc &a, long long bound) {
+    struct Frame {
+        int lo, cnt, state;
+        Ext left;
+    };
+    Frame f[8];   // 99 points: halved at most six times
+    int sp = 0;
+    f[0].lo = lo;
+    f[0].cnt = cnt;
+    f[0].state = 0;
+    Ext ret{0, 0, 0, 0};
+    while (sp >= 0) {
+        Frame &F = f[sp];
+        if (F.cnt < 4) {
+            ret = base_case(G, pts + F.lo, F.cnt, a);
+            --sp;
+            continue;
+        }
+        const int mid = F.cnt / 2;
+        if (F.state == 2) {
+            ret = merge_halves(G, horiz != (bool)(sp & 1), F.left, ret, a, bound);
+            --sp;
+            continue;
+        }
+        Frame &C = f[sp + 1];
+        C.state = 0;
+        if (F.state == 0) {
+            C.lo = F.lo;
+            C.cnt = mid;
+        } else {
+            F.left = ret;
+            C.lo = F.lo + mid;
+            C.cnt = F.cnt - mid;
+        }
+        ++F.state;
+        ++sp;
     }
-    root.idx = a.idx;
+    return ret;
 }
 
-// A node of 100 points or more (TriangulateHorizontalThreaded /
-// TriangulateVerticalThreaded): its halves drew from split slices of its
-// stack, which are concatenated (EdgeList::MergeEdgeLists) before the merge.
-VLL_TIN_HD inline void threaded_merge(const TinGraph &G, TinNode *nodes, int ni, long long bound) {
-    TinNode &N = nodes[ni];
-    Alloc a{6 * N.lo, nodes[N.left].idx + nodes[N.right].idx};
-    merge_node(G, nodes, ni, a, bound);
-    N.idx = a.idx;
-}
-
-// The triangles around point p (Grid::GetAllTris, grid.cpp:16-51, and
+// The triangles around a point (Grid::GetAllTris, grid.cpp:16-51, and
 // AdjTriIter, grid_iterators.hpp:63-110): counter-clockwise from the first
-// face that is a triangle at or after its stored edge `e`, those of which p
-// is the (col, row)-smallest vertex, passed to emit(q0, q1, q2).  Points of
-// degree <= 2 whose edges are collinear have none.
+// face that is a triangle at or after its stored edge `e`, those of which it
+// is the (col, row)-smallest vertex, passed to emit(e0, e1, e2), the edges out
+// of its vertices.  Points of degree <= 2 whose edges are collinear have none.
 template <class Emit>
-VLL_TIN_HD inline void point_tris(const TinGraph &G, int e, long long bound, Emit emit) {
+__device__ inline void point_tris(const TinGraph &G, int e, long long bound, Emit emit) {
     if (e < 0) return;
-    const int f = G.dnext[G.twin[G.dnext[G.twin[e]]]];
-    const int p1 = G.orig[e], p2 = G.orig[G.twin[e]], p3 = G.orig[G.twin[G.dnext[G.twin[e]]]];
-    const bool collinear = (G.col[p1] - G.col[p2]) * (G.row[p1] - G.row[p3]) ==
-                           (G.row[p1] - G.row[p2]) * (G.col[p1] - G.col[p3]);
+    const int g = dnext(G, e ^ 1);
+    const int f = dnext(G, g ^ 1);
+    const Pt p1 = orig(G, e), p2 = dest(G, e), p3 = dest(G, g);
+    const bool collinear = (p1.c - p2.c) * (p1.r - p3.r) == (p1.r - p2.r) * (p1.c - p3.c);
     if (f == e && collinear) return;
     long long steps = 0;
     int start = e;
-    while (G.dnext[G.dnext[G.dnext[start]]] != start && step_ok(G, steps, bound))
-        start = G.dnext[G.twin[start]];
+    while (dnext(G, dnext(G, dnext(G, start))) != start && step_ok(G, steps, bound))
+        start = dnext(G, start ^ 1);
     int cur = start;
     do {
-        const int q0 = G.orig[cur], q1 = G.orig[G.dnext[cur]], q2 = G.orig[G.dnext[G.dnext[cur]]];
-        if (less_xy(G, q0, q1) && less_xy(G, q0, q2)) emit(q0, q1, q2);
-        cur = G.dnext[G.twin[cur]];
-        while (G.dnext[G.dnext[G.dnext[cur]]] != cur && step_ok(G, steps, bound))
-            cur = G.dnext[G.twin[cur]];
+        const int4 E0 = rec(G, cur);
+        const int e1 = E0.x;
+        const int4 E1 = rec(G, e1);
+        const int e2 = E1.x;
+        const Pt q0 = pt_of(E0), q1 = pt_of(E1), q2 = orig(G, e2);
+        if (less_xy(q0, q1) && less_xy(q0, q2)) emit(cur, e1, e2);
+        cur = dnext(G, cur ^ 1);
+        while (dnext(G, dnext(G, dnext(G, cur))) != cur && step_ok(G, steps, bound))
+            cur = dnext(G, cur ^ 1);
     } while (cur != start && step_ok(G, steps, bound));
 }
 
