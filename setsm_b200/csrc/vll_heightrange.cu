@@ -11,6 +11,7 @@
 // is set by the first triangle that contains it; here one warp per triangle
 // marks, per node, the smallest containing triangle index (atomicMin), and a
 // pass over the nodes then applies that triangle's update -- the same result.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -132,8 +133,32 @@ __device__ __forceinline__ double node_y(const DevLevel &P, int64_t row) {
     return __dadd_rn(__dmul_rn((double)row, P.grid_res), P.boundary[1]);
 }
 
-// Per triangle (one warp): the running extent of the vertex heights and,
-// per node of its box inside it, the smallest containing triangle index.
+// Boxes of more cells than this are swept by the whole warp, 32 cells at a
+// time; a smaller one by its triangle's own lane.  A TIN of most grid nodes
+// has boxes of 9 to 16 cells, which leave most of a warp idle.
+constexpr int64_t kLaneBox = 48;
+
+// Marks the box cells of triangle t inside it, from cell `first` on, every
+// `step`-th, with the smallest triangle index.
+__device__ __forceinline__ void cover_cells(const DevLevel &P, const Tri3 &T, const BBox &b,
+                                            unsigned int t, int64_t first, int64_t step,
+                                            unsigned int *winner) {
+    const int ncol = b.x1 - b.x0 + 1;
+    const int64_t ncell = (int64_t)ncol * (b.y1 - b.y0 + 1);
+    for (int64_t i = first; i < ncell; i += step) {
+        const int r = ncell < (1 << 30) ? (int)i / ncol : (int)(i / ncol);
+        const int64_t row = b.y0 + r, col = b.x0 + (i - (int64_t)r * ncol);
+        float z;
+        if (tin_inside(T, node_x(P, col), node_y(P, row), z))
+            atomicMin(winner + row * P.grid_w + col, t);
+    }
+}
+
+// The extent of the triangles' vertex heights and, per node inside a
+// triangle, the smallest containing triangle index.  A triangle per lane;
+// the extent is reduced per warp before its two atomics (one pair per
+// triangle, all on the same words, took 0.78 of the kernel's 0.87 ms for the
+// 650 k triangles of a 600 x 600 grid, which now takes 0.12).
 __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__ Pp,
                                                     const vll_point3 *pts, int64_t n_pts,
                                                     const vll_tri *tris, int64_t n_tris,
@@ -143,24 +168,48 @@ __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t t = warp; t < n_tris; t += n_warps) {
-        const vll_tri tr = tris[t];
-        if (!(tr.a < n_pts && tr.b < n_pts && tr.c < n_pts)) continue;
-        const Tri3 T = tri_of(pts, tr);
-        if (lane == 0) {
-            atomicMin(zext, dkey(dmin(dmin(T.z[0], T.z[1]), T.z[2])));
-            atomicMax(zext + 1, dkey(dmax(dmax(T.z[0], T.z[1]), T.z[2])));
+    unsigned long long zmin = ~0ull, zmax = 0;
+    bool any = false;
+    for (int64_t t0 = warp * 32; t0 < n_tris; t0 += n_warps * 32) {
+        const int64_t t = t0 + lane;
+        Tri3 T;
+        BBox b{0, 0, -1, -1};
+        if (t < n_tris) {
+            const vll_tri tr = tris[t];
+            if (tr.a < n_pts && tr.b < n_pts && tr.c < n_pts) {
+                T = tri_of(pts, tr);
+                const unsigned long long lo = dkey(dmin(dmin(T.z[0], T.z[1]), T.z[2]));
+                const unsigned long long hi = dkey(dmax(dmax(T.z[0], T.z[1]), T.z[2]));
+                zmin = lo < zmin ? lo : zmin;
+                zmax = hi > zmax ? hi : zmax;
+                any = true;
+                b = tin_box(P, T);
+            }
         }
-        const BBox b = tin_box(P, T);
-        if (b.x1 < b.x0 || b.y1 < b.y0) continue;
-        const int64_t ncol = b.x1 - b.x0 + 1;
-        const int64_t ncell = ncol * (b.y1 - b.y0 + 1);
-        for (int64_t i = lane; i < ncell; i += 32) {
-            const int64_t row = b.y0 + i / ncol, col = b.x0 + i % ncol;
-            float z;
-            if (tin_inside(T, node_x(P, col), node_y(P, row), z))
-                atomicMin(winner + row * P.grid_w + col, (unsigned int)t);
+        const bool box = b.x1 >= b.x0 && b.y1 >= b.y0;
+        const bool large =
+            box && (int64_t)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1) > kLaneBox;
+        if (box && !large) cover_cells(P, T, b, (unsigned int)t, 0, 1, winner);
+        unsigned m = __ballot_sync(0xffffffffu, large);
+        while (m) {
+            // the warp sweeps lane l's box
+            const int l = __ffs(m) - 1;
+            m &= m - 1;
+            const vll_tri tr = tris[t0 + l];
+            const Tri3 U = tri_of(pts, tr);
+            const BBox c = tin_box(P, U);
+            cover_cells(P, U, c, (unsigned int)(t0 + l), lane, 32, winner);
         }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long lo = __shfl_xor_sync(0xffffffffu, zmin, o);
+        const unsigned long long hi = __shfl_xor_sync(0xffffffffu, zmax, o);
+        zmin = lo < zmin ? lo : zmin;
+        zmax = hi > zmax ? hi : zmax;
+    }
+    if (__any_sync(0xffffffffu, any) && lane == 0) {
+        atomicMin(zext, zmin);
+        atomicMax(zext + 1, zmax);
     }
 }
 
@@ -431,8 +480,9 @@ cudaError_t run_height_range(const DevLevel *dP, const DevLevel &hP, const vll_p
     if ((e = cudaMemsetAsync(out, 0, N * sizeof(vll_ugrid), s))) return e;
     const RangeArgs a{buffer, th_hg, iteration};
     if (n_tris > 0)
-        cover_kernel<<<blocks_for(n_tris * 32, 128), 128, 0, s>>>(dP, pts, n_pts, tris, n_tris,
-                                                                 winner, zkey);
+        // (few enough warps that their extent atomics do not count)
+        cover_kernel<<<std::min(blocks_for(n_tris, 128), 148u * 16u), 128, 0, s>>>(
+            dP, pts, n_pts, tris, n_tris, winner, zkey);
     zext_kernel<<<1, 1, 0, s>>>(zkey, zext);
     node_update_kernel<<<blocks_for(N, 128), 128, 0, s>>>(dP, pts, tris, winner, gp3, newh, mb, a);
     snapshot_kernel<<<blocks_for(N, 256), 256, 0, s>>>(gp3, newh, snap, N);
