@@ -677,13 +677,19 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
     const int64_t oh = (int64_t)((P.boundary[3] - P.boundary[1]) / im_res) + 1;
     if (ow <= 0 || oh <= 0) return fail(ctx, VLL_ERR_INVALID, "empty orthoimage boundary");
     const size_t total = (size_t)(ow * oh);
+    // a raster of samples per target image, or (large windows) of coordinates
+    // per image
+    const bool sampled = vll::ortho_sampled(H);
     double2 *ptrs[2 * VLL_MAX_IMAGES] = {};
-    for (int ti = 0; ti < P.num_images; ++ti) {
+    for (int ti = sampled ? 1 : 0; ti < P.num_images; ++ti) {
         if (!P.im[ti].selected) continue;
-        VLL_CUDA(ctx, ensure(ctx->ocd[ti], total * sizeof(double2)));
-        VLL_CUDA(ctx, cudaMemsetAsync(ctx->ocd[ti].p, 0, total * sizeof(double2), ctx->stream));
+        const size_t bytes = sampled ? vll::ortho_sample_bytes((int64_t)total) : total * sizeof(double2);
+        VLL_CUDA(ctx, ensure(ctx->ocd[ti], bytes));
+        if (!sampled) VLL_CUDA(ctx, cudaMemsetAsync(ctx->ocd[ti].p, 0, bytes, ctx->stream));
         ptrs[ti] = (double2 *)ctx->ocd[ti].p;
     }
+    if (sampled)
+        VLL_CUDA(ctx, ensure(ctx->tin_scratch, vll::ortho_sampled_scratch(P.n_nodes)));
     P.gp3 = d_gp3;
     int rc = upload_level_block(ctx, P);
     if (rc) return rc;
@@ -697,15 +703,23 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
         VLL_CUDA(ctx, cudaEventCreate(&ctx->e1));
     }
     VLL_CUDA(ctx, cudaEventRecord(ctx->e0, ctx->stream));
-    VLL_CUDA(ctx, vll::launch_ortho_raster(dP, dptr, ow, oh, im_res, use_b ? 1 : 0, ctx->stream));
-    if (d_ncc)
-        VLL_CUDA(ctx, vll::launch_blunder(dP, P.n_nodes, dptr, ow, oh, im_res, H, d_gp3, d_ncc,
-                                          ctx->stream));
-    else
-        VLL_CUDA(ctx, vll::launch_seeddem(dP, P.n_nodes, dptr, ow, oh, im_res, H, use_b ? 1 : 0,
-                                          d_gp3, ctx->stream));
+    if (sampled) {
+        VLL_CUDA(ctx, vll::launch_ortho_sampled(dP, P, P.n_nodes, (void *const *)ptrs,
+                                                (void *const *)dptr, ow, oh, im_res, H,
+                                                use_b ? 1 : 0, d_gp3, d_ncc, ctx->tin_scratch.p,
+                                                ctx->stream));
+    } else {
+        VLL_CUDA(ctx, vll::launch_ortho_raster(dP, dptr, ow, oh, im_res, use_b ? 1 : 0,
+                                               ctx->stream));
+        if (d_ncc)
+            VLL_CUDA(ctx, vll::launch_blunder(dP, P.n_nodes, dptr, ow, oh, im_res, H, d_gp3, d_ncc,
+                                              ctx->stream));
+        else
+            VLL_CUDA(ctx, vll::launch_seeddem(dP, P.n_nodes, dptr, ow, oh, im_res, H,
+                                              use_b ? 1 : 0, d_gp3, ctx->stream));
+    }
     VLL_CUDA(ctx, cudaEventRecord(ctx->e1, ctx->stream));
-    ctx->launches_total += 2;
+    ctx->launches_total += sampled ? 4 : 2;
     if (stats) {
         VLL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         float ms = 0;
