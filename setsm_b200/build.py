@@ -37,6 +37,7 @@ SOURCES = {
     "vll_tinblunder.cu": ["-fmad=false"],
     "vll_tin.cu": ["-fmad=false"],
     "vll_split.cu": [],
+    "vll_combined.cu": [],
     "vll_capi.cu": [],
     "vll_shim.cu": [],
 }

@@ -35,10 +35,9 @@
 #include <cub/device/device_scan.cuh>
 #include <cuda.h>
 
-#include "vll_exact.cuh"
 #include "vll_internal.h"
 #include "vll_split.h"
-#include "vll_window.cuh"
+#include "vll_stream.cuh"
 
 namespace vll {
 
@@ -51,46 +50,6 @@ inline cudaError_t scan64(void *tmp, size_t &bytes, const int32_t *in, int64_t *
     return cub::DeviceScan::ExclusiveScan(tmp, bytes, in, out, cub::Sum(), (int64_t)0, n, s);
 }
 
-
-// Half-width of the FP32 error band of rho: decisions whose FP32 inputs lie
-// closer than this to their boundary are settled in FP64.  The FP32-vs-FP64
-// error of rho measured over 4.2 M slots of 7x7 and 11x11 windows stays below
-// 6.8e-7 (tests/test_gpu_accuracy.py asserts < kBand / 2), a margin of ~3x.
-constexpr float kBand = 4e-6f;
-constexpr double kEdge = 1e-7;          // coordinate distance to an integer / clamp
-constexpr int kSlotCap = 512;           // slots per node the peak kernel holds in shared memory
-constexpr int kWarpPerSlotMax = 8;      // re-checks per round done a warp per slot (more: a lane each)
-constexpr int kMaxRounds = 3;           // scan / re-check rounds before a full FP64 pass
-
-// Per-slot markers in the rho buffer (.x):
-constexpr float kNotEvaluated = INFINITY;    // slot skipped (range / image bounds)
-constexpr float kRejected = -INFINITY;       // orientation check failed
-
-// ---------------------------------------------------------------------------
-// Level set: the levels matched by one pass of the pipeline (one level for a
-// VerticalLineLocus call; many tiles and pyramid levels for a batch).  Their
-// nodes are numbered consecutively: global node g belongs to the level l with
-// base[l] <= g < base[l + 1] and is that level's node g - base[l].  Per-node
-// and per-slot work arrays are indexed by g.
-// ---------------------------------------------------------------------------
-struct LevelSet {
-    const DevLevel *lv;       // [n] level blocks (device)
-    const int64_t *base;      // [n + 1] first global node of each level (device)
-    int n;
-    int64_t total;            // base[n]
-};
-
-__device__ __forceinline__ int level_of(const LevelSet &S, int64_t g) {
-    int lo = 0, hi = S.n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(S.base + mid) <= g)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
 
 // ---------------------------------------------------------------------------
 // prep: per-node setup (setsm_code.cpp:6158-6328)
@@ -150,82 +109,6 @@ __global__ void __launch_bounds__(256) prep_kernel(const LevelSet S,
 }
 
 // ---------------------------------------------------------------------------
-// geometry helpers of the window kernel
-// ---------------------------------------------------------------------------
-// Per-node RPC: normalised L, P (with the reference's +-360 wrap) and the
-// four cubics in the normalised height.  RPC00B terms grouped by power of H:
-//   a0: 1 L P LP LL PP LLL LPP LLP PPP   a1: H LH PH PLH LLH PPH
-//   a2: HH LHH PHH                        a3: HHH
-// Coefficients a0..a3 of one of the four RPC cubics (j: LINE_NUM, LINE_DEN,
-// SAMP_NUM, SAMP_DEN) as a polynomial in the normalised height, for fixed
-// normalised L, P (with the reference's +-360 wrap).
-__device__ __forceinline__ void node_horner_poly(const double *rpc, double lon, double lat, int j,
-                                                 double *a) {
-    double L = (lon - rpc[2]) / rpc[7];
-    double P = (lat - rpc[3]) / rpc[8];
-    if (L < -10.0 || L > 10.0) {
-        const double X = lon > 0 ? lon - 360 : lon + 360;
-        L = (X - rpc[2]) / rpc[7];
-    }
-    if (P < -10.0 || P > 10.0) {
-        const double Y = lat > 0 ? lat - 360 : lat + 360;
-        P = (Y - rpc[3]) / rpc[8];
-    }
-    const double *c = rpc + 10 + 20 * j;
-    a[0] = c[0] + c[1] * L + c[2] * P + c[4] * L * P + c[7] * L * L + c[8] * P * P +
-           c[11] * L * L * L + c[12] * L * P * P + c[14] * L * L * P + c[15] * P * P * P;
-    a[1] = c[3] + c[5] * L + c[6] * P + c[10] * P * L + c[17] * L * L + c[18] * P * P;
-    a[2] = c[9] + c[13] * L + c[16] * P;
-    a[3] = c[19];
-}
-
-// Reciprocal for the fast geometry path: FP32 seed refined by two Newton
-// steps (relative error ~1e-16).  A seed that is not a finite non-zero float
-// sends the slot to the exact projection.
-__device__ __forceinline__ double fast_rcp(double v, bool &edge) {
-    const float f = __frcp_rn((float)v);
-    if (!(fabsf(f) > 0.f && fabsf(f) < 3.0e38f)) edge = true;
-    double r = (double)f;
-    r = fma(r, fma(-v, r, 1.0), r);
-    r = fma(r, fma(-v, r, 1.0), r);
-    return r;
-}
-
-// Image coordinate (pyramid level) of one slot from the per-node cubics.
-// Sets `edge` when a coordinate is too close to an integer, or to a clamp,
-// for the Horner rounding to be trusted with the reference's integer tests.
-__device__ __forceinline__ double2 fast_coord(const double (*a)[4], const double *hn,
-                                              const DevImage &im, double hgt, double inv_s,
-                                              bool &edge) {
-    const double H = (hgt - hn[0]) * hn[1];   // hn[1]: reciprocal of the height scale
-    double v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = fma(fma(fma(a[j][3], H, a[j][2]), H, a[j][1]), H, a[j][0]);
-    double y = im.adj[0] + ((v[0] * fast_rcp(v[1], edge)) * im.rpc[5] + im.rpc[0]);
-    double x = im.adj[1] + ((v[2] * fast_rcp(v[3], edge)) * im.rpc[6] + im.rpc[1]);
-    const double ymax = im.rpc[0] + im.rpc[5] * 1.2, xmax = im.rpc[1] + im.rpc[6] * 1.2;
-    if (fabs(y) < kEdge || fabs(y - ymax) < kEdge || fabs(x) < kEdge || fabs(x - xmax) < kEdge)
-        edge = true;
-    y = y < 0 ? 0 : (y > ymax ? ymax : y);
-    x = x < 0 ? 0 : (x > xmax ? xmax : x);
-    const double px = x * inv_s - im.sx, py = y * inv_s - im.sy;   // inv_s = 2^-L (exact)
-    const double fx = px - floor(px), fy = py - floor(py);
-    if (fx < kEdge || fx > 1.0 - kEdge || fy < kEdge || fy > 1.0 - kEdge) edge = true;
-    return make_double2(px, py);
-}
-
-__device__ __forceinline__ bool near_round(double v) {
-    const double x = v * 1000.0;
-    return fabs(x - floor(x) - 0.5) < (double)kBand * 1000.0;
-}
-__device__ __forceinline__ bool near_trunc(double v) {
-    const double x = v * 1000.0;
-    return fabs(x - rint(x)) < (double)kBand * 1000.0;
-}
-
-
-
-// ---------------------------------------------------------------------------
 // FindPeakNcc decisions over the slots of one node, lane-parallel (shared by
 // the window kernel's FP32 pass and the exact pass)
 // ---------------------------------------------------------------------------
@@ -241,16 +124,6 @@ __device__ __forceinline__ int dir_sign(double a, double b) {
     else
         d = -1;
     return d > 0 ? 1 : (d < 0 ? -1 : 0);
-}
-
-__device__ __forceinline__ bool bit(const uint32_t *m, int k) { return (m[k >> 5] >> (k & 31)) & 1u; }
-__device__ __forceinline__ void set_bit(uint32_t *m, int k) { atomicOr(&m[k >> 5], 1u << (k & 31)); }
-
-// Index of the last evaluated slot before k (or -1); `carry` is the last
-// evaluated slot of earlier 32-slot groups.
-__device__ __forceinline__ int prev_eval(uint32_t mask, int lane, int carry) {
-    const uint32_t below = mask & ((1u << lane) - 1u);
-    return below ? (31 - __clz(below)) : carry;
 }
 
 // Bit masks over the slots of one node (kSlotCap at most), in shared memory.
@@ -465,28 +338,6 @@ __device__ void node_exact_chunked(const DevLevel &P, int64_t pt, int K, const P
 // ---------------------------------------------------------------------------
 // window kernel
 // ---------------------------------------------------------------------------
-// Warps per window block and the minimum resident blocks per SM (the latter
-// sets the register budget: 65536 / (warps * 32 * blocks)).
-#ifndef VLL_WIN_WARPS
-#define VLL_WIN_WARPS 4
-#endif
-#ifndef VLL_WIN_MINB
-#define VLL_WIN_MINB 3
-#endif
-constexpr int kWinWarps = VLL_WIN_WARPS;
-constexpr int kWinMaxBlocksPerSm = 2048 / (kWinWarps * 32);
-constexpr int kZeroCap = 32;          // zero intensity texels listed per staged group
-
-// Node flags of the window kernel
-constexpr uint32_t kNfCmr = 1u;       // memory-tight route (FindPeakNcc on the values)
-constexpr uint32_t kNfOri = 2u;       // orientation-difference test (level >= 3)
-constexpr uint32_t kNfVox = 4u;       // voxel rows written
-constexpr uint32_t kNfChc = 8u;       // check_height_change (max_WNCC written)
-constexpr uint32_t kNfGncc = 16u;     // rho blends the INCC with the node's GNCC
-constexpr uint32_t kNfVec = 32u;      // image rows 16-byte aligned (vector staging)
-constexpr uint32_t kNfTma = 64u;      // the level has tensor maps for its footprints
-constexpr uint32_t kNfDbg = 128u;     // per-slot debug values written
-
 // Optional instrumentation of the window kernel's phases (compiled with
 // -DVLL_PHASE_CYCLES: `python -m setsm_b200.build --phase-cycles` builds
 // lib/libsetsm_vll_phases.so).  Each warp sums clock64 deltas per phase
@@ -520,259 +371,6 @@ __device__ unsigned long long g_phase_cycles[16];
 #define PHASE_COUNT(i) (void)0
 #define PHASE_FLUSH() (void)0
 #endif
-
-// Per-node state of the window kernel in shared memory: the RPC cubics, the
-// level constants the slot loop reads (here rather than from the level block
-// in global memory), the record folded by lane 0 and the streamed scan's
-// carry.  A warp holds two: the node of the group being evaluated and the
-// node of the group being fetched.
-struct NodeCtx {
-    double horner[2][4][4];           // [image][num/den poly][a0..a3]
-    double hnorm[2][2];               // [image] {h_off, 1 / h_scale}
-    double geo[2][8];                 // [image] adj0, adj1, rpc0, rpc1, rpc5, rpc6, sx, sy
-    double inv_s, hbase, hstep, bin_angle, alpha, gterm;
-    const uint16_t *img[2], *mag[2];
-    const uint8_t *ori[2];
-    const DevLevel *P;
-    vll_voxel *vrow;
-    int64_t gn, pt;
-    uint32_t w[2], h[2];
-    int tma_w[2], tma_h[2];
-    int K, H, start_H, end_H;
-    uint32_t flags;
-    vll_nccresult R;
-    float pre_v;                      // streamed scan: the last evaluated slot's value,
-    int pre_dir, pre_k, have;         // direction and index, and whether there is one
-};
-
-// The constants of the launch's first level, loaded once per block: node
-// set-ups on that level (every node of a single-level call) read them from
-// shared memory and fetch only the node's own records from global memory.
-struct LevelConst {
-    double rpc[2][90];                // [image] RPC00B block (offsets, scales, 4 x 20 terms)
-    double geo[2][8];                 // as NodeCtx::geo
-    double inv_s, hstep, bin_angle, alpha, beta;
-    const uint16_t *img[2], *mag[2];
-    const uint8_t *ori[2];
-    uint32_t w[2], h[2];
-    int tma_w[2], tma_h[2];
-    int H, is_ra, cmr, check_ortho, voxels;
-    uint32_t flags;                   // kNfOri | kNfVec | kNfTma | kNfDbg
-};
-
-// Per-warp shared state of the window kernel.
-struct WinShared {
-    NodeCtx node[2];
-    uint32_t zl[kZeroCap];            // zero intensity texels of the staged boxes
-    int zn;                           // their count (more than kZeroCap: not listed)
-    uint64_t mbar;                    // completion of the group's tile copies
-    const DevLevel *tmap_level;       // level whose tensor maps lane 0 has acquired
-};
-
-__host__ __device__ constexpr size_t win_level_offset() {
-    return (sizeof(WinShared) * kWinWarps + 15) & ~(size_t)15;
-}
-
-__host__ __device__ constexpr size_t win_boxes_offset() {
-    return (win_level_offset() + sizeof(LevelConst) + 15) & ~(size_t)15;
-}
-
-// Fills the block's LevelConst from level P (every thread of the block takes
-// part; the caller synchronises the block afterwards).
-__device__ void level_const_load(LevelConst &C, const DevLevel &P) {
-    const int t = threadIdx.x, nt = blockDim.x;
-    for (int i = t; i < 180; i += nt) {
-        const int im = i / 90;
-        C.rpc[im][i - im * 90] = P.im[im == 0 ? P.ref : 1].rpc[i - im * 90];
-    }
-    if (t < 2) {
-        const DevImage &I = P.im[t == 0 ? P.ref : 1];
-        double *g = C.geo[t];
-        g[0] = I.adj[0];
-        g[1] = I.adj[1];
-        g[2] = I.rpc[0];
-        g[3] = I.rpc[1];
-        g[4] = I.rpc[5];
-        g[5] = I.rpc[6];
-        g[6] = I.sx;
-        g[7] = I.sy;
-        C.img[t] = I.img;
-        C.mag[t] = I.mag;
-        C.ori[t] = I.ori;
-        C.w[t] = I.w;
-        C.h[t] = I.h;
-        C.tma_w[t] = P.tma_w[t];
-        C.tma_h[t] = P.tma_h[t];
-    } else if (t == 2) {
-        const DevImage &ri = P.im[P.ref], &tI = P.im[1];
-        C.inv_s = 1.0 / (double)(1 << P.L);
-        C.hstep = P.height_step;
-        C.bin_angle = P.bin_angle;
-        C.alpha = P.alpha;
-        C.beta = P.beta;
-        C.H = P.H;
-        C.is_ra = P.is_ra;
-        C.cmr = P.cmr;
-        C.check_ortho = P.check_ortho;
-        C.voxels = P.vox && !P.cmr && !P.is_ra;
-        const bool vec_ok = (ri.w % 8 == 0) && (tI.w % 8 == 0) &&
-                            ((reinterpret_cast<uintptr_t>(ri.img) | reinterpret_cast<uintptr_t>(ri.mag) |
-                              reinterpret_cast<uintptr_t>(tI.img) |
-                              reinterpret_cast<uintptr_t>(tI.mag)) & 15) == 0;
-        C.flags = ((!P.is_ra && P.L >= 3) ? kNfOri : 0u) | (vec_ok ? kNfVec : 0u) |
-                  (P.tma_w[0] > 0 ? kNfTma : 0u) | (P.dbg_rho ? kNfDbg : 0u);
-    }
-}
-
-// the TMA tiles follow the boxes, 128-byte aligned (warp_raw is a multiple of 128)
-__host__ __device__ constexpr size_t win_raw_offset(int warp_quads) {
-    return (win_boxes_offset() + (size_t)kWinWarps * warp_quads * 16 + 127) & ~(size_t)127;
-}
-
-// FP32 window statistics of one slot for the level's window half-size
-// (the window code is unrolled per half-size; a batch may mix them).
-__device__ __forceinline__ void window_any(int H, const float4 *qr, int rbw, float rfx, float rfy,
-                                           const TgtBox &tb, float tfx, float tfy, float c,
-                                           float s, float &incc, bool &unsure) {
-    switch (H) {
-        case 2: window_fp32<2>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 3: window_fp32<3>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 4: window_fp32<4>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 5: window_fp32<5>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 6: window_fp32<6>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        default: window_fp32<7>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-    }
-}
-
-// Fills the warp's node context for global node gn (level lvl, K slots);
-// every lane takes part, the context is complete after the final __syncwarp.
-__device__ __noinline__ void node_setup(NodeCtx &N, const LevelSet &LS, int lvl, int64_t gn, int K,
-                                        const double *__restrict__ gsum,
-                                        const double *__restrict__ gcnt,
-                                        const LevelConst *lc, int lane) {
-    const DevLevel &P = LS.lv[lvl];
-    const int64_t pt = gn - __ldg(LS.base + lvl);
-    if (lc) {
-        // the level's constants from the block's copy; the node's own
-        // records from global memory, one load per lane
-        if (lane < 8) {
-            const int im = lane >> 2, j = lane & 3;
-            const double *rpc = lc->rpc[im];
-            node_horner_poly(rpc, P.grid_wgs[2 * pt], P.grid_wgs[2 * pt + 1], j, N.horner[im][j]);
-            if (j == 0) {
-                N.hnorm[im][0] = rpc[4];
-                N.hnorm[im][1] = 1.0 / rpc[9];
-            }
-        } else if (lane < 26) {
-            const int i = lane - 8;   // 16 geo values, then 2 lanes of pointers
-            if (i < 16) {
-                N.geo[i >> 3][i & 7] = lc->geo[i >> 3][i & 7];
-            } else {
-                const int im = i - 16;
-                N.img[im] = lc->img[im];
-                N.mag[im] = lc->mag[im];
-                N.ori[im] = lc->ori[im];
-                N.w[im] = lc->w[im];
-                N.h[im] = lc->h[im];
-                N.tma_w[im] = lc->tma_w[im];
-                N.tma_h[im] = lc->tma_h[im];
-            }
-        } else if (lane == 26) {
-            const vll_ugrid g = P.gp3[pt];
-            const vll_nccresult R = P.ncc[pt];
-            const double cnt_g = gcnt ? gcnt[gn] : 0.0;
-            const double sum_g = gcnt ? gsum[gn] : 0.0;
-            N.P = &P;
-            N.gn = gn;
-            N.pt = pt;
-            N.K = K;
-            N.H = lc->H;
-            N.start_H = g.minHeight;
-            N.end_H = g.maxHeight;
-            N.R = R;
-            N.hbase = (double)((lc->is_ra || lc->cmr) ? g.minHeight : R.minHeight);
-            N.hstep = lc->hstep;
-            N.inv_s = lc->inv_s;
-            N.bin_angle = lc->bin_angle;
-            N.alpha = lc->alpha;
-            const bool gncc = lc->check_ortho && cnt_g > 0;
-            N.gterm = gncc ? (sum_g / cnt_g) * lc->beta : 0.0;
-            N.vrow = lc->voxels ? P.vox + P.vox_off[pt] : nullptr;
-            N.flags = lc->flags | (lc->cmr ? kNfCmr : 0u) | (lc->voxels ? kNfVox : 0u) |
-                      (R.check_height_change ? kNfChc : 0u) | (gncc ? kNfGncc : 0u);
-            N.pre_v = -1.0f;
-            N.pre_dir = 0;
-            N.pre_k = -1;
-            N.have = 0;
-        }
-        __syncwarp();
-        return;
-    }
-    if (lane < 8) {
-        // per-node RPC cubics: lanes 0..7 = (image, polynomial)
-        const int im = lane >> 2, j = lane & 3;
-        const double *rpc = P.im[im == 0 ? P.ref : 1].rpc;
-        node_horner_poly(rpc, P.grid_wgs[2 * pt], P.grid_wgs[2 * pt + 1], j, N.horner[im][j]);
-        if (j == 0) {
-            N.hnorm[im][0] = rpc[4];
-            N.hnorm[im][1] = 1.0 / rpc[9];
-        }
-    } else if (lane < 10) {
-        const int im = lane - 8;
-        const DevImage &I = P.im[im == 0 ? P.ref : 1];
-        double *g = N.geo[im];
-        g[0] = I.adj[0];
-        g[1] = I.adj[1];
-        g[2] = I.rpc[0];
-        g[3] = I.rpc[1];
-        g[4] = I.rpc[5];
-        g[5] = I.rpc[6];
-        g[6] = I.sx;
-        g[7] = I.sy;
-        N.img[im] = I.img;
-        N.mag[im] = I.mag;
-        N.ori[im] = I.ori;
-        N.w[im] = I.w;
-        N.h[im] = I.h;
-        N.tma_w[im] = P.tma_w[im];
-        N.tma_h[im] = P.tma_h[im];
-    } else if (lane == 10) {
-        const vll_ugrid g = P.gp3[pt];
-        const vll_nccresult R = P.ncc[pt];
-        const DevImage &ri = P.im[P.ref], &tI = P.im[1];
-        N.P = &P;
-        N.gn = gn;
-        N.pt = pt;
-        N.K = K;
-        N.H = P.H;
-        N.start_H = g.minHeight;
-        N.end_H = g.maxHeight;
-        N.R = R;
-        N.hbase = (double)((P.is_ra || P.cmr) ? g.minHeight : R.minHeight);
-        N.hstep = P.height_step;
-        N.inv_s = 1.0 / (double)(1 << P.L);
-        N.bin_angle = P.bin_angle;
-        N.alpha = P.alpha;
-        const double cnt_g = gcnt ? gcnt[gn] : 0.0;
-        const bool gncc = P.check_ortho && cnt_g > 0;
-        N.gterm = gncc ? (gsum[gn] / cnt_g) * P.beta : 0.0;
-        const bool voxels = P.vox && !P.cmr && !P.is_ra;
-        N.vrow = voxels ? P.vox + P.vox_off[pt] : nullptr;
-        const bool vec_ok = (ri.w % 8 == 0) && (tI.w % 8 == 0) &&
-                            ((reinterpret_cast<uintptr_t>(ri.img) | reinterpret_cast<uintptr_t>(ri.mag) |
-                              reinterpret_cast<uintptr_t>(tI.img) |
-                              reinterpret_cast<uintptr_t>(tI.mag)) & 15) == 0;
-        N.flags = (P.cmr ? kNfCmr : 0u) | ((!P.is_ra && P.L >= 3) ? kNfOri : 0u) |
-                  (voxels ? kNfVox : 0u) | (R.check_height_change ? kNfChc : 0u) |
-                  (gncc ? kNfGncc : 0u) | (vec_ok ? kNfVec : 0u) | (P.tma_w[0] > 0 ? kNfTma : 0u) |
-                  (P.dbg_rho ? kNfDbg : 0u);
-        N.pre_v = -1.0f;
-        N.pre_dir = 0;
-        N.pre_k = -1;
-        N.have = 0;
-    }
-    __syncwarp();
-}
 
 // Image coordinate (pyramid level) of one slot of node N in image im from
 // the node's cubics (fast_coord's arithmetic on the node context).
@@ -835,8 +433,9 @@ __device__ __noinline__ void slot_coords_exact(const NodeCtx &N, double hgt, dou
 // any other node is queued for the exact pass with its FP32 values (NaN
 // marking the slots that need an exact value) in the pending buffer, or with
 // offset -1 (evaluated wholly in FP64 there) when the buffer is full.  Nodes
-// of combined-level INCC, or with more slots than kSlotCap, are queued with
-// offset -2 (evaluated wholly in FP64 by the exact pass).
+// with more slots than kSlotCap are queued with offset -2 (evaluated wholly in
+// FP64 by the exact pass).  Levels of combined INCC are combined_kernel's: the
+// slot counts given here are 0 for their nodes.
 __global__ void __launch_bounds__(kWinWarps * 32, VLL_WIN_MINB) window_kernel(
     const LevelSet LS, const int32_t *__restrict__ node_k, const double *__restrict__ gsum,
     const double *__restrict__ gcnt, float *__restrict__ pend_vals, int64_t pend_cap,
@@ -1450,8 +1049,9 @@ __device__ __forceinline__ double slot_value(const WarpShared &w, int k, bool &e
 // the samples in the reference's scan order; lane 0 combines them in
 // ComputeMultiNCC's order.  `scratch` holds (2H+1)^2 x 4 doubles + flags.
 template <int H>
-__device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, const PatchSrc &S, float hgt,
-                                  double cnt_g, double sum_g, double *scratch, int lane) {
+__device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, const PatchSrc &S,
+                                               const PatchSrc &Sn, float hgt, double cnt_g,
+                                               double sum_g, double *scratch, int lane) {
     constexpr int D = 2 * H + 1;
     SlotOut o;
     o.evaluated = false;
@@ -1470,89 +1070,109 @@ __device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, co
     }
     const double2 rc = make_double2(__shfl_sync(0xffffffffu, c.x, 0), __shfl_sync(0xffffffffu, c.y, 0));
     const double2 tc = make_double2(__shfl_sync(0xffffffffu, c.x, 1), __shfl_sync(0xffffffffu, c.y, 1));
-    const double2 rp = to_pyramid(rc, ri.sx, ri.sy, P.L);
-    const double2 tp = to_pyramid(tc, tI.sx, tI.sy, P.L);
+    double2 rp = to_pyramid(rc, ri.sx, ri.sy, P.L);
+    double2 tp = to_pyramid(tc, tI.sx, tI.sy, P.L);
     if (!(in_image(rp, ri.w, ri.h) && in_image(tp, tI.w, tI.h))) return o;
-    const int od = (int)ri.ori[(int64_t)(int)rp.y * ri.w + (int)rp.x] -
-                   (int)tI.ori[(int64_t)(int)tp.y * tI.w + (int)tp.x];
+    // twice the orientation difference (the sum over both levels when combined)
+    int twice = (int)ri.ori[(int64_t)(int)rp.y * ri.w + (int)rp.x] -
+                (int)tI.ori[(int64_t)(int)tp.y * tI.w + (int)tp.x];
+    if (P.combined_incc) {
+        const double2 rn = to_pyramid(rc, ri.sxn, ri.syn, P.L - 1);
+        const double2 tn = to_pyramid(tc, tI.sxn, tI.syn, P.L - 1);
+        if (!(in_image(rn, ri.wn, ri.hn) && in_image(tn, tI.wn, tI.hn))) return o;
+        twice += (int)ri.ori_n[(int64_t)(int)rn.y * ri.wn + (int)rn.x] -
+                 (int)tI.ori_n[(int64_t)(int)tn.y * tI.wn + (int)tn.x];
+    } else {
+        twice *= 2;
+    }
     if (!P.is_ra && P.L >= 3) {
-        const double a = __dmul_rn((double)od, P.bin_angle);
+        const double a = __dmul_rn(__ddiv_rn((double)twice, 2.0), P.bin_angle);
         if (!(a < 90 && a > -90)) {
             o.orient_reject = true;
             return o;
         }
     }
     o.evaluated = true;
-    const double c0 = P.rot_cos[2 * od + kRotOffset], s0 = P.rot_sin[2 * od + kRotOffset];
+    const double c0 = P.rot_cos[twice + kRotOffset], s0 = P.rot_sin[twice + kRotOffset];
     unsigned char *flag = reinterpret_cast<unsigned char *>(scratch + 4 * D * D);
-    for (int idx = lane; idx < D * D; idx += 32) {
-        const int row = idx / D - H, col = idx % D - H;
-        const int r2 = row * row + col * col;
-        unsigned char f = 0;
-        if (r2 <= (H + 1) * (H + 1)) {
-            const double ox = __dadd_rn(__dmul_rn(c0, (double)col), -__dmul_rn(s0, (double)row));
-            const double oy = __dadd_rn(__dmul_rn(s0, (double)col), __dmul_rn(c0, (double)row));
-            const double2 pl = make_double2(__dadd_rn(rp.x, (double)col), __dadd_rn(rp.y, (double)row));
-            const double2 pr = make_double2(__dadd_rn(tp.x, ox), __dadd_rn(tp.y, oy));
-            double v[4];
-            if (sample4(S, pl, pr, v)) {
-                f = (unsigned char)(1 + window_depth(H, row, col, r2));   // 1 + depth
+    double count = 0, sum = 0;
+#pragma unroll 1
+    for (int lev = 0; lev <= (P.combined_incc ? 1 : 0); ++lev) {
+        if (lev) {
+            rp = to_pyramid(rc, ri.sxn, ri.syn, P.L - 1);
+            tp = to_pyramid(tc, tI.sxn, tI.syn, P.L - 1);
+        }
+        const PatchSrc &Q = lev ? Sn : S;
+        for (int idx = lane; idx < D * D; idx += 32) {
+            const int row = idx / D - H, col = idx % D - H;
+            const int r2 = row * row + col * col;
+            unsigned char f = 0;
+            if (r2 <= (H + 1) * (H + 1)) {
+                const double ox = __dadd_rn(__dmul_rn(c0, (double)col), -__dmul_rn(s0, (double)row));
+                const double oy = __dadd_rn(__dmul_rn(s0, (double)col), __dmul_rn(c0, (double)row));
+                const double2 pl =
+                    make_double2(__dadd_rn(rp.x, (double)col), __dadd_rn(rp.y, (double)row));
+                const double2 pr = make_double2(__dadd_rn(tp.x, ox), __dadd_rn(tp.y, oy));
+                double v[4];
+                if (sample4(Q, pl, pr, v)) {
+                    f = (unsigned char)(1 + window_depth(H, row, col, r2));   // 1 + depth
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) scratch[4 * idx + ch] = v[ch];
+                    for (int ch = 0; ch < 4; ++ch) scratch[4 * idx + ch] = v[ch];
+                }
             }
+            flag[idx] = f;
         }
-        flag[idx] = f;
-    }
-    __syncwarp();
-    // lanes 0..5: Correlate for (window w, channel pair p), SubFunctions.cpp:974-1018
-    double r = -99.0;
-    int n = 0;
-    if (lane < 6) {
-        const int w = lane >> 1, p = lane & 1;
-        double Ls = 0, Rs = 0;
-        for (int idx = 0; idx < D * D; ++idx) {
-            const int f = flag[idx];
-            if (f == 0 || f - 1 < w) continue;
-            Ls = __dadd_rn(Ls, scratch[4 * idx + p]);
-            Rs = __dadd_rn(Rs, scratch[4 * idx + p + 2]);
-            ++n;
-        }
-        if (n > 0) {
-            const double Lm = __ddiv_rn(Ls, (double)n), Rm = __ddiv_rn(Rs, (double)n);
-            double slr = 0, sl2 = 0, sr2 = 0;
+        __syncwarp();
+        // lanes 0..5: Correlate for (window w, channel pair p), SubFunctions.cpp:974-1018
+        double r = -99.0;
+        int n = 0;
+        if (lane < 6) {
+            const int w = lane >> 1, p = lane & 1;
+            double Ls = 0, Rs = 0;
             for (int idx = 0; idx < D * D; ++idx) {
                 const int f = flag[idx];
                 if (f == 0 || f - 1 < w) continue;
-                const double dl = __dadd_rn(scratch[4 * idx + p], -Lm);
-                const double dr = __dadd_rn(scratch[4 * idx + p + 2], -Rm);
-                slr = __dadd_rn(slr, __dmul_rn(dl, dr));
-                sl2 = __dadd_rn(sl2, __dmul_rn(dl, dl));
-                sr2 = __dadd_rn(sr2, __dmul_rn(dr, dr));
+                Ls = __dadd_rn(Ls, scratch[4 * idx + p]);
+                Rs = __dadd_rn(Rs, scratch[4 * idx + p + 2]);
+                ++n;
             }
-            if (sl2 > 1e-8 && sr2 > 1e-8) r = __ddiv_rn(slr, sqrt(__dmul_rn(sl2, sr2)));
-        }
-    }
-    double rv[6];
-    int nv[3];
-#pragma unroll
-    for (int j = 0; j < 6; ++j) rv[j] = __shfl_sync(0xffffffffu, r, j);
-#pragma unroll
-    for (int w = 0; w < 3; ++w) nv[w] = __shfl_sync(0xffffffffu, n, 2 * w);
-    __syncwarp();
-    o.all_pos = nv[0] > 0 && nv[1] > 0 && nv[2] > 0;
-    double count = 0, sum = 0;
-    if (o.all_pos) {
-        double tot = 0, cntv = 0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            if (rv[j] != -99.0) {
-                cntv = __dadd_rn(cntv, 1.0);
-                tot = __dadd_rn(tot, rv[j]);
+            if (n > 0) {
+                const double Lm = __ddiv_rn(Ls, (double)n), Rm = __ddiv_rn(Rs, (double)n);
+                double slr = 0, sl2 = 0, sr2 = 0;
+                for (int idx = 0; idx < D * D; ++idx) {
+                    const int f = flag[idx];
+                    if (f == 0 || f - 1 < w) continue;
+                    const double dl = __dadd_rn(scratch[4 * idx + p], -Lm);
+                    const double dr = __dadd_rn(scratch[4 * idx + p + 2], -Rm);
+                    slr = __dadd_rn(slr, __dmul_rn(dl, dr));
+                    sl2 = __dadd_rn(sl2, __dmul_rn(dl, dl));
+                    sr2 = __dadd_rn(sr2, __dmul_rn(dr, dr));
+                }
+                if (sl2 > 1e-8 && sr2 > 1e-8) r = __ddiv_rn(slr, sqrt(__dmul_rn(sl2, sr2)));
             }
         }
-        if (cntv > 0) {
-            sum = __ddiv_rn(tot, cntv);
-            count = 1.0;
+        double rv[6];
+        int nv[3];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) rv[j] = __shfl_sync(0xffffffffu, r, j);
+#pragma unroll
+        for (int w = 0; w < 3; ++w) nv[w] = __shfl_sync(0xffffffffu, n, 2 * w);
+        __syncwarp();
+        const bool all_pos = nv[0] > 0 && nv[1] > 0 && nv[2] > 0;
+        if (lev == 0) o.all_pos = all_pos;
+        if (all_pos) {
+            double tot = 0, cntv = 0;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                if (rv[j] != -99.0) {
+                    cntv = __dadd_rn(cntv, 1.0);
+                    tot = __dadd_rn(tot, rv[j]);
+                }
+            }
+            if (cntv > 0) {
+                sum = __dadd_rn(sum, __ddiv_rn(tot, cntv));
+                count = __dadd_rn(count, 1.0);
+            }
         }
     }
     o.count_incc = count;
@@ -1573,15 +1193,16 @@ __host__ __device__ constexpr size_t exact_scratch_bytes(int H) {
 
 // Exact FP64 evaluation of one slot by the warp for the level's half-size.
 __device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, int64_t pt,
-                                                      const PatchSrc &S, float hgt, double cnt_g,
-                                                      double sum_g, double *scratch, int lane) {
+                                                      const PatchSrc &S, const PatchSrc &Sn,
+                                                      float hgt, double cnt_g, double sum_g,
+                                                      double *scratch, int lane) {
     switch (P.H) {
-        case 2: return eval_slot_warp<2>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
-        case 3: return eval_slot_warp<3>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
-        case 4: return eval_slot_warp<4>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
-        case 5: return eval_slot_warp<5>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
-        case 6: return eval_slot_warp<6>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
-        default: return eval_slot_warp<7>(P, pt, S, hgt, cnt_g, sum_g, scratch, lane);
+        case 2: return eval_slot_warp<2>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        case 3: return eval_slot_warp<3>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        case 4: return eval_slot_warp<4>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        case 5: return eval_slot_warp<5>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        case 6: return eval_slot_warp<6>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        default: return eval_slot_warp<7>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
     }
 }
 
@@ -1628,9 +1249,9 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
         const int start_H = P.gp3[pt].minHeight;
         const double cnt_g = gcnt ? gcnt[gn] : 0.0, sum_g = gsum ? gsum[gn] : 0.0;
         vll_voxel *vrow = voxels ? P.vox + P.vox_off[pt] : nullptr;
-        if (off < 0 || K > kSlotCap || P.combined_incc) {
-            // queued without FP32 values: not evaluated yet (-2: combined-level
-            // INCC or more slots than kSlotCap), or the pending buffer was full
+        if (off < 0 || K > kSlotCap) {
+            // queued without FP32 values: not evaluated yet (-2: more slots than
+            // kSlotCap), or the pending buffer was full
             const bool first = off == -2;
             if (lane == 0) atomicAdd(&counters[5], 1ull);
             node_exact_chunked(P, pt, K, S, Sn, cnt_g, sum_g, R, vrow, W.chunk, lane, first,
@@ -1692,7 +1313,7 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
                 for (int j = 0; j < n_todo; ++j) {
                     const int k = W.todo[j];
                     const float hh = slot_height(P, start_H, R.minHeight, k);
-                    const SlotOut o = eval_slot_warp_any(P, pt, S, hh, cnt_g, sum_g,
+                    const SlotOut o = eval_slot_warp_any(P, pt, S, Sn, hh, cnt_g, sum_g,
                                                         reinterpret_cast<double *>(boxes), lane);
                     if (lane == 0) {
                         if (P.dbg_rho && o.evaluated && isnan(P.dbg_rho[P.dbg_off[pt] + k]))
@@ -1787,7 +1408,8 @@ void host_rpc(const double *rpc, double lon, double lat, double h, double &x, do
 // The boxes covering 32 consecutive height slots of one node in both images
 // -- the reference window and the target window (rotated; its samples lie
 // within H + 1 of the centre) swept along their epipolar lines -- in texel
-// pairs (w x h), per image [0] reference, [1] target.  The sweep per slot,
+// pairs (w x h), per image [0] reference, [1] target, at pyramid level lev.
+// The sweep per slot,
 // along x and y, is measured from the RPCs over the image footprint; the
 // boxes are the worst case times `margin` (an item with a larger footprint
 // falls back to slower staging or to FP64).
@@ -1795,7 +1417,7 @@ struct WindowBoxes {
     int w[2], h[2];
 };
 
-WindowBoxes window_boxes(const DevLevel &P, float margin) {
+WindowBoxes window_boxes(const DevLevel &P, float margin, int lev) {
     const int H = P.H;
     double rx[2] = {0, 0}, ry[2] = {0, 0};
     for (int ti = 0; ti < 2; ++ti) {
@@ -1806,8 +1428,8 @@ WindowBoxes window_boxes(const DevLevel &P, float margin) {
                 double x0, y0, x1, y1;
                 host_rpc(r, lon, lat, r[4] - 50.0, x0, y0);
                 host_rpc(r, lon, lat, r[4] + 50.0, x1, y1);
-                rx[ti] = std::max(rx[ti], fabs(x1 - x0) / 100.0 / (1 << P.L));
-                ry[ti] = std::max(ry[ti], fabs(y1 - y0) / 100.0 / (1 << P.L));
+                rx[ti] = std::max(rx[ti], fabs(x1 - x0) / 100.0 / (1 << lev));
+                ry[ti] = std::max(ry[ti], fabs(y1 - y0) / 100.0 / (1 << lev));
             }
     }
     // one slot's box (texel pairs, rows: the reference window 2H + 2, the
@@ -1831,7 +1453,7 @@ struct WarpBudget {
 };
 
 WarpBudget window_warp_budget(const DevLevel &P, float margin) {
-    const WindowBoxes B = window_boxes(P, margin);
+    const WindowBoxes B = window_boxes(P, margin, P.L);
     WarpBudget wb;
     // boxes up to the budget's sides, rows of odd stride
     wb.quads = (B.w[0] | 1) * B.h[0] + (B.w[1] | 1) * B.h[1];
@@ -1848,16 +1470,43 @@ WarpBudget window_warp_budget(const DevLevel &P, float margin) {
     return wb;
 }
 
-// Budget of a level set: the largest of its levels' budgets.
+// Budget of a level set: the largest of its levels' budgets (combined levels
+// aside).
 WarpBudget set_warp_budget(const DevLevel *hl, int n, float margin) {
     WarpBudget q{1, 128};
     for (int l = 0; l < n; ++l)
-        if (hl[l].n_nodes > 0) {
+        if (hl[l].n_nodes > 0 && !hl[l].combined_incc) {
             const WarpBudget b = window_warp_budget(hl[l], margin);
             q.quads = std::max(q.quads, b.quads);
             q.raw = std::max(q.raw, b.raw);
         }
     return q;
+}
+
+// Texel pairs per warp of the set's combined levels (both levels' boxes use
+// the same room).
+int combined_quads(const DevLevel *hl, int n, float margin) {
+    int q = 0;
+    for (int l = 0; l < n; ++l)
+        if (hl[l].n_nodes > 0 && hl[l].combined_incc)
+            for (int lev = hl[l].L - 1; lev <= hl[l].L; ++lev) {
+                const WindowBoxes B = window_boxes(hl[l], margin, lev);
+                q = std::max(q, (B.w[0] | 1) * B.h[0] + (B.w[1] | 1) * B.h[1]);
+            }
+    return q;
+}
+
+// Whether the set has a level for the window kernel, and one for the
+// combined kernel.
+bool any_plain_level(const DevLevel *hl, int n) {
+    for (int l = 0; l < n; ++l)
+        if (hl[l].n_nodes > 0 && !hl[l].combined_incc) return true;
+    return false;
+}
+bool any_combined_level(const DevLevel *hl, int n) {
+    for (int l = 0; l < n; ++l)
+        if (hl[l].n_nodes > 0 && hl[l].combined_incc) return true;
+    return false;
 }
 
 int set_max_h(const DevLevel *hl, int n) {
@@ -1925,9 +1574,10 @@ cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
 
 // the window and exact stages of the pipeline on given buffers (ctl cleared
 // by the caller: [0] node queue, [1] exact-pass queue, [2] queued nodes,
-// [4] pending-buffer cursor)
+// [4] pending-buffer cursor, [5] listed voxel slots, [6] the combined
+// kernel's node queue); plain_k: room for a mixed set's slot counts
 cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, const int32_t *node_k,
-                             const double *gsum, const double *gcnt, float *pend_vals,
+                             int32_t *plain_k, const double *gsum, const double *gcnt, float *pend_vals,
                              int64_t pend_cap, int64_t *pend_node, int64_t *pend_off,
                              int64_t fix_cap, unsigned long long *counters,
                              unsigned long long *ctl, const SplitTuning &tu, cudaStream_t s,
@@ -1935,8 +1585,22 @@ cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, cons
     // the voxel slots listed for an exact INCC follow the warps' scratch
     int64_t *fix_list = reinterpret_cast<int64_t *>(
         pend_vals + ((pend_cap + window_scratch_floats() + 1) & ~(int64_t)1));
-    cudaError_t e = launch_window(hl, n, LS, node_k, gsum, gcnt, pend_vals, pend_cap, pend_node,
-                                  pend_off, fix_list, fix_cap, counters, ctl, tu, s);
+    cudaError_t e = cudaSuccess;
+    if (any_plain_level(hl, n)) {
+        // a mixed set's window kernel sees no slots at the combined levels
+        const int32_t *window_k = node_k;
+        if (any_combined_level(hl, n)) {
+            e = launch_plain_counts(LS, node_k, plain_k, s);
+            window_k = plain_k;
+        }
+        if (e == cudaSuccess)
+            e = launch_window(hl, n, LS, window_k, gsum, gcnt, pend_vals, pend_cap, pend_node,
+                              pend_off, fix_list, fix_cap, counters, ctl, tu, s);
+    }
+    if (e == cudaSuccess && any_combined_level(hl, n))
+        e = launch_combined(LS, node_k, gsum, gcnt, pend_vals, pend_cap, pend_node, pend_off,
+                            fix_list, fix_cap, counters, ctl,
+                            combined_quads(hl, n, tu.box_margin), window_max_blocks_per_sm(), s);
     if (e != cudaSuccess) return e;
     if (fix_cap > 0) {
         int dev = 0, sms = 148;
@@ -2052,7 +1716,7 @@ void split_prepare_tma(DevLevel &P, float margin) {
     P.tma_w[0] = P.tma_w[1] = P.tma_h[0] = P.tma_h[1] = 0;
     EncodeTiledFn enc = encode_tiled();
     if (!enc || !split_supported(P) || P.combined_incc) return;
-    const WindowBoxes B = window_boxes(P, margin);
+    const WindowBoxes B = window_boxes(P, margin, P.L);
     int tw[2], th[2];
     for (int ti = 0; ti < 2; ++ti) {
         const DevImage &im = P.im[ti == 0 ? P.ref : 1];
@@ -2089,7 +1753,7 @@ bool split_supported(const DevLevel &P) {
 }
 
 void split_release(SplitBuffers &b) {
-    void **all[] = {&b.node_k, &b.slot_off, &b.rho, &b.gsum, &b.gcnt, &b.scan_tmp, &b.ctl,
+    void **all[] = {&b.node_k, &b.plain_k, &b.slot_off, &b.rho, &b.gsum, &b.gcnt, &b.scan_tmp, &b.ctl,
                     &b.pending, &b.pend_off, &b.base, &b.acc_level};
     for (void **p : all) {
         if (*p) cudaFree(*p);
@@ -2137,8 +1801,12 @@ cudaError_t split_front(SplitBuffers &b, const DevLevel *hl, const DevLevel *dl,
             *p = nullptr;
             SPLIT_CUDA(cudaMalloc(p, (size_t)(N + 1) * 8));
         }
+        if (b.plain_k) cudaFree(b.plain_k);
+        b.plain_k = nullptr;
         b.cap_nodes = (size_t)(N + 1);
     }
+    if (!b.plain_k && any_plain_level(hl, n_levels) && any_combined_level(hl, n_levels))
+        SPLIT_CUDA(cudaMalloc(&b.plain_k, b.cap_nodes * sizeof(int32_t)));
     if ((size_t)n_levels + 1 > b.cap_levels) {
         if (b.base) cudaFree(b.base);
         if (b.acc_level) cudaFree(b.acc_level);
@@ -2197,7 +1865,8 @@ cudaError_t split_back(SplitBuffers &b, const DevLevel *hl, int n_levels, const 
         if (tm && tm->enabled) cudaEventRecord(tm->ev[i], s);
     };
     mark(4);
-    cudaError_t e = window_and_peaks(hl, n_levels, LS, (const int32_t *)b.node_k, gsum, gcnt,
+    cudaError_t e = window_and_peaks(hl, n_levels, LS, (const int32_t *)b.node_k,
+                                     (int32_t *)b.plain_k, gsum, gcnt,
                                      (float *)b.rho, b.pend_cap, (int64_t *)b.pending,
                                      (int64_t *)b.pend_off, b.fix_cap, counters,
                                      (unsigned long long *)b.ctl, tu, s, tm);
@@ -2205,7 +1874,9 @@ cudaError_t split_back(SplitBuffers &b, const DevLevel *hl, int n_levels, const 
         *err = "window / exact kernel launch";
         return e;
     }
-    *launches += 2 + (b.fix_cap > 0 ? 1 : 0);
+    const bool plain = any_plain_level(hl, n_levels), combined = any_combined_level(hl, n_levels);
+    *launches += 1 + (plain ? 1 : 0) + (combined ? 1 : 0) + (plain && combined ? 1 : 0) +
+                 (b.fix_cap > 0 ? 1 : 0);
     mark(7);
     mark(8);
     return cudaSuccess;
@@ -2510,7 +2181,7 @@ extern "C" int vll_vertical_line_locus_noalloc(const vll_level_desc *desc,
     prep_kernel<<<grid_1d(N, 256, 148 * 32), 256, 0, s>>>(LS, nullptr, nullptr, node_k, counters,
                                                           acc_level);
     NA_CUDA(cudaGetLastError());
-    NA_CUDA(window_and_peaks(&P, 1, LS, node_k, nullptr, nullptr, pend_vals, pend_cap, pending,
+    NA_CUDA(window_and_peaks(&P, 1, LS, node_k, nullptr, nullptr, nullptr, pend_vals, pend_cap, pending,
                              pend_off, 0, counters, ctl, SplitTuning(), s, nullptr));
     unsigned long long acc = 0;
     NA_CUDA(cudaMemcpyAsync(&acc, counters, sizeof(acc), cudaMemcpyDeviceToHost, s));

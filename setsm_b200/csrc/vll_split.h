@@ -16,9 +16,23 @@ struct DevLevel;
 // least `bytes`, never lowering it (thread-safe; see vll_split.cu).
 cudaError_t ensure_smem_limit(const void *func, size_t bytes);
 
+// vll_combined.cu: the slot counts of a mixed set without its combined
+// levels, and the streaming pass over the nodes of combined levels (quads:
+// texel pairs per warp; the grid holds at most max_blocks_per_sm blocks per SM).
+struct LevelSet;
+cudaError_t launch_plain_counts(const LevelSet &LS, const int32_t *node_k, int32_t *plain_k,
+                                cudaStream_t s);
+cudaError_t launch_combined(const LevelSet &LS, const int32_t *node_k, const double *gsum,
+                            const double *gcnt, float *pend_vals, int64_t pend_cap,
+                            int64_t *pend_node, int64_t *pend_off, int64_t *fix_list,
+                            int64_t fix_cap, unsigned long long *counters,
+                            unsigned long long *ctl, int quads, int max_blocks_per_sm,
+                            cudaStream_t s);
+
 // Device scratch of the split pipeline, grown on demand and owned by a context.
 struct SplitBuffers {
     void *node_k = nullptr;        // int32  [N+1] slots per active node (0 = inactive)
+    void *plain_k = nullptr;       // int32  [N+1] the same without combined levels (mixed sets)
     void *slot_off = nullptr;      // int64  [N+1] prefix sum of node_k (the slot total)
     void *rho = nullptr;           // float  [pend_cap] FP32 slot values of queued nodes, then
                                    // the window kernel's per-warp slot scratch, then the
