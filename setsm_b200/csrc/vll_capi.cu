@@ -1007,6 +1007,7 @@ int vll_debug_slot_rho(vll_context *ctx, const vll_level_desc *desc, const vll_u
         off[i + 1] = off[i] + nh;
     }
     if (capacity < off[N]) return fail(ctx, VLL_ERR_CAPACITY, "rho buffer too small");
+    const bool next = vll::needs_next(P);
     for (int ti = 0; ti < P.num_images; ++ti) {
         const vll_image_desc &s = desc->images[ti];
         if (!s.selected) continue;
@@ -1017,6 +1018,16 @@ int vll_debug_slot_rho(vll_context *ctx, const vll_level_desc *desc, const vll_u
         P.im[ti].img = (const uint16_t *)ctx->img[ti][0].p;
         P.im[ti].mag = (const uint16_t *)ctx->img[ti][1].p;
         P.im[ti].ori = (const uint8_t *)ctx->img[ti][2].p;
+        if (!next) continue;
+        if (!s.image_next || !s.mag_next || !s.ori_next || s.width_next < 2 || s.height_next < 2)
+            return fail(ctx, VLL_ERR_INVALID, "combined level needs the next pyramid level");
+        const size_t nn = (size_t)s.width_next * s.height_next;
+        if ((rc = upload(ctx, ctx->img[ti][3], s.image_next, nn * 2))) return rc;
+        if ((rc = upload(ctx, ctx->img[ti][4], s.mag_next, nn * 2))) return rc;
+        if ((rc = upload(ctx, ctx->img[ti][5], s.ori_next, nn))) return rc;
+        P.im[ti].img_n = (const uint16_t *)ctx->img[ti][3].p;
+        P.im[ti].mag_n = (const uint16_t *)ctx->img[ti][4].p;
+        P.im[ti].ori_n = (const uint8_t *)ctx->img[ti][5].p;
     }
     if ((rc = upload(ctx, ctx->wgs, desc->grid_wgs, (size_t)N * 16))) return rc;
     if ((rc = upload(ctx, ctx->pts, desc->grid_pts, (size_t)N * 16))) return rc;

@@ -64,20 +64,31 @@ struct Acc2 {
     float2 sl, sr, sll, srr, slr;
 };
 
-// The target box lives in the block's shared memory at byte offsets from
-// `base`; `tq` is the offset of the window centre's texel, biased so that
-// the fixed-point bits of the round-to-nearest constant index it directly:
-// offset of texel (cx + dx, cy + dy) = tq + bits(M + dy) * row + bits(M + dx) * 16
+// The target box lives in the block's shared memory; `tq` is the 32-bit
+// shared address of the window centre's texel, biased so that the
+// fixed-point bits of the round-to-nearest constant index it directly:
+// address of texel (cx + dx, cy + dy) = tq + bits(M + dy) * row + bits(M + dx) * 16
 // (mod 2^32), M = 1.5 * 2^23.
 struct TgtBox {
-    const unsigned char *base;   // shared-memory window of the block
-    uint32_t tq;                 // biased offset (see above)
-    uint32_t row;                // row stride in bytes
+    uint32_t tq;    // biased shared-memory address (see above)
+    uint32_t row;   // row stride in bytes
 };
 
 __device__ __forceinline__ TgtBox tgt_box(const unsigned char *base, uint32_t centre_off,
                                           uint32_t row) {
-    return TgtBox{base, centre_off - 0x4B400000u * (row + 16u), row};
+    return TgtBox{(uint32_t)__cvta_generic_to_shared(base) + centre_off -
+                      0x4B400000u * (row + 16u), row};
+}
+
+// 128-bit shared load by its 32-bit address (through pointers the address
+// cost three more instructions per sample: 11x11 77.5 against 73.8 ms).
+__device__ __forceinline__ float4 lds128(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
 }
 
 struct WinCtx {
@@ -110,79 +121,29 @@ __device__ __forceinline__ float2 tgt_sample(const TgtBox &tb, float2 f, float2 
     const float2 fr = __fadd2_rn(f, __ffma2_rn(t, make_float2(-1.f, -1.f), bc2(kMagic)));
     const uint32_t a = (uint32_t)__float_as_int(t.y) * tb.row +
                        ((uint32_t)__float_as_int(t.x) << 4) + tb.tq;
-    const float4 ta = *reinterpret_cast<const float4 *>(tb.base + a);
-    const float4 tv = *reinterpret_cast<const float4 *>(tb.base + a + tb.row);
+    const float4 ta = lds128(a);
+    const float4 tv = lds128(a + tb.row);
     const float2 fx = bc2(fr.x), fy = bc2(fr.y);
     const float2 top = __ffma2_rn(fx, hi2(ta), lo2(ta));
     const float2 bot = __ffma2_rn(fx, hi2(tv), lo2(tv));
     return __fadd2_rn(__ffma2_rn(fy, sub2(bot, top), top), init);
 }
 
-// First window column of rows with |row| = AR (the circle r^2 <= (H+1)^2).
-__host__ __device__ constexpr int row_cmin(int H, int AR) {
-    int c = -H;
-    while (AR * AR + c * c > (H + 1) * (H + 1)) ++c;
+// Largest |col| of window row |row| = ar in the sub-window of `ring` and
+// those inside it (0: the whole window), -1 when the row lies outside it.
+__host__ __device__ constexpr int ring_cols(int H, int ring, int ar) {
+    int c = -1;
+    for (int col = 0; col <= H; ++col)
+        if (ar * ar + col * col <= (H + 1) * (H + 1) && ring_of(H, ar, col) >= ring) c = col;
     return c;
 }
 
-// One window row of sub-window pattern |row| = AR at signed offset `row`:
-// columns unrolled, each accumulating into its compile-time ring.
-template <int H, int AR>
-__device__ __forceinline__ void win_row(const WinCtx &x, int row, const float4 *__restrict__ qr,
-                                        float2 tf, Acc2 (&acc)[3]) {
-    const float4 *q0 = qr + (row + H) * x.rbw;
-    const float4 *q1 = q0 + x.rbw;
-    const float2 b = __ffma2_rn(x.nsc, bc2((float)row), tf);
-    // Reference texel pairs {I(c), M(c), I(c+1), M(c+1)} are read only at even
-    // offsets from the row's first column: a sample at an odd offset takes
-    // its left texel from the previous pair's high half and its right texel
-    // from the next pair's low half, so each pair feeds two samples.
-    constexpr int c0 = row_cmin(H, AR);
-    float4 a0 = q0[c0 + H], b0 = q1[c0 + H];   // pair at the last even offset
-    float4 a1 = a0, b1 = b0;                   // pair at the next even offset
-#pragma unroll
-    for (int col = -H; col <= H; ++col) {
-        if (AR * AR + col * col > (H + 1) * (H + 1)) continue;
-        const int ring = ring_of(H, AR, col);
-        float2 l;
-        if (((col - c0) & 1) == 0) {
-            if (col != c0) {
-                a0 = a1;
-                b0 = b1;
-            }
-            l = ref_sample(x, a0, b0, x.ncl);
-        } else {
-            a1 = q0[col + 1 + H];
-            b1 = q1[col + 1 + H];
-            l = ref_sample(x, make_float4(a0.z, a0.w, a1.x, a1.y),
-                           make_float4(b0.z, b0.w, b1.x, b1.y), x.ncl);
-        }
-        const float2 r = tgt_sample(x.tb, __ffma2_rn(x.cs, bc2((float)col), b), x.ntc);
-        Acc2 &u = acc[ring];
-        u.sl = __fadd2_rn(u.sl, l);
-        u.sr = __fadd2_rn(u.sr, r);
-        u.sll = __ffma2_rn(l, l, u.sll);
-        u.srr = __ffma2_rn(r, r, u.srr);
-        u.slr = __ffma2_rn(l, r, u.slr);
-    }
-}
-
-// Rows +AR and -AR share the pattern of |row| = AR (the sub-windows are
-// symmetric), so each pattern's unrolled code serves two rows.
-template <int H, int AR>
-__device__ __forceinline__ void win_rows(const WinCtx &x, const float4 *__restrict__ qr,
-                                         float2 tf, Acc2 (&acc)[3]) {
-    if constexpr (AR <= H) {
-#pragma unroll 1
-        for (int sgn = (AR == 0 ? 1 : -1); sgn <= 1; sgn += 2)
-            win_row<H, AR>(x, sgn * AR, qr, tf, acc);
-        win_rows<H, AR + 1>(x, qr, tf, acc);
-    }
-}
-
-__device__ __forceinline__ Acc plane(const Acc2 &a, int p) {
-    return p == 0 ? Acc{a.sl.x, a.sr.x, a.sll.x, a.srr.x, a.slr.x}
-                  : Acc{a.sl.y, a.sr.y, a.sll.y, a.srr.y, a.slr.y};
+// Rows |row| (bit mask) whose samples of sub-window `ring` end at column c.
+__host__ __device__ constexpr uint32_t rows_ending(int H, int ring, int c) {
+    uint32_t m = 0;
+    for (int ar = 0; ar <= H; ++ar)
+        if (ring_cols(H, ring, ar) == c) m |= 1u << ar;
+    return m;
 }
 
 __device__ __forceinline__ void add_to(Acc2 &w, const Acc2 &a) {
@@ -191,6 +152,97 @@ __device__ __forceinline__ void add_to(Acc2 &w, const Acc2 &a) {
     w.sll = __fadd2_rn(w.sll, a.sll);
     w.srr = __fadd2_rn(w.srr, a.srr);
     w.slr = __fadd2_rn(w.slr, a.slr);
+}
+
+__device__ __forceinline__ void add_sample(Acc2 &u, float2 l, float2 r) {
+    u.sl = __fadd2_rn(u.sl, l);
+    u.sr = __fadd2_rn(u.sr, r);
+    u.sll = __ffma2_rn(l, l, u.sll);
+    u.srr = __ffma2_rn(r, r, u.srr);
+    u.slr = __ffma2_rn(l, r, u.slr);
+}
+
+// The sample columns -K and K of a row, then those further out.  The row's sums
+// are added to a sub-window's when the last of its columns has been taken.
+// q0, q1: the shared-memory addresses of the two texel rows' pairs at column
+// -H; (la, lb), (ra, rb4): the pairs {I(c), M(c), I(c+1), M(c+1)} last read to
+// the left and right.  Pairs are read at even columns only: a sample at an odd
+// one takes its texels from the halves of its neighbours (the last column of
+// an odd H reads its own).
+template <int H, int K>
+__device__ __forceinline__ void win_cols(const WinCtx &x, uint32_t rb, uint32_t q0, uint32_t q1,
+                                         float2 b, Acc2 &a, Acc2 (&w)[3], float4 la, float4 lb,
+                                         float4 ra, float4 rb4) {
+    float2 l, m;
+    if constexpr ((K & 1) && K == H) {
+        l = ref_sample(x, lds128(q0 + 16 * (H - K)), lds128(q1 + 16 * (H - K)), x.ncl);
+        m = ref_sample(x, lds128(q0 + 16 * (H + K)), lds128(q1 + 16 * (H + K)), x.ncl);
+    } else if constexpr (K & 1) {
+        const float4 na = lds128(q0 + 16 * (H - K - 1)), nb = lds128(q1 + 16 * (H - K - 1));
+        l = ref_sample(x, make_float4(na.z, na.w, la.x, la.y),
+                       make_float4(nb.z, nb.w, lb.x, lb.y), x.ncl);
+        const float4 pa = lds128(q0 + 16 * (H + K + 1)), pb = lds128(q1 + 16 * (H + K + 1));
+        m = ref_sample(x, make_float4(ra.z, ra.w, pa.x, pa.y),
+                       make_float4(rb4.z, rb4.w, pb.x, pb.y), x.ncl);
+        la = na;
+        lb = nb;
+        ra = pa;
+        rb4 = pb;
+    } else {
+        l = ref_sample(x, la, lb, x.ncl);
+        m = ref_sample(x, ra, rb4, x.ncl);
+    }
+    const float2 r = tgt_sample(x.tb, __ffma2_rn(x.cs, bc2((float)-K), b), x.ntc);
+    add_sample(a, l, r);
+    const float2 t = tgt_sample(x.tb, __ffma2_rn(x.cs, bc2((float)K), b), x.ntc);
+    add_sample(a, m, t);
+    constexpr uint32_t m2 = rows_ending(H, 2, K), m1 = rows_ending(H, 1, K),
+                       m0 = rows_ending(H, 0, K);
+    if constexpr (m2 != 0)
+        if (rb & m2) add_to(w[2], a);
+    if constexpr (m1 != 0)
+        if (rb & m1) add_to(w[1], a);
+    if constexpr (K < H && m0 != 0)
+        if (rb & m0) return;
+    if constexpr (K < H) win_cols<H, K + 1>(x, rb, q0, q1, b, a, w, la, lb, ra, rb4);
+}
+
+// The window's rows by one body: 2 H + 1 unrolled sample columns, taken from
+// the middle outwards, so that a row's share of each nested sub-window is a
+// prefix of its sums, added where the row's pattern (by |row|, the same on
+// every lane) ends it.  (H = 2: the inner sub-window is the centre sample
+// alone, without variance either way; its sums stay zero.)  The kernel is bound by instruction fetch: with a body
+// for each |row|, as before, the 4096^2 pair's 1 M nodes took 25.1 ms at 7x7
+// and 75.3 ms at 11x11 (64 sample bodies), with this one (11) 23.2 and 63.8.
+// A body of two columns in a loop is slower again (7x7 by 9 %, 11x11 by 12 %:
+// no overlap between its samples' loads).
+template <int H>
+__device__ __forceinline__ void win_rows(const WinCtx &x, const float4 *__restrict__ qr,
+                                         float2 tf, Acc2 (&w)[3]) {
+    const uint32_t qs = (uint32_t)__cvta_generic_to_shared(qr);
+#pragma unroll 1
+    for (int row = -H; row <= H; ++row) {
+        const uint32_t rb = 1u << (row < 0 ? -row : row);
+        const uint32_t q0 = qs + (uint32_t)((row + H) * x.rbw) * 16u;
+        const uint32_t q1 = q0 + 16u * (uint32_t)x.rbw;
+        const float2 b = __ffma2_rn(x.nsc, bc2((float)row), tf);
+        const float4 pa = lds128(q0 + 16 * H), pb = lds128(q1 + 16 * H);
+        const float2 l = ref_sample(x, pa, pb, x.ncl);
+        const float2 r = tgt_sample(x.tb, b, x.ntc);
+        Acc2 a;
+        a.sl = l;
+        a.sr = r;
+        a.sll = __fmul2_rn(l, l);
+        a.srr = __fmul2_rn(r, r);
+        a.slr = __fmul2_rn(l, r);
+        win_cols<H, 1>(x, rb, q0, q1, b, a, w, pa, pb, pa, pb);
+        add_to(w[0], a);
+    }
+}
+
+__device__ __forceinline__ Acc plane(const Acc2 &a, int p) {
+    return p == 0 ? Acc{a.sl.x, a.sr.x, a.sll.x, a.srr.x, a.slr.x}
+                  : Acc{a.sl.y, a.sr.y, a.sll.y, a.srr.y, a.slr.y};
 }
 
 // FP32 multi-window NCC of one slot (ComputeMultiNCC over the three nested
@@ -223,22 +275,18 @@ __device__ __forceinline__ void window_fp32(const float4 *__restrict__ qr, int r
         x.ncl = make_float2(-cl.x, -cl.y);
         x.ntc = make_float2(-ct.x, -ct.y);
     }
-    win_rows<H, 0>(x, qr, tf, acc);
+    win_rows<H>(x, qr, tf, acc);
     // nested windows: 2 = ring 2; 1 = rings 1+2; 0 = all rings
     constexpr int n2 = ring_count(H, 2);
     constexpr int n1 = n2 + ring_count(H, 1);
     constexpr int n0 = n1 + ring_count(H, 0);
-    Acc2 w1 = acc[2];
-    add_to(w1, acc[1]);
-    Acc2 w0 = w1;
-    add_to(w0, acc[0]);
     float tot = 0.f;
     int nv = 0;
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
         const float r2 = corr_from(plane(acc[2], p), (float)n2, unsure);
-        const float r1 = corr_from(plane(w1, p), (float)n1, unsure);
-        const float r0 = corr_from(plane(w0, p), (float)n0, unsure);
+        const float r1 = corr_from(plane(acc[1], p), (float)n1, unsure);
+        const float r0 = corr_from(plane(acc[0], p), (float)n0, unsure);
         if (r0 != -99.0f) { tot += r0; ++nv; }
         if (r1 != -99.0f) { tot += r1; ++nv; }
         if (r2 != -99.0f) { tot += r2; ++nv; }
@@ -421,6 +469,22 @@ __device__ __forceinline__ void tmap_acquire(const void *tmap) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
 }
 
+// Lists the zero texels of [0, bw] x rows [0, bh) of a raw tile in `zl` as
+// tag | row << 16 | x, counted in *zn (entries beyond `cap` are counted, not
+// stored).
+__device__ __forceinline__ void list_zeros(const unsigned char *__restrict__ rI, int nb, int bw,
+                                               int bh, uint32_t *zl, int *zn, int cap,
+                                               uint32_t tag, int lane) {
+#pragma unroll 1
+    for (int by = 0; by < bh; ++by)
+#pragma unroll 1
+        for (int bx = lane; bx <= bw; bx += 32)
+            if (*reinterpret_cast<const uint16_t *>(rI + by * nb + 2 * bx) == 0) {
+                const int k = atomicAdd(zn, 1);
+                if (k < cap) zl[k] = tag | ((uint32_t)by << 16) | (uint32_t)bx;
+            }
+}
+
 // Box texels of [x0, x0 + bw) x rows [0, bh) from the raw tiles in shared
 // memory: rawI / rawM hold, per box row (stride `nb` bytes), the uint16
 // texels from xa = x0 rounded down to 8 on.  Two adjacent box texels per
@@ -429,9 +493,8 @@ __device__ __forceinline__ void tmap_acquire(const void *tmap) {
 // (dm = 0: reference pairs; dm = -1: target value and difference, exact for
 // integers), each value placed in the mantissa of 2^23 and shifted by
 // -(2^23 + shift) in one exact addition.  Zero intensity texels among the
-// texels the box reads ([x0, x0 + bw] of each row) are listed in `zl` as
-// tag | row << 16 | (x - x0), counted in *zn (entries beyond `cap` are
-// counted, not stored).
+// texels the box reads ([x0, x0 + bw] of each row) are listed in `zl`
+// (list_zeros): they are rare, so the conversion only takes the minimum.
 __device__ __forceinline__ void convert_tile(float4 *__restrict__ dst, int ds,
                                              const unsigned char *__restrict__ rawI,
                                              const unsigned char *__restrict__ rawM, int nb,
@@ -451,6 +514,7 @@ __device__ __forceinline__ void convert_tile(float4 *__restrict__ dst, int ds,
     const float rbp = __fdividef(1.f, (float)bp);
     int by = (int)(((float)lane + 0.5f) * rbp), bq = lane - by * bp;
     const int dby = (int)(32.5f * rbp), dbq = 32 - dby * bp;
+    uint32_t zmin = 1;
     for (int q = lane; q < n2; q += 32) {
         const int bx = 2 * bq;
         const bool two = bx + 1 < bw;
@@ -461,19 +525,8 @@ __device__ __forceinline__ void convert_tile(float4 *__restrict__ dst, int ds,
         const uint32_t m1 = *reinterpret_cast<const uint16_t *>(rM + ro + 2);
         const uint32_t i2 = two ? *reinterpret_cast<const uint16_t *>(rI + ro + 4) : 1u;
         const uint32_t m2 = two ? *reinterpret_cast<const uint16_t *>(rM + ro + 4) : 0u;
-        // zero texels among those the box reads ([0, bw] of the row): this
-        // lane lists texels bx and bx + 1, and texel bx + 2 when it ends the
-        // row (otherwise the next pair lists it)
-        const bool end2 = two && bx + 2 == bw;
-        if (i0 == 0 || i1 == 0 || (end2 && i2 == 0)) {
-            const uint32_t t3[3] = {i0, i1, i2};
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-                if (t3[t] == 0 && (t < 2 || end2)) {
-                    const int k = atomicAdd(zn, 1);
-                    if (k < cap) zl[k] = tag | ((uint32_t)by << 16) | (uint32_t)(bx + t);
-                }
-        }
+        zmin = min(zmin, min(i0, i1));
+        zmin = min(zmin, i2);
         const float2 a = __fadd2_rn(make_float2(__int_as_float(i0 | 0x4B000000u),
                                                 __int_as_float(m0 | 0x4B000000u)), ns);
         const float2 b = __fadd2_rn(make_float2(__int_as_float(i1 | 0x4B000000u),
@@ -494,6 +547,8 @@ __device__ __forceinline__ void convert_tile(float4 *__restrict__ dst, int ds,
             ++by;
         }
     }
+    if (__any_sync(0xffffffffu, zmin == 0))
+        list_zeros(rI, nb, bw, bh, zl, zn, cap, tag, lane);
 }
 
 }  // namespace vll
