@@ -1206,6 +1206,85 @@ __device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, int64_t
     }
 }
 
+// ---------------------------------------------------------------------------
+// open slots: those the FP32 pass left without a value, a lane per slot
+// ---------------------------------------------------------------------------
+// Nodes near an image edge, over empty areas or over flat ones leave whole runs
+// of slots without an FP32 value (NaN in the pending buffer).  One warp had to
+// evaluate all of its node's, so the longest node set the exact pass's time
+// (a 100 x 92 grid: 141 us).  They are listed over all queued nodes and
+// evaluated a lane per slot, 32 of a node's neighbouring slots per warp; a
+// listed slot's NaN holds 1 + its place in the list, where the exact pass
+// finds the value.  The list takes the window kernel's per-warp scratch, free
+// by then; slots that find it full are left to the exact pass.
+struct OpenSlots {
+    int64_t *slot;   // [cap] index among the queued nodes * kSlotCap + slot
+    double *rho;     // [cap] eval_slot's value
+    int64_t cap;
+};
+constexpr uint32_t kNanPlace = 0x003FFFFFu;   // payload bits of a quiet NaN
+
+__global__ void __launch_bounds__(128) open_list_kernel(const int32_t *__restrict__ node_k,
+                                                        float *__restrict__ pend_vals,
+                                                        const int64_t *__restrict__ pend_node,
+                                                        const int64_t *__restrict__ pend_off,
+                                                        const OpenSlots L,
+                                                        unsigned long long *__restrict__ ctl) {
+    const int lane = threadIdx.x & 31;
+    const int64_t n = (int64_t)ctl[2];
+    const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t idx = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; idx < n; idx += step) {
+        const int64_t off = pend_off[idx];
+        const int K = node_k[pend_node[idx]];
+        if (off < 0 || K > kSlotCap) continue;
+        for (int k0 = 0; k0 < K; k0 += 32) {
+            const int k = k0 + lane;
+            const bool open = k < K && isnan(pend_vals[off + k]);
+            const uint32_t m = __ballot_sync(0xffffffffu, open);
+            if (!m) continue;
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(&ctl[7], (unsigned long long)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (open && (int64_t)at < L.cap) {
+                L.slot[at] = idx * kSlotCap + k;
+                pend_vals[off + k] = __uint_as_float(0x7FC00000u | (uint32_t)(at + 1));
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(128) open_eval_kernel(const LevelSet LS,
+                                                        const int64_t *__restrict__ pend_node,
+                                                        const OpenSlots L,
+                                                        const double *__restrict__ gsum,
+                                                        const double *__restrict__ gcnt,
+                                                        unsigned long long *__restrict__ counters,
+                                                        const unsigned long long *__restrict__ ctl) {
+    const int64_t n = min((int64_t)ctl[7], L.cap);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = L.slot[i];
+        const int64_t gn = pend_node[e / kSlotCap];
+        const int k = (int)(e % kSlotCap);
+        const int lvl = level_of(LS, gn);
+        const DevLevel &P = LS.lv[lvl];
+        const int64_t pt = gn - __ldg(LS.base + lvl);
+        PatchSrc S, Sn;
+        make_src(P, 1, S, Sn);
+        const float hgt = slot_height(P, P.gp3[pt].minHeight, P.ncc[pt].minHeight, k);
+        const SlotOut o = eval_slot(P, pt, 1, S, Sn, hgt, gcnt ? gcnt[gn] : 0.0, gsum ? gsum[gn] : 0.0);
+        L.rho[i] = o.rho;
+        if (P.dbg_rho && o.evaluated && isnan(P.dbg_rho[P.dbg_off[pt] + k]))
+            P.dbg_rho[P.dbg_off[pt] + k] = o.rho;
+        if (P.vox && !P.cmr && !P.is_ra) {
+            vll_voxel *v = P.vox + P.vox_off[pt] + k;
+            if (o.all_pos) v->flag_cal = 1;
+            v->INCC = q_voxel(o.count_incc > 0 ? __ddiv_rn(o.sum_incc, o.count_incc) : -1.0);
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(&counters[2], (unsigned long long)n);
+}
+
 // The exact pass for the nodes the window kernel could not settle in FP32:
 // the decisions within the error band are re-taken on exact FP64 values of
 // the slots involved (rounds of scan and re-evaluation: a few slots a warp
@@ -1219,8 +1298,8 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
     const LevelSet LS, int max_h, const int32_t *__restrict__ node_k,
     const float *__restrict__ pend_vals, const int64_t *__restrict__ pend_node,
     const int64_t *__restrict__ pend_off, const double *__restrict__ gsum,
-    const double *__restrict__ gcnt, unsigned long long *__restrict__ counters,
-    unsigned long long *__restrict__ ctl) {
+    const double *__restrict__ gcnt, const double *__restrict__ open_rho,
+    unsigned long long *__restrict__ counters, unsigned long long *__restrict__ ctl) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1262,7 +1341,6 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
             W.m.evaluated[lane] = 0;
             W.m.need[lane] = 0;
             W.m.peak[lane] = 0;
-            W.exact[lane] = 0;
         }
         __syncwarp();
         for (int k0 = 0; k0 < K; k0 += 32) {
@@ -1273,10 +1351,15 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
             const bool nd = ev && isnan(v);
             const uint32_t em = __ballot_sync(0xffffffffu, ev);
             const uint32_t nm = __ballot_sync(0xffffffffu, nd);
+            // (an open slot that was listed has its exact value)
+            const uint32_t place = nd ? __float_as_uint(v) & kNanPlace : 0u;
+            const uint32_t xm = __ballot_sync(0xffffffffu, place != 0);
             if (k < K) W.rho[k] = nd ? 0.f : v;
+            if (place) W.xrho[k] = open_rho[place - 1];
             if (lane == 0) {
                 W.m.evaluated[k0 >> 5] = em;
                 W.m.need[k0 >> 5] = nm;
+                W.exact[k0 >> 5] = xm;
             }
         }
         __syncwarp();
@@ -1538,8 +1621,11 @@ cudaError_t launch_window(const DevLevel *hl, int n, const LevelSet &LS, const i
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, window_kernel, kWinWarps * 32, smem);
     if (tu.blocks_per_sm > 0 && tu.blocks_per_sm < per_sm) per_sm = tu.blocks_per_sm;
     per_sm = std::max(1, std::min(per_sm, window_max_blocks_per_sm()));
-    // nodes per queue access (their slot counts are read one per lane)
-    const int grab = tu.grab > 0 ? std::min(tu.grab, 32) : 1;
+    // nodes per queue access (their slot counts are read one per lane): fewer
+    // on small grids, where whole batches would leave warps without a node
+    // (9200 nodes over 1776 warps)
+    const int64_t share = LS.total / (4ll * sms * per_sm * kWinWarps);
+    const int grab = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(tu.grab, 32), share));
     // the warps' slot scratch follows the pending buffer's pend_cap values
     // (window_scratch_floats sizes it for the largest grid)
     float *warp_vals = pend_vals + pend_cap;
@@ -1553,8 +1639,8 @@ cudaError_t launch_window(const DevLevel *hl, int n, const LevelSet &LS, const i
 
 cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
                          const float *pend_vals, const int64_t *pend_node, const int64_t *pend_off,
-                         const double *gsum, const double *gcnt, unsigned long long *counters,
-                         unsigned long long *ctl, cudaStream_t s) {
+                         const double *gsum, const double *gcnt, const double *open_rho,
+                         unsigned long long *counters, unsigned long long *ctl, cudaStream_t s) {
     const size_t ws = (sizeof(WarpShared) + 15) & ~(size_t)15;
     const size_t xs = (exact_scratch_bytes(max_h) + 15) & ~(size_t)15;
     const size_t smem = (ws + xs) * kPeakWarps;
@@ -1568,14 +1654,37 @@ cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
     if (per_sm < 1) per_sm = 1;
     peaks_kernel<<<sms * per_sm, kPeakWarps * 32, smem, s>>>(LS, max_h, node_k, pend_vals,
                                                              pend_node, pend_off, gsum, gcnt,
-                                                             counters, ctl);
+                                                             open_rho, counters, ctl);
+    return cudaGetLastError();
+}
+
+// The open slots of the queued nodes: listed in the window kernel's scratch (at
+// `scratch`) and evaluated.
+cudaError_t launch_open_slots(const LevelSet &LS, const int32_t *node_k, float *pend_vals,
+                              const int64_t *pend_node, const int64_t *pend_off, float *scratch,
+                              const double *gsum, const double *gcnt, double **open_rho,
+                              unsigned long long *counters, unsigned long long *ctl,
+                              cudaStream_t s) {
+    const uintptr_t at = ((uintptr_t)scratch + 15) & ~(uintptr_t)15;
+    OpenSlots L;
+    L.cap = std::min<int64_t>(window_scratch_floats() / 4 - 1, kNanPlace);
+    L.slot = reinterpret_cast<int64_t *>(at);
+    L.rho = reinterpret_cast<double *>(at) + L.cap;
+    *open_rho = L.rho;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    open_list_kernel<<<sms * 8, 128, 0, s>>>(node_k, pend_vals, pend_node, pend_off, L, ctl);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    open_eval_kernel<<<sms * 4, 128, 0, s>>>(LS, pend_node, L, gsum, gcnt, counters, ctl);
     return cudaGetLastError();
 }
 
 // the window and exact stages of the pipeline on given buffers (ctl cleared
 // by the caller: [0] node queue, [1] exact-pass queue, [2] queued nodes,
 // [4] pending-buffer cursor, [5] listed voxel slots, [6] the combined
-// kernel's node queue); plain_k: room for a mixed set's slot counts
+// kernel's node queue, [7] open slots); plain_k: room for a mixed set's slot counts
 cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, const int32_t *node_k,
                              int32_t *plain_k, const double *gsum, const double *gcnt, float *pend_vals,
                              int64_t pend_cap, int64_t *pend_node, int64_t *pend_off,
@@ -1614,8 +1723,12 @@ cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, cons
         cudaEventRecord(tm->ev[5], s);
         cudaEventRecord(tm->ev[6], s);
     }
+    double *open_rho = nullptr;
+    e = launch_open_slots(LS, node_k, pend_vals, pend_node, pend_off, pend_vals + pend_cap, gsum,
+                          gcnt, &open_rho, counters, ctl, s);
+    if (e != cudaSuccess) return e;
     return launch_peaks(LS, set_max_h(hl, n), node_k, pend_vals, pend_node, pend_off, gsum, gcnt,
-                        counters, ctl, s);
+                        open_rho, counters, ctl, s);
 }
 
 // Most window-kernel CTAs an SM can hold whatever the footprint budget (its
@@ -1875,7 +1988,7 @@ cudaError_t split_back(SplitBuffers &b, const DevLevel *hl, int n_levels, const 
         return e;
     }
     const bool plain = any_plain_level(hl, n_levels), combined = any_combined_level(hl, n_levels);
-    *launches += 1 + (plain ? 1 : 0) + (combined ? 1 : 0) + (plain && combined ? 1 : 0) +
+    *launches += 3 + (plain ? 1 : 0) + (combined ? 1 : 0) + (plain && combined ? 1 : 0) +
                  (b.fix_cap > 0 ? 1 : 0);
     mark(7);
     mark(8);
