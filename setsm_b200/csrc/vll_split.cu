@@ -1041,17 +1041,29 @@ __device__ __forceinline__ double slot_value(const WarpShared &w, int k, bool &e
     return ex ? w.xrho[k] : (double)w.rho[k];
 }
 
+// One image's coordinates (full resolution) of a slot by the reference's own
+// RPC order: a chain of some 500 dependent FP64 operations, so callers project
+// their slots side by side, an image of a slot per lane.
+__device__ __forceinline__ double2 project_slot(const DevLevel &P, int64_t pt, float hgt, int image) {
+    const DevImage &im = P.im[image == 0 ? P.ref : 1];
+    return rpc_project(im.rpc, im.adj, P.grid_wgs[2 * pt], P.grid_wgs[2 * pt + 1], (double)hgt);
+}
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
 // Exact FP64 evaluation of one slot by the whole warp, bit-identical with
-// eval_slot (the reference's operation order): lanes 0/1 project into the two
-// images; every lane bilinear-samples its share of the window offsets (each
+// eval_slot (the reference's operation order), from the slot's image
+// coordinates (project_slot): every lane bilinear-samples its share of the window offsets (each
 // sample is computed independently, so this is exact); lanes 0..5 then run
 // the six two-pass Pearson sums (3 sub-windows x {intensity, magnitude}) over
 // the samples in the reference's scan order; lane 0 combines them in
 // ComputeMultiNCC's order.  `scratch` holds (2H+1)^2 x 4 doubles + flags.
 template <int H>
-__device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, const PatchSrc &S,
-                                               const PatchSrc &Sn, float hgt, double cnt_g,
-                                               double sum_g, double *scratch, int lane) {
+__device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, const PatchSrc &S,
+                                               const PatchSrc &Sn, double2 rc, double2 tc,
+                                               double cnt_g, double sum_g, double *scratch,
+                                               int lane) {
     constexpr int D = 2 * H + 1;
     SlotOut o;
     o.evaluated = false;
@@ -1062,14 +1074,6 @@ __device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, co
     o.sum_incc = 0;
     const DevImage &ri = P.im[P.ref];
     const DevImage &tI = P.im[1];
-    const double lon = P.grid_wgs[2 * pt], lat = P.grid_wgs[2 * pt + 1];
-    double2 c = make_double2(0, 0);
-    if (lane < 2) {
-        const DevImage &im = lane == 0 ? ri : tI;
-        c = rpc_project(im.rpc, im.adj, lon, lat, (double)hgt);
-    }
-    const double2 rc = make_double2(__shfl_sync(0xffffffffu, c.x, 0), __shfl_sync(0xffffffffu, c.y, 0));
-    const double2 tc = make_double2(__shfl_sync(0xffffffffu, c.x, 1), __shfl_sync(0xffffffffu, c.y, 1));
     double2 rp = to_pyramid(rc, ri.sx, ri.sy, P.L);
     double2 tp = to_pyramid(tc, tI.sx, tI.sy, P.L);
     if (!(in_image(rp, ri.w, ri.h) && in_image(tp, tI.w, tI.h))) return o;
@@ -1129,21 +1133,23 @@ __device__ __noinline__ SlotOut eval_slot_warp(const DevLevel &P, int64_t pt, co
         if (lane < 6) {
             const int w = lane >> 1, p = lane & 1;
             double Ls = 0, Rs = 0;
+            // (a sample outside the window adds an exact zero: no branch, so the
+            // loads of several samples run ahead of the chain of additions)
+#pragma unroll 8
             for (int idx = 0; idx < D * D; ++idx) {
-                const int f = flag[idx];
-                if (f == 0 || f - 1 < w) continue;
-                Ls = __dadd_rn(Ls, scratch[4 * idx + p]);
-                Rs = __dadd_rn(Rs, scratch[4 * idx + p + 2]);
-                ++n;
+                const bool in = flag[idx] > w;
+                Ls = __dadd_rn(Ls, in ? scratch[4 * idx + p] : 0.0);
+                Rs = __dadd_rn(Rs, in ? scratch[4 * idx + p + 2] : 0.0);
+                n += in ? 1 : 0;
             }
             if (n > 0) {
                 const double Lm = __ddiv_rn(Ls, (double)n), Rm = __ddiv_rn(Rs, (double)n);
                 double slr = 0, sl2 = 0, sr2 = 0;
+#pragma unroll 8
                 for (int idx = 0; idx < D * D; ++idx) {
-                    const int f = flag[idx];
-                    if (f == 0 || f - 1 < w) continue;
-                    const double dl = __dadd_rn(scratch[4 * idx + p], -Lm);
-                    const double dr = __dadd_rn(scratch[4 * idx + p + 2], -Rm);
+                    const bool in = flag[idx] > w;
+                    const double dl = in ? __dadd_rn(scratch[4 * idx + p], -Lm) : 0.0;
+                    const double dr = in ? __dadd_rn(scratch[4 * idx + p + 2], -Rm) : 0.0;
                     slr = __dadd_rn(slr, __dmul_rn(dl, dr));
                     sl2 = __dadd_rn(sl2, __dmul_rn(dl, dl));
                     sr2 = __dadd_rn(sr2, __dmul_rn(dr, dr));
@@ -1192,17 +1198,17 @@ __host__ __device__ constexpr size_t exact_scratch_bytes(int H) {
 }
 
 // Exact FP64 evaluation of one slot by the warp for the level's half-size.
-__device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, int64_t pt,
-                                                      const PatchSrc &S, const PatchSrc &Sn,
-                                                      float hgt, double cnt_g, double sum_g,
+__device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, const PatchSrc &S,
+                                                      const PatchSrc &Sn, double2 rc, double2 tc,
+                                                      double cnt_g, double sum_g,
                                                       double *scratch, int lane) {
     switch (P.H) {
-        case 2: return eval_slot_warp<2>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
-        case 3: return eval_slot_warp<3>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
-        case 4: return eval_slot_warp<4>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
-        case 5: return eval_slot_warp<5>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
-        case 6: return eval_slot_warp<6>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
-        default: return eval_slot_warp<7>(P, pt, S, Sn, hgt, cnt_g, sum_g, scratch, lane);
+        case 2: return eval_slot_warp<2>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
+        case 3: return eval_slot_warp<3>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
+        case 4: return eval_slot_warp<4>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
+        case 5: return eval_slot_warp<5>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
+        case 6: return eval_slot_warp<6>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
+        default: return eval_slot_warp<7>(P, S, Sn, rc, tc, cnt_g, sum_g, scratch, lane);
     }
 }
 
@@ -1392,12 +1398,17 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
             }
             __syncwarp();
             if (n_todo <= kWarpPerSlotMax) {
-                // a few slots: the whole warp per slot
+                // a few slots: the whole warp per slot, all projected at once
+                // (two lanes each)
+                double2 c = make_double2(0, 0);
+                if ((lane >> 1) < n_todo)
+                    c = project_slot(P, pt, slot_height(P, start_H, R.minHeight, W.todo[lane >> 1]),
+                                     lane & 1);
+                __syncwarp();
                 for (int j = 0; j < n_todo; ++j) {
                     const int k = W.todo[j];
-                    const float hh = slot_height(P, start_H, R.minHeight, k);
-                    const SlotOut o = eval_slot_warp_any(P, pt, S, Sn, hh, cnt_g, sum_g,
-                                                        reinterpret_cast<double *>(boxes), lane);
+                    const SlotOut o = eval_slot_warp_any(P, S, Sn, shfl2(c, 2 * j), shfl2(c, 2 * j + 1),
+                                                        cnt_g, sum_g, boxes, lane);
                     if (lane == 0) {
                         if (P.dbg_rho && o.evaluated && isnan(P.dbg_rho[P.dbg_off[pt] + k]))
                             P.dbg_rho[P.dbg_off[pt] + k] = o.rho;
