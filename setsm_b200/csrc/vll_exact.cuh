@@ -12,14 +12,20 @@ struct PatchSrc {
     uint32_t lw, lh, rw, rh;
 };
 
+// Exact double of an unsigned integer by one addition (the conversion
+// instructions run at a fraction of its rate).
+__device__ __forceinline__ double u32_to_double(uint32_t v) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)v), -4503599627370496.0);
+}
+
 // InterpolatePatch, SubFunctions.cpp:3317-3326
 __device__ __forceinline__ double interp(const uint16_t *__restrict__ I, int64_t pos, uint32_t w,
                                          double dx, double dy) {
     const double omx = __dadd_rn(1.0, -dx), omy = __dadd_rn(1.0, -dy);
-    const double t0 = __dmul_rn(__dmul_rn((double)I[pos], omx), omy);
-    const double t1 = __dmul_rn(__dmul_rn((double)I[pos + 1], dx), omy);
-    const double t2 = __dmul_rn(__dmul_rn((double)I[pos + w], omx), dy);
-    const double t3 = __dmul_rn(__dmul_rn((double)I[pos + 1 + w], dx), dy);
+    const double t0 = __dmul_rn(__dmul_rn(u32_to_double(I[pos]), omx), omy);
+    const double t1 = __dmul_rn(__dmul_rn(u32_to_double(I[pos + 1]), dx), omy);
+    const double t2 = __dmul_rn(__dmul_rn(u32_to_double(I[pos + w]), omx), dy);
+    const double t3 = __dmul_rn(__dmul_rn(u32_to_double(I[pos + 1 + w]), dx), dy);
     return __dadd_rn(__dadd_rn(__dadd_rn(t0, t1), t2), t3);
 }
 
@@ -30,10 +36,13 @@ __device__ __forceinline__ bool sample4(const PatchSrc &S, double2 pl, double2 p
           __dadd_rn(pr.x, 1.0) < (double)S.rw && pl.y >= 0 && __dadd_rn(pl.y, 1.0) < (double)S.lh &&
           pl.x >= 0 && __dadd_rn(pl.x, 1.0) < (double)S.lw))
         return false;
-    const int64_t pos = (int64_t)pl.x + (int64_t)pl.y * (int64_t)S.lw;
-    const int64_t posr = (int64_t)pr.x + (int64_t)pr.y * (int64_t)S.rw;
-    const double dx = __dadd_rn(pl.x, -floor(pl.x)), dy = __dadd_rn(pl.y, -floor(pl.y));
-    const double dxr = __dadd_rn(pr.x, -floor(pr.x)), dyr = __dadd_rn(pr.y, -floor(pr.y));
+    // (inside the images: the positions' integer parts are theirs truncated)
+    const uint32_t lx = __double2uint_rz(pl.x), ly = __double2uint_rz(pl.y);
+    const uint32_t rx = __double2uint_rz(pr.x), ry = __double2uint_rz(pr.y);
+    const int64_t pos = (int64_t)lx + (int64_t)ly * (int64_t)S.lw;
+    const int64_t posr = (int64_t)rx + (int64_t)ry * (int64_t)S.rw;
+    const double dx = __dadd_rn(pl.x, -u32_to_double(lx)), dy = __dadd_rn(pl.y, -u32_to_double(ly));
+    const double dxr = __dadd_rn(pr.x, -u32_to_double(rx)), dyr = __dadd_rn(pr.y, -u32_to_double(ry));
     v[0] = interp(S.li, pos, S.lw, dx, dy);
     v[1] = interp(S.lm, pos, S.lw, dx, dy);
     v[2] = interp(S.ri, posr, S.rw, dxr, dyr);

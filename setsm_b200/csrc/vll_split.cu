@@ -1218,11 +1218,12 @@ __device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, const P
 // Nodes near an image edge, over empty areas or over flat ones leave whole runs
 // of slots without an FP32 value (NaN in the pending buffer).  One warp had to
 // evaluate all of its node's, so the longest node set the exact pass's time
-// (a 100 x 92 grid: 141 us).  They are listed over all queued nodes and
+// (a 100 x 90 grid: 141 us).  They are listed over all queued nodes and
 // evaluated a lane per slot, 32 of a node's neighbouring slots per warp; a
 // listed slot's NaN holds 1 + its place in the list, where the exact pass
-// finds the value.  The list takes the window kernel's per-warp scratch, free
-// by then; slots that find it full are left to the exact pass.
+// finds the value.  The list takes what the queued nodes left of the pending
+// buffer and the window kernel's per-warp scratch behind it, free by then;
+// slots that find it full are left to the exact pass.
 struct OpenSlots {
     int64_t *slot;   // [cap] index among the queued nodes * kSlotCap + slot
     double *rho;     // [cap] eval_slot's value
@@ -1230,12 +1231,25 @@ struct OpenSlots {
 };
 constexpr uint32_t kNanPlace = 0x003FFFFFu;   // payload bits of a quiet NaN
 
+// The list's place: `floats` values at pend_vals, of which the queued nodes
+// hold the first ctl[4] (or all of the buffer's pend_cap).
+__device__ __forceinline__ OpenSlots open_slots(float *pend_vals, int64_t pend_cap, int64_t floats,
+                                                const unsigned long long *ctl) {
+    const int64_t used = (min((int64_t)ctl[4], pend_cap) + 3) & ~(int64_t)3;
+    OpenSlots L;
+    L.cap = max((int64_t)0, min((floats - used) / 4, (int64_t)kNanPlace));
+    L.slot = reinterpret_cast<int64_t *>(pend_vals + used);
+    L.rho = reinterpret_cast<double *>(L.slot + L.cap);
+    return L;
+}
+
 __global__ void __launch_bounds__(128) open_list_kernel(const int32_t *__restrict__ node_k,
-                                                        float *__restrict__ pend_vals,
+                                                        float *pend_vals,
                                                         const int64_t *__restrict__ pend_node,
                                                         const int64_t *__restrict__ pend_off,
-                                                        const OpenSlots L,
+                                                        int64_t pend_cap, int64_t floats,
                                                         unsigned long long *__restrict__ ctl) {
+    const OpenSlots L = open_slots(pend_vals, pend_cap, floats, ctl);
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)ctl[2];
     const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1261,11 +1275,13 @@ __global__ void __launch_bounds__(128) open_list_kernel(const int32_t *__restric
 
 __global__ void __launch_bounds__(128) open_eval_kernel(const LevelSet LS,
                                                         const int64_t *__restrict__ pend_node,
-                                                        const OpenSlots L,
+                                                        float *pend_vals, int64_t pend_cap,
+                                                        int64_t floats,
                                                         const double *__restrict__ gsum,
                                                         const double *__restrict__ gcnt,
                                                         unsigned long long *__restrict__ counters,
                                                         const unsigned long long *__restrict__ ctl) {
+    const OpenSlots L = open_slots(pend_vals, pend_cap, floats, ctl);
     const int64_t n = min((int64_t)ctl[7], L.cap);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -1302,10 +1318,10 @@ __global__ void __launch_bounds__(128) open_eval_kernel(const LevelSet LS,
 #endif
 __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
     const LevelSet LS, int max_h, const int32_t *__restrict__ node_k,
-    const float *__restrict__ pend_vals, const int64_t *__restrict__ pend_node,
+    float *pend_vals, int64_t pend_cap, int64_t floats, const int64_t *__restrict__ pend_node,
     const int64_t *__restrict__ pend_off, const double *__restrict__ gsum,
-    const double *__restrict__ gcnt, const double *__restrict__ open_rho,
-    unsigned long long *__restrict__ counters, unsigned long long *__restrict__ ctl) {
+    const double *__restrict__ gcnt, unsigned long long *__restrict__ counters,
+    unsigned long long *__restrict__ ctl) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1315,6 +1331,7 @@ __global__ void __launch_bounds__(kPeakWarps * 32, VLL_PEAK_MINB) peaks_kernel(
     double *boxes = reinterpret_cast<double *>(smem_raw + ws * kPeakWarps + xs * warp);
     unsigned long long rechecks = 0, evals = 0;
     const unsigned long long n_pend = ctl[2];
+    const double *open_rho = open_slots(pend_vals, pend_cap, floats, ctl).rho;
     for (;;) {
         unsigned long long idx = 0;
         if (lane == 0) idx = atomicAdd(&ctl[1], 1ull);
@@ -1649,9 +1666,10 @@ cudaError_t launch_window(const DevLevel *hl, int n, const LevelSet &LS, const i
 }
 
 cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
-                         const float *pend_vals, const int64_t *pend_node, const int64_t *pend_off,
-                         const double *gsum, const double *gcnt, const double *open_rho,
-                         unsigned long long *counters, unsigned long long *ctl, cudaStream_t s) {
+                         float *pend_vals, int64_t pend_cap, int64_t floats,
+                         const int64_t *pend_node, const int64_t *pend_off, const double *gsum,
+                         const double *gcnt, unsigned long long *counters,
+                         unsigned long long *ctl, cudaStream_t s) {
     const size_t ws = (sizeof(WarpShared) + 15) & ~(size_t)15;
     const size_t xs = (exact_scratch_bytes(max_h) + 15) & ~(size_t)15;
     const size_t smem = (ws + xs) * kPeakWarps;
@@ -1664,31 +1682,26 @@ cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, peaks_kernel, kPeakWarps * 32, smem);
     if (per_sm < 1) per_sm = 1;
     peaks_kernel<<<sms * per_sm, kPeakWarps * 32, smem, s>>>(LS, max_h, node_k, pend_vals,
-                                                             pend_node, pend_off, gsum, gcnt,
-                                                             open_rho, counters, ctl);
+                                                             pend_cap, floats, pend_node, pend_off,
+                                                             gsum, gcnt, counters, ctl);
     return cudaGetLastError();
 }
 
-// The open slots of the queued nodes: listed in the window kernel's scratch (at
-// `scratch`) and evaluated.
+// The open slots of the queued nodes: listed and evaluated.
 cudaError_t launch_open_slots(const LevelSet &LS, const int32_t *node_k, float *pend_vals,
-                              const int64_t *pend_node, const int64_t *pend_off, float *scratch,
-                              const double *gsum, const double *gcnt, double **open_rho,
+                              int64_t pend_cap, int64_t floats, const int64_t *pend_node,
+                              const int64_t *pend_off, const double *gsum, const double *gcnt,
                               unsigned long long *counters, unsigned long long *ctl,
                               cudaStream_t s) {
-    const uintptr_t at = ((uintptr_t)scratch + 15) & ~(uintptr_t)15;
-    OpenSlots L;
-    L.cap = std::min<int64_t>(window_scratch_floats() / 4 - 1, kNanPlace);
-    L.slot = reinterpret_cast<int64_t *>(at);
-    L.rho = reinterpret_cast<double *>(at) + L.cap;
-    *open_rho = L.rho;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    open_list_kernel<<<sms * 8, 128, 0, s>>>(node_k, pend_vals, pend_node, pend_off, L, ctl);
+    open_list_kernel<<<sms * 8, 128, 0, s>>>(node_k, pend_vals, pend_node, pend_off, pend_cap,
+                                             floats, ctl);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    open_eval_kernel<<<sms * 4, 128, 0, s>>>(LS, pend_node, L, gsum, gcnt, counters, ctl);
+    open_eval_kernel<<<sms * 4, 128, 0, s>>>(LS, pend_node, pend_vals, pend_cap, floats, gsum, gcnt,
+                                             counters, ctl);
     return cudaGetLastError();
 }
 
@@ -1734,12 +1747,13 @@ cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, cons
         cudaEventRecord(tm->ev[5], s);
         cudaEventRecord(tm->ev[6], s);
     }
-    double *open_rho = nullptr;
-    e = launch_open_slots(LS, node_k, pend_vals, pend_node, pend_off, pend_vals + pend_cap, gsum,
-                          gcnt, &open_rho, counters, ctl, s);
+    // the buffer's values and the warps' scratch behind them
+    const int64_t floats = pend_cap + window_scratch_floats();
+    e = launch_open_slots(LS, node_k, pend_vals, pend_cap, floats, pend_node, pend_off, gsum, gcnt,
+                          counters, ctl, s);
     if (e != cudaSuccess) return e;
-    return launch_peaks(LS, set_max_h(hl, n), node_k, pend_vals, pend_node, pend_off, gsum, gcnt,
-                        open_rho, counters, ctl, s);
+    return launch_peaks(LS, set_max_h(hl, n), node_k, pend_vals, pend_cap, floats, pend_node,
+                        pend_off, gsum, gcnt, counters, ctl, s);
 }
 
 // Most window-kernel CTAs an SM can hold whatever the footprint budget (its
