@@ -988,40 +988,6 @@ __global__ void __launch_bounds__(kWinWarps * 32, VLL_WIN_MINB) window_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// slot fix: exact voxel INCC of the listed slots
-// ---------------------------------------------------------------------------
-// One lane per slot listed by the window kernel (node * kSlotCap + slot):
-// the slot is evaluated in exact FP64 (eval_slot, the reference's operation
-// order) and its voxel's INCC rewritten; the node's other outputs did not
-// depend on the truncation.
-__global__ void __launch_bounds__(128) slot_fix_kernel(const LevelSet LS,
-                                                       const int64_t *__restrict__ fix_list,
-                                                       int64_t fix_cap,
-                                                       const double *__restrict__ gsum,
-                                                       const double *__restrict__ gcnt,
-                                                       const unsigned long long *__restrict__ ctl) {
-    const int64_t n = min((int64_t)ctl[5], fix_cap);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = fix_list[i];
-        const int64_t gn = e / kSlotCap;
-        const int k = (int)(e - gn * kSlotCap);
-        const int lvl = level_of(LS, gn);
-        const DevLevel &P = LS.lv[lvl];
-        const int64_t pt = gn - __ldg(LS.base + lvl);
-        PatchSrc S, Sn;
-        make_src(P, 1, S, Sn);
-        const int start_H = P.gp3[pt].minHeight;
-        const float hgt = slot_height(P, start_H, P.ncc[pt].minHeight, k);
-        const double cnt_g = gcnt ? gcnt[gn] : 0.0, sum_g = gsum ? gsum[gn] : 0.0;
-        const SlotOut o = eval_slot(P, pt, 1, S, Sn, hgt, cnt_g, sum_g);
-        if (o.evaluated)
-            P.vox[P.vox_off[pt] + k].INCC =
-                o.count_incc > 0 ? q_voxel(__ddiv_rn(o.sum_incc, o.count_incc)) : q_voxel(-1.0);
-    }
-}
-
-// ---------------------------------------------------------------------------
 // peak kernel: the exact pass, one warp per queued node
 // ---------------------------------------------------------------------------
 constexpr int kPeakWarps = 4;
@@ -1213,17 +1179,17 @@ __device__ __forceinline__ SlotOut eval_slot_warp_any(const DevLevel &P, const P
 }
 
 // ---------------------------------------------------------------------------
-// open slots: those the FP32 pass left without a value, a lane per slot
+// open slots: those the FP32 pass left without a value
 // ---------------------------------------------------------------------------
 // Nodes near an image edge, over empty areas or over flat ones leave whole runs
 // of slots without an FP32 value (NaN in the pending buffer).  One warp had to
 // evaluate all of its node's, so the longest node set the exact pass's time
 // (a 100 x 90 grid: 141 us).  They are listed over all queued nodes and
-// evaluated a lane per slot, 32 of a node's neighbouring slots per warp; a
-// listed slot's NaN holds 1 + its place in the list, where the exact pass
-// finds the value.  The list takes what the queued nodes left of the pending
-// buffer and the window kernel's per-warp scratch behind it, free by then;
-// slots that find it full are left to the exact pass.
+// evaluated four per warp (listed_slots); a listed slot's NaN holds 1 + its
+// place in the list, where the exact pass finds the value.  The list takes
+// what the queued nodes left of the pending buffer and the window kernel's
+// per-warp scratch behind it, free by then; slots that find it full are left
+// to the exact pass.
 struct OpenSlots {
     int64_t *slot;   // [cap] index among the queued nodes * kSlotCap + slot
     double *rho;     // [cap] eval_slot's value
@@ -1273,38 +1239,248 @@ __global__ void __launch_bounds__(128) open_list_kernel(const int32_t *__restric
     }
 }
 
-__global__ void __launch_bounds__(128) open_eval_kernel(const LevelSet LS,
-                                                        const int64_t *__restrict__ pend_node,
-                                                        float *pend_vals, int64_t pend_cap,
-                                                        int64_t floats,
-                                                        const double *__restrict__ gsum,
-                                                        const double *__restrict__ gcnt,
-                                                        unsigned long long *__restrict__ counters,
-                                                        const unsigned long long *__restrict__ ctl) {
-    const OpenSlots L = open_slots(pend_vals, pend_cap, floats, ctl);
-    const int64_t n = min((int64_t)ctl[7], L.cap);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = L.slot[i];
-        const int64_t gn = pend_node[e / kSlotCap];
-        const int k = (int)(e % kSlotCap);
-        const int lvl = level_of(LS, gn);
-        const DevLevel &P = LS.lv[lvl];
-        const int64_t pt = gn - __ldg(LS.base + lvl);
-        PatchSrc S, Sn;
-        make_src(P, 1, S, Sn);
-        const float hgt = slot_height(P, P.gp3[pt].minHeight, P.ncc[pt].minHeight, k);
-        const SlotOut o = eval_slot(P, pt, 1, S, Sn, hgt, gcnt ? gcnt[gn] : 0.0, gsum ? gsum[gn] : 0.0);
-        L.rho[i] = o.rho;
-        if (P.dbg_rho && o.evaluated && isnan(P.dbg_rho[P.dbg_off[pt] + k]))
-            P.dbg_rho[P.dbg_off[pt] + k] = o.rho;
-        if (P.vox && !P.cmr && !P.is_ra) {
-            vll_voxel *v = P.vox + P.vox_off[pt] + k;
-            if (o.all_pos) v->flag_cal = 1;
-            v->INCC = q_voxel(o.count_incc > 0 ? __ddiv_rn(o.sum_incc, o.count_incc) : -1.0);
+// ---------------------------------------------------------------------------
+// listed slots: exact evaluation, four slots of a level per warp
+// ---------------------------------------------------------------------------
+// Per warp: each of four slots' window samples (intensity pair, magnitude
+// pair) and its 1 + depth flags, zero where there is no sample.
+__host__ __device__ constexpr size_t listed_flags_offset(int H) {
+    return (size_t)4 * (2 * H + 1) * (2 * H + 1) * 4 * sizeof(double);
+}
+__host__ __device__ constexpr size_t listed_scratch_bytes(int H) {
+    return (listed_flags_offset(H) + (size_t)4 * (2 * H + 1) * (2 * H + 1) + 15) & ~(size_t)15;
+}
+
+// The value of every listed slot, bit-identical with eval_slot (the
+// reference's operation order).  A warp projects sixteen slots (an image of a
+// slot per lane) and evaluates four at a time: eight lanes sample a slot's
+// window into shared memory (each sample is independent), then six lanes per
+// slot run its two-pass Pearson sums (3 sub-windows x {intensity, magnitude})
+// in scan order.  A lane per slot had to sample every window twice, in one
+// chain: 1.7 M slots of 11x11 windows 7.0 -> 4.6 ms, 0.66 M of 7x7 1.43 ->
+// 0.86 ms, the few thousand of a 100 x 90 grid 64 -> 38 us.
+//   kFix false: the open slots; slot lists hold an index into pend_node, rho
+//               takes the values;
+//   kFix true:  the voxel slots whose INCC truncation FP32 could not decide;
+//               lists hold the node itself.
+template <bool kFix>
+__device__ __forceinline__ void listed_slots(const LevelSet &LS, int max_h, int64_t n,
+                                             const int64_t *__restrict__ slot,
+                                             const int64_t *__restrict__ pend_node,
+                                             double *__restrict__ rho,
+                                             const double *__restrict__ gsum,
+                                             const double *__restrict__ gcnt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    unsigned char *mine = smem_raw + listed_scratch_bytes(max_h) * (threadIdx.x >> 5);
+    double *smp = reinterpret_cast<double *>(mine);
+    unsigned char *flags = mine + listed_flags_offset(max_h);
+    const int64_t step = (((int64_t)gridDim.x * blockDim.x) >> 5) * 16;
+    for (int64_t i0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 16; i0 < n; i0 += step) {
+        // lane pair: a slot
+        const int64_t e = slot[min(i0 + (lane >> 1), n - 1)];
+        const int k_l = (int)(e % kSlotCap);
+        const int64_t gn_l = kFix ? e / kSlotCap : pend_node[e / kSlotCap];
+        const int lvl_l = level_of(LS, gn_l);
+        double2 c;
+        {
+            const DevLevel &P = LS.lv[lvl_l];
+            const int64_t pt = gn_l - __ldg(LS.base + lvl_l);
+            c = project_slot(P, pt, slot_height(P, P.gp3[pt].minHeight, P.ncc[pt].minHeight, k_l),
+                             lane & 1);
+        }
+        __syncwarp();
+        const int have = (int)min((int64_t)16, n - i0);
+        for (int q0 = 0; q0 < have;) {
+            // up to four slots of one level
+            const int lvl = __shfl_sync(0xffffffffu, lvl_l, 2 * q0);
+            int m = 1;
+            for (int t = 1; t < 4; ++t) {
+                const int lt = __shfl_sync(0xffffffffu, lvl_l, 2 * min(q0 + t, 15));
+                if (m == t && q0 + t < have && lt == lvl) m = t + 1;
+            }
+            const DevLevel &P = LS.lv[lvl];
+            const int H = P.H, D = 2 * H + 1, DD = D * D;
+            const DevImage &ri = P.im[P.ref];
+            const DevImage &tI = P.im[1];
+            // sampling: slot lane / 8 of the four
+            const int u = lane >> 3;
+            const int src = 2 * (q0 + min(u, m - 1));
+            const double2 rc = shfl2(c, src), tc = shfl2(c, src + 1);
+            double2 rp = to_pyramid(rc, ri.sx, ri.sy, P.L);
+            double2 tp = to_pyramid(tc, tI.sx, tI.sy, P.L);
+            bool go = u < m && in_image(rp, ri.w, ri.h) && in_image(tp, tI.w, tI.h);
+            double2 rn = make_double2(0, 0), tn = make_double2(0, 0);
+            if (P.combined_incc) {
+                rn = to_pyramid(rc, ri.sxn, ri.syn, P.L - 1);
+                tn = to_pyramid(tc, tI.sxn, tI.syn, P.L - 1);
+                go = go && in_image(rn, ri.wn, ri.hn) && in_image(tn, tI.wn, tI.hn);
+            }
+            double c0 = 1.0, s0 = 0.0;
+            if (go) {
+                // twice the orientation difference (the sum over both levels
+                // when combined)
+                int twice = (int)ri.ori[(int64_t)(int)rp.y * ri.w + (int)rp.x] -
+                            (int)tI.ori[(int64_t)(int)tp.y * tI.w + (int)tp.x];
+                if (P.combined_incc)
+                    twice += (int)ri.ori_n[(int64_t)(int)rn.y * ri.wn + (int)rn.x] -
+                             (int)tI.ori_n[(int64_t)(int)tn.y * tI.wn + (int)tn.x];
+                else
+                    twice *= 2;
+                c0 = P.rot_cos[twice + kRotOffset];
+                s0 = P.rot_sin[twice + kRotOffset];
+                if (!P.is_ra && P.L >= 3) {
+                    const double a = __dmul_rn(__ddiv_rn((double)twice, 2.0), P.bin_angle);
+                    if (!(a < 90 && a > -90)) go = false;
+                }
+            }
+            const uint32_t gone = __ballot_sync(0xffffffffu, go);
+            PatchSrc S, Sn;
+            make_src(P, 1, S, Sn);
+            // sums: slot lane / 6 of the four, sub-window w, plane p
+            const int q = min(lane / 6, 3), j = lane - 6 * q;
+            const int w = j >> 1, p = j & 1;
+            const bool sums = lane < 24 && ((gone >> (8 * q)) & 1u);
+            double count = 0, sum = 0;
+            bool all_pos0 = false;
+            const int rD = 65536 / D + 1;   // idx / D as a product, exact for idx < D * D
+#pragma unroll 1
+            for (int lev = 0; lev <= (P.combined_incc ? 1 : 0); ++lev) {
+                if (lev) {
+                    rp = rn;
+                    tp = tn;
+                    S = Sn;
+                }
+                if (go) {
+                    for (int idx = lane & 7; idx < DD; idx += 8) {
+                        const int t = (idx * rD) >> 16;
+                        const int row = t - H, col = idx - t * D - H;
+                        const int r2 = row * row + col * col;
+                        unsigned char f = 0;
+                        if (r2 <= (H + 1) * (H + 1)) {
+                            const double ox = __dadd_rn(__dmul_rn(c0, (double)col), -__dmul_rn(s0, (double)row));
+                            const double oy = __dadd_rn(__dmul_rn(s0, (double)col), __dmul_rn(c0, (double)row));
+                            const double2 pl = make_double2(__dadd_rn(rp.x, (double)col),
+                                                            __dadd_rn(rp.y, (double)row));
+                            const double2 pr = make_double2(__dadd_rn(tp.x, ox), __dadd_rn(tp.y, oy));
+                            double v[4];
+                            if (sample4(S, pl, pr, v)) {
+                                f = (unsigned char)(1 + window_depth(H, row, col, r2));
+                                double2 *d = reinterpret_cast<double2 *>(smp + 4 * (u * DD + idx));
+                                d[0] = make_double2(v[0], v[2]);
+                                d[1] = make_double2(v[1], v[3]);
+                            }
+                        }
+                        flags[u * DD + idx] = f;
+                    }
+                }
+                __syncwarp();
+                // Correlate for (w, p), SubFunctions.cpp:974-1018; a sample outside
+                // the window adds an exact zero
+                double r = -99.0;
+                int cnt = 0;
+                if (sums) {
+                    const double2 *d = reinterpret_cast<const double2 *>(smp) + 2 * q * DD + p;
+                    const unsigned char *fl = flags + q * DD;
+                    double Ls = 0, Rs = 0;
+#pragma unroll 4
+                    for (int idx = 0; idx < DD; ++idx) {
+                        const bool in = fl[idx] > w;
+                        const double2 x = d[2 * idx];
+                        Ls = __dadd_rn(Ls, in ? x.x : 0.0);
+                        Rs = __dadd_rn(Rs, in ? x.y : 0.0);
+                        cnt += in ? 1 : 0;
+                    }
+                    if (cnt > 0) {
+                        const double Lm = __ddiv_rn(Ls, (double)cnt), Rm = __ddiv_rn(Rs, (double)cnt);
+                        double slr = 0, sl2 = 0, sr2 = 0;
+#pragma unroll 4
+                        for (int idx = 0; idx < DD; ++idx) {
+                            const bool in = fl[idx] > w;
+                            const double2 x = d[2 * idx];
+                            const double dl = in ? __dadd_rn(x.x, -Lm) : 0.0;
+                            const double dr = in ? __dadd_rn(x.y, -Rm) : 0.0;
+                            slr = __dadd_rn(slr, __dmul_rn(dl, dr));
+                            sl2 = __dadd_rn(sl2, __dmul_rn(dl, dl));
+                            sr2 = __dadd_rn(sr2, __dmul_rn(dr, dr));
+                        }
+                        if (sl2 > 1e-8 && sr2 > 1e-8) r = __ddiv_rn(slr, sqrt(__dmul_rn(sl2, sr2)));
+                    }
+                }
+                __syncwarp();
+                // every lane of the six: its slot's correlations in
+                // ComputeMultiNCC's order
+                double tot = 0, cntv = 0;
+                bool all_pos = true;
+#pragma unroll
+                for (int t = 0; t < 6; ++t) {
+                    const double rt = __shfl_sync(0xffffffffu, r, 6 * q + t);
+                    const int nt = __shfl_sync(0xffffffffu, cnt, 6 * q + t);
+                    all_pos = all_pos && nt > 0;
+                    if (rt != -99.0) {
+                        cntv = __dadd_rn(cntv, 1.0);
+                        tot = __dadd_rn(tot, rt);
+                    }
+                }
+                if (lev == 0) all_pos0 = all_pos;
+                if (all_pos && cntv > 0) {
+                    sum = __dadd_rn(sum, __ddiv_rn(tot, cntv));
+                    count = __dadd_rn(count, 1.0);
+                }
+            }
+            // lane 6 q: the slot's outputs
+            const int from = 2 * (q0 + min(q, m - 1));
+            const int64_t gn = __shfl_sync(0xffffffffu, (long long)gn_l, from);
+            const int k = __shfl_sync(0xffffffffu, k_l, from);
+            if (lane < 24 && j == 0 && q < m) {
+                const int64_t pt = gn - __ldg(LS.base + lvl);
+                const bool evaluated = (gone >> (8 * q)) & 1u;
+                const double cnt_g = gcnt ? gcnt[gn] : 0.0;
+                double v = count > 0 ? __ddiv_rn(sum, count) : -1.0;
+                if (P.vox && !P.cmr && !P.is_ra) {
+                    vll_voxel *x = P.vox + P.vox_off[pt] + k;
+                    if (!kFix && all_pos0) x->flag_cal = 1;
+                    if (!kFix || evaluated) x->INCC = q_voxel(v);
+                }
+                if (evaluated && P.check_ortho && cnt_g > 0)
+                    v = __dadd_rn(__dmul_rn(__ddiv_rn(sum, count), P.alpha),
+                                  __dmul_rn(__ddiv_rn(gsum[gn], cnt_g), P.beta));
+                if (!kFix) {
+                    rho[i0 + q0 + q] = v;
+                    if (P.dbg_rho && evaluated && isnan(P.dbg_rho[P.dbg_off[pt] + k]))
+                        P.dbg_rho[P.dbg_off[pt] + k] = v;
+                }
+            }
+            __syncwarp();
+            q0 += m;
         }
     }
+}
+
+__global__ void __launch_bounds__(128, 3) open_eval_kernel(const LevelSet LS, int max_h,
+                                                           const int64_t *__restrict__ pend_node,
+                                                           float *pend_vals, int64_t pend_cap,
+                                                           int64_t floats,
+                                                           const double *__restrict__ gsum,
+                                                           const double *__restrict__ gcnt,
+                                                           unsigned long long *__restrict__ counters,
+                                                           const unsigned long long *__restrict__ ctl) {
+    const OpenSlots L = open_slots(pend_vals, pend_cap, floats, ctl);
+    const int64_t n = min((int64_t)ctl[7], L.cap);
+    listed_slots<false>(LS, max_h, n, L.slot, pend_node, L.rho, gsum, gcnt);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(&counters[2], (unsigned long long)n);
+}
+
+// Exact voxel INCC of the slots the window kernel listed (node * kSlotCap +
+// slot); the node's other outputs did not depend on the truncation.
+__global__ void __launch_bounds__(128, 3) slot_fix_kernel(const LevelSet LS, int max_h,
+                                                          const int64_t *__restrict__ fix_list,
+                                                          int64_t fix_cap,
+                                                          const double *__restrict__ gsum,
+                                                          const double *__restrict__ gcnt,
+                                                          const unsigned long long *__restrict__ ctl) {
+    listed_slots<true>(LS, max_h, min((int64_t)ctl[5], fix_cap), fix_list, nullptr, nullptr, gsum,
+                       gcnt);
 }
 
 // The exact pass for the nodes the window kernel could not settle in FP32:
@@ -1687,21 +1863,37 @@ cudaError_t launch_peaks(const LevelSet &LS, int max_h, const int32_t *node_k,
     return cudaGetLastError();
 }
 
+// Launch shape of the listed-slot kernels (at most three blocks per SM).
+cudaError_t listed_shape(const void *kernel, int max_h, int *blocks, size_t *smem) {
+    *smem = listed_scratch_bytes(max_h) * 4;
+    cudaError_t e = ensure_smem_limit(kernel, *smem);
+    if (e != cudaSuccess) return e;
+    int dev = 0, sms = 148, per_sm = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, *smem);
+    *blocks = sms * std::max(per_sm, 1);
+    return cudaSuccess;
+}
+
 // The open slots of the queued nodes: listed and evaluated.
-cudaError_t launch_open_slots(const LevelSet &LS, const int32_t *node_k, float *pend_vals,
-                              int64_t pend_cap, int64_t floats, const int64_t *pend_node,
-                              const int64_t *pend_off, const double *gsum, const double *gcnt,
+cudaError_t launch_open_slots(const LevelSet &LS, int max_h, const int32_t *node_k,
+                              float *pend_vals, int64_t pend_cap, int64_t floats,
+                              const int64_t *pend_node, const int64_t *pend_off,
+                              const double *gsum, const double *gcnt,
                               unsigned long long *counters, unsigned long long *ctl,
                               cudaStream_t s) {
-    int dev = 0, sms = 148;
+    int dev = 0, sms = 148, blocks = 0;
+    size_t smem = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     open_list_kernel<<<sms * 8, 128, 0, s>>>(node_k, pend_vals, pend_node, pend_off, pend_cap,
                                              floats, ctl);
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = listed_shape((const void *)open_eval_kernel, max_h, &blocks, &smem);
     if (e != cudaSuccess) return e;
-    open_eval_kernel<<<sms * 4, 128, 0, s>>>(LS, pend_node, pend_vals, pend_cap, floats, gsum, gcnt,
-                                             counters, ctl);
+    open_eval_kernel<<<blocks, 128, smem, s>>>(LS, max_h, pend_node, pend_vals, pend_cap, floats,
+                                               gsum, gcnt, counters, ctl);
     return cudaGetLastError();
 }
 
@@ -1736,10 +1928,12 @@ cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, cons
                             combined_quads(hl, n, tu.box_margin), window_max_blocks_per_sm(), s);
     if (e != cudaSuccess) return e;
     if (fix_cap > 0) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        slot_fix_kernel<<<sms * 8, 128, 0, s>>>(LS, fix_list, fix_cap, gsum, gcnt, ctl);
+        int blocks = 0;
+        size_t smem = 0;
+        const int max_h = set_max_h(hl, n);
+        e = listed_shape((const void *)slot_fix_kernel, max_h, &blocks, &smem);
+        if (e != cudaSuccess) return e;
+        slot_fix_kernel<<<blocks, 128, smem, s>>>(LS, max_h, fix_list, fix_cap, gsum, gcnt, ctl);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1749,8 +1943,8 @@ cudaError_t window_and_peaks(const DevLevel *hl, int n, const LevelSet &LS, cons
     }
     // the buffer's values and the warps' scratch behind them
     const int64_t floats = pend_cap + window_scratch_floats();
-    e = launch_open_slots(LS, node_k, pend_vals, pend_cap, floats, pend_node, pend_off, gsum, gcnt,
-                          counters, ctl, s);
+    e = launch_open_slots(LS, set_max_h(hl, n), node_k, pend_vals, pend_cap, floats, pend_node,
+                          pend_off, gsum, gcnt, counters, ctl, s);
     if (e != cudaSuccess) return e;
     return launch_peaks(LS, set_max_h(hl, n), node_k, pend_vals, pend_cap, floats, pend_node,
                         pend_off, gsum, gcnt, counters, ctl, s);
