@@ -363,13 +363,13 @@ typedef struct vll_level_io {
  * VerticalLineLocus (setsm_code.cpp:6049-6548) on n_levels independent
  * levels -- tiles of one or several scenes, pyramid levels, window sizes --
  * in ONE pass of the split pipeline: one prep pass over all their nodes, ONE
- * persistent window launch draining every level's (node, 32-slot) work items,
- * one peak scan and one exact FP64 pass.  Each level's outputs are exactly
+ * persistent window launch over every level's nodes (32 height slots at a
+ * time) and one exact FP64 pass.  Each level's outputs are exactly
  * those of vll_vertical_line_locus_device on that level alone.  Every level
  * must be one the split kernel implements (stereo, window half-size 2..7);
  * otherwise VLL_ERR_UNSUPPORTED.  Levels matched in combined mode (the
- * next finer level's window added to the INCC, setsm_code.cpp:6378-6464) are
- * evaluated in exact FP64 inside the same launch.  accessable (optional, host, n_levels)
+ * next finer level's window added to the INCC, setsm_code.cpp:6378-6464) have
+ * a launch of their own in the same pass.  accessable (optional, host, n_levels)
  * receives each level's Accessable_grid.  Waits for the GPU.
  */
 int vll_vertical_line_locus_batch(vll_context *ctx, const vll_level_io *levels, int n_levels,

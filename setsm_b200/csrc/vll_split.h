@@ -69,9 +69,8 @@ struct SplitPlan {
 void split_release(SplitBuffers &b);
 
 // Whether the split pipeline implements this level (stereo, no frame sensor,
-// no relative-adjustment mode, H within the compiled window sizes; levels
-// with combined-level INCC are evaluated in FP64 inside it); other levels run
-// the plain FP64 kernel.
+// no relative-adjustment mode, H within the compiled window sizes); other
+// levels run the plain FP64 kernel.
 bool split_supported(const DevLevel &P);
 
 // Encodes the level's TMA tiles (tensor maps of the reference and target

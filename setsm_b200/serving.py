@@ -10,7 +10,7 @@ per-node height ranges.  The server
   keeps the rest waiting in arrival order;
 * hands every idle worker the admitted requests that are ready -- up to
   ``max_batch`` of them -- as ONE batch: one pass of the split pipeline with a
-  single persistent window launch over all the batch's (node, 32-slot) items
+  single persistent window launch over all the batch's nodes
   (``vll_vertical_line_locus_batch``);
 * runs ``n_workers`` workers, each with its own GPU context and stream, so a
   batch formed from requests that arrived while another batch was on the GPU
