@@ -134,7 +134,7 @@ __device__ __forceinline__ double node_y(const DevLevel &P, int64_t row) {
 }
 
 // Boxes of more cells than this are swept by the whole warp, 32 cells at a
-// time; a smaller one by its triangle's own lane.  A TIN of most grid nodes
+// time; a smaller one by its triangle's own lanes.  A TIN of most grid nodes
 // has boxes of 9 to 16 cells, which leave most of a warp idle.
 constexpr int64_t kLaneBox = 48;
 
@@ -155,10 +155,14 @@ __device__ __forceinline__ void cover_cells(const DevLevel &P, const Tri3 &T, co
 }
 
 // The extent of the triangles' vertex heights and, per node inside a
-// triangle, the smallest containing triangle index.  A triangle per lane;
+// triangle, the smallest containing triangle index.  A triangle per kLanes
+// lanes: one where the triangles fill the chip, up to eight where they do not
+// and a lane's chain of FP64 cell tests would set the time (27 k triangles: the
+// points' calls 313 -> 273 us);
 // the extent is reduced per warp before its two atomics (one pair per
 // triangle, all on the same words, took 0.78 of the kernel's 0.87 ms for the
 // 650 k triangles of a 600 x 600 grid, which now takes 0.12).
+template <int kLanes>
 __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__ Pp,
                                                     const vll_point3 *pts, int64_t n_pts,
                                                     const vll_tri *tris, int64_t n_tris,
@@ -170,8 +174,9 @@ __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long zmin = ~0ull, zmax = 0;
     bool any = false;
-    for (int64_t t0 = warp * 32; t0 < n_tris; t0 += n_warps * 32) {
-        const int64_t t = t0 + lane;
+    constexpr int kPer = 32 / kLanes;   // triangles of a warp's step
+    for (int64_t t0 = warp * kPer; t0 < n_tris; t0 += n_warps * kPer) {
+        const int64_t t = t0 + lane / kLanes;
         Tri3 T;
         BBox b{0, 0, -1, -1};
         if (t < n_tris) {
@@ -188,12 +193,13 @@ __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__
         }
         const bool box = b.x1 >= b.x0 && b.y1 >= b.y0;
         const bool large =
-            box && (int64_t)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1) > kLaneBox;
-        if (box && !large) cover_cells(P, T, b, (unsigned int)t, 0, 1, winner);
-        unsigned m = __ballot_sync(0xffffffffu, large);
+            box && (int64_t)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1) > kLaneBox * kLanes;
+        if (box && !large)
+            cover_cells(P, T, b, (unsigned int)t, lane % kLanes, kLanes, winner);
+        unsigned m = __ballot_sync(0xffffffffu, large && lane % kLanes == 0);
         while (m) {
-            // the warp sweeps lane l's box
-            const int l = __ffs(m) - 1;
+            // the warp sweeps the box of lane l's triangle
+            const int l = (__ffs(m) - 1) / kLanes;
             m &= m - 1;
             const vll_tri tr = tris[t0 + l];
             const Tri3 U = tri_of(pts, tr);
@@ -479,10 +485,16 @@ cudaError_t run_height_range(const DevLevel *dP, const DevLevel &hP, const vll_p
     if ((e = cudaMemcpyAsync(hext, hinit, 8, cudaMemcpyHostToDevice, s))) return e;
     if ((e = cudaMemsetAsync(out, 0, N * sizeof(vll_ugrid), s))) return e;
     const RangeArgs a{buffer, th_hg, iteration};
-    if (n_tris > 0)
+    if (n_tris > 0) {
         // (few enough warps that their extent atomics do not count)
-        cover_kernel<<<std::min(blocks_for(n_tris, 128), 148u * 16u), 128, 0, s>>>(
-            dP, pts, n_pts, tris, n_tris, winner, zkey);
+        constexpr int64_t kResident = 148 * 2048;   // threads
+        const int lanes = n_tris * 8 <= kResident ? 8 : n_tris * 4 <= kResident ? 4 : 1;
+        const unsigned blocks = std::min(blocks_for(n_tris * lanes, 128), 148u * 16u);
+        (lanes == 8   ? cover_kernel<8>
+         : lanes == 4 ? cover_kernel<4>
+                      : cover_kernel<1>)<<<blocks, 128, 0, s>>>(dP, pts, n_pts, tris, n_tris, winner,
+                                                                zkey);
+    }
     zext_kernel<<<1, 1, 0, s>>>(zkey, zext);
     node_update_kernel<<<blocks_for(N, 128), 128, 0, s>>>(dP, pts, tris, winner, gp3, newh, mb, a);
     snapshot_kernel<<<blocks_for(N, 256), 256, 0, s>>>(gp3, newh, snap, N);
