@@ -5,17 +5,21 @@
 //   gncc    FP64 GNCC per node (height independent), when the level uses it
 //   prep    per node: image-boundary and blunder tests, the nccresult fields
 //           VerticalLineLocus sets before its height loop, slot count K
-//   scan    exclusive prefix sums -> slot offsets and (node, 32-slot) items
-//   window  persistent kernel draining the item queue: one warp per item,
-//           one lane per height slot.  The RPC numerators / denominators are
+//   scan    exclusive prefix sum of the slot counts
+//   window  persistent kernel draining the node queue: a warp per node, 32
+//           height slots at a time, a lane per slot.  The RPC numerators / denominators are
 //           cubics in the normalised height per node (FP64, Horner), with the
 //           reference-order RPC wherever a coordinate lies within 1e-7 px of
 //           an integer or a clamp, so every integer decision (orientation
 //           pixel, image bounds) equals the reference's.  The warp's window
 //           footprints in both images are staged in shared memory as FP32
 //           texel pairs; bilinear sampling and window sums in FP32, each sum
-//           centred on its window's centre sample -> per-slot rho (float2:
-//           rho, INCC average or NaN when FP32 cannot decide a variance test).
+//           centred on its window's centre sample, then FindPeakNcc streamed
+//           over the slots; a node with a decision inside the error band is
+//           queued with its slots' rho (NaN where FP32 has no value).
+//           Combined levels: vll_combined.cu
+//   open    the queued nodes' NaN slots and the undecided voxel slots, listed
+//           over all nodes, in exact FP64, four slots per warp
 //   peaks   one warp per node: the FindPeakNcc scan, warp-parallel (a slot's
 //           direction and whether its predecessor is a peak depend only on
 //           neighbouring evaluated values); every decision whose FP32 inputs
@@ -596,12 +600,9 @@ __global__ void __launch_bounds__(kWinWarps * 32, VLL_WIN_MINB) window_kernel(
                 }
                 if (K == 0) continue;
                 const int lvl = level_of(LS, gn);
-                if (LS.lv[lvl].combined_incc || K > kSlotCap) {
-                    // combined-level INCC (setsm_code.cpp:6378-6464: the windows at
-                    // this level and the next finer one, the averaged orientation
-                    // and both bounds tests), or a range longer than the slot
-                    // scratch: the node is evaluated wholly in FP64 by the exact
-                    // pass (offset -2: not evaluated yet)
+                if (K > kSlotCap) {
+                    // a range longer than the slot scratch: the node is evaluated
+                    // wholly in FP64 by the exact pass (offset -2: not evaluated yet)
                     if (lane == 0) {
                         const unsigned long long idx = atomicAdd(&ctl[2], 1ull);
                         pend_node[idx] = gn;
