@@ -49,8 +49,8 @@ constexpr int kThreadedCutoff = 100;
 // Nodes of at most this many points are partitioned down to the leaves by one
 // block in shared memory; larger ones a depth at a time over all points.
 constexpr int kBlockPoints = 1024;
-// Up to this many points the three orders are made by counting : three library sorts of so few
-// keys are some forty dependent passes (7500 points: the call
+// Up to this many points the three orders are made by counting: three library
+// sorts of so few keys are some forty dependent passes (7500 points: the call
 // 1288 -> 1100 us, 48 points: 280 -> 241 us; the counting grows with the square).
 constexpr int kRankPoints = 8192;
 constexpr int kRankLanes = 8, kRankTile = 1024;
