@@ -523,13 +523,14 @@ __device__ __forceinline__ void node_end(int64_t pt, NodeState &n, vll_ugrid *go
 
 // Whether a value within `band` of ncc could be rounded or compared otherwise
 // (the blunder pass also returns it as a float, whose last bit a value near 0,
-// a cancellation of the six correlations, does not fix).
+// a cancellation of the correlations it is the mean of, does not fix; the
+// reference's two-pass sums leave 1e-17 where these cancel to 0).
 template <bool kBlunder>
-__device__ __forceinline__ bool near_decision(double ncc, double band) {
+__device__ __forceinline__ bool near_decision(double ncc, bool counted, double band) {
     const double x = ncc * 1000.0;
     bool near = fabs(x - floor(x) - 0.5) <= band * 1000.0;
     if (kBlunder)
-        near = near || (ncc != 0.0 && fabs(ncc) < 1e-4);
+        near = near || (counted && fabs(ncc) < 1e-4);
     else
         near = near || fabs(ncc - 0.3) <= band || fabs(ncc - 0.1) <= band || fabs(ncc - 0.2) <= band;
     return near || !(fabs(ncc) <= 2.0);
@@ -703,9 +704,9 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
             // nested windows: 2 = ring 2; 1 = rings 1 + 2; 0 = all rings
             ring_join(acc[1], acc[2]);
             ring_join(acc[0], acc[1]);
-            double ncc = 0;
+            double ncc = 0, cnt = 0;
             if (acc[0].n > 0 && acc[1].n > 0 && acc[2].n > 0) {
-                double tot = 0, cnt = 0;
+                double tot = 0;
 #pragma unroll
                 for (int w = 0; w < 3; ++w) {
                     const double inv = 1.0 / acc[w].n;
@@ -729,7 +730,7 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                 }
                 if (cnt > 0) ncc = tot / cnt;
             }
-            if (near_decision<kBlunder>(ncc, A.band)) unsure = true;
+            if (near_decision<kBlunder>(ncc, cnt > 0, A.band)) unsure = true;
             node_image<kBlunder>(P, ti, ncc, (int)acc[0].n, st);
         }
         // (any of the node's lanes)
