@@ -597,6 +597,11 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                                                        int64_t *__restrict__ todo,
                                                        unsigned long long *__restrict__ n_todo) {
     __shared__ int2 row_at[128 / kNodeLanes][2 * kMaxSampledH + 1];
+    // A constant area's samples are equal in the fast raster and differ by
+    // rounding (1e-11 at most) in the reference's order, which alone listed
+    // every node over such an area (240 k nodes, two fifths of the images
+    // constant: 1.37 -> 0.39 ms).
+    constexpr double kNone = kBlunder ? 1e-10 : 0.0;
     const DevLevel &P = *Pp;
     const int sub = threadIdx.x & (kNodeLanes - 1);
     int2 *rows = row_at[threadIdx.x / kNodeLanes];
@@ -716,11 +721,11 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                         const double vr = fma(-acc[w].sr[p] * inv, acc[w].sr[p], acc[w].srr[p]);
                         const double cv = fma(-acc[w].sl[p] * inv, acc[w].sr[p], acc[w].slr[p]);
                         // a variance that cancels, or that the sums do not
-                        // decide against 1e-8 (samples all equal to the shift
-                        // have none in any order)
+                        // decide against 1e-8 (squares that add up to kNone
+                        // about the shift have none in any order)
                         const double ql = acc[w].sll[p], qr = acc[w].srr[p];
-                        if ((ql > 0 && vl < fma(1e-3, ql, 1e-4)) ||
-                            (qr > 0 && vr < fma(1e-3, qr, 1e-4)))
+                        if ((ql > kNone && vl < fma(1e-3, ql, 1e-4)) ||
+                            (qr > kNone && vr < fma(1e-3, qr, 1e-4)))
                             unsure = true;
                         if (vl > 1e-8 && vr > 1e-8) {
                             tot += cv / sqrt(vl * vr);

@@ -1,0 +1,52 @@
+"""Calls whose time depends on the inputs' kind and not only on their size:
+each against a call of the same sizes in the same process.  The factors leave
+room for half as much again as measured."""
+import time
+
+import numpy as np
+import pytest
+
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def median_time(call, prepare, n=9):
+    import torch
+    t = []
+    for _ in range(n + 2):
+        args = prepare()
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        call(*args)
+        torch.cuda.synchronize()
+        t.append(time.perf_counter() - t0)
+    return float(np.median(t[2:]))
+
+
+def on_device(inp):
+    import torch
+    io, keep = cases.device_level(torch, inp, inp.new_nccresult())
+    return io[0], keep["gp3"], keep
+
+
+def test_blunder_over_constant_areas(gpu_ctx):
+    """Two fifths of both images constant: at most twice the scene's time
+    (1.1 times as measured; 3.6 when every node there was evaluated exactly)."""
+    import torch
+    times = {}
+    for flat in (False, True):
+        inp = cases.make_variant_case(seed=14, size=768, nodes=360, res=1.0, blunder_level=0)
+        if flat:
+            for im in inp.images:
+                y, x = np.ogrid[:768, :768]
+                m = ((y // 61 * 7 + x // 61 * 13) % 5) < 2
+                im.image_b, im.mag_b = np.where(m, 500, im.image_b).astype(np.uint16), im.mag_b.copy()
+                im.mag_b[m] = 0
+        d, gp3, keep = on_device(inp)
+        out = torch.empty(inp.n, dtype=torch.float32, device="cuda")
+        first = gp3.clone()
+        times[flat] = median_time(
+            lambda g: gpu_ctx.blunder_device(d, g.data_ptr(), 1, False, out.data_ptr()),
+            lambda: (first.clone(),))
+    assert times[True] < 2.0 * times[False], times
