@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
     constexpr double kNone = kBlunder ? 1e-10 : 0.0;
     const DevLevel &P = *Pp;
     const int sub = threadIdx.x & (kNodeLanes - 1);
+    const unsigned group = ((1u << kNodeLanes) - 1u) << ((threadIdx.x & 31) - sub);
     int2 *rows = row_at[threadIdx.x / kNodeLanes];
     const int64_t stride = (int64_t)gridDim.x * (blockDim.x / kNodeLanes);
     const int H = A.H;
@@ -652,13 +653,37 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                 const int64_t a = (int64_t)__ddiv_rn(__dadd_rn(gx, -B[0]), A.im_res);
                 const int64_t b = (int64_t)__ddiv_rn(__dadd_rn(gy, -B[1]), A.im_res);
                 const bool in = a >= 0 && a < A.ow && b >= 0 && b < A.oh;
-                const double2 l = in ? R.ref[b * A.ow + a] : make_double2(0, 0);
-                const double2 r = in ? R.tgt[b * A.ow + a] : make_double2(0, 0);
-                const bool nan = isnan(l.x);
-                sh[0] = nan ? 0.0 : l.x;
-                sh[1] = nan ? 0.0 : l.y;
-                sh[2] = nan ? 0.0 : r.x;
-                sh[3] = nan ? 0.0 : r.y;
+                double2 l = in ? R.ref[b * A.ow + a] : make_double2(nan(""), 0);
+                double2 r = in ? R.tgt[b * A.ow + a] : make_double2(0, 0);
+                const bool none = isnan(l.x);
+                if (none) {
+                    // ... else one of the innermost window's (whose sums would
+                    // cancel about 0 and list every node beside an empty
+                    // area); all of the node's lanes are here
+                    for (int row = -e2; row <= e2 && isnan(l.x); ++row) {
+                        const int2 at_row = rows[row + H];
+                        if (at_row.x < 0) continue;
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j) {
+                            const int c = -H + sub + kNodeLanes * j;
+                            if (!isnan(l.x) || c < -e2 || c > e2 || tc[j] < 0) continue;
+                            const int64_t q = (int64_t)at_row.x * A.ow + tc[j];
+                            l = R.ref[q];
+                            r = R.tgt[q];
+                        }
+                    }
+                    const unsigned have = __ballot_sync(group, !isnan(l.x));
+                    const int src = have ? __ffs(have) - 1 : 0;
+                    l.x = __shfl_sync(group, l.x, src);
+                    l.y = __shfl_sync(group, l.y, src);
+                    r.x = __shfl_sync(group, r.x, src);
+                    r.y = __shfl_sync(group, r.y, src);
+                    if (!have) l = r = make_double2(0, 0);
+                }
+                sh[0] = l.x;
+                sh[1] = l.y;
+                sh[2] = r.x;
+                sh[3] = r.y;
             }
 #pragma unroll 1
             for (int row = -H; row <= H; ++row) {
@@ -739,7 +764,6 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
             node_image<kBlunder>(P, ti, ncc, (int)acc[0].n, st);
         }
         // (any of the node's lanes)
-        const unsigned group = ((1u << kNodeLanes) - 1u) << ((threadIdx.x & 31) - sub);
         unsure = (__ballot_sync(0xffffffffu, unsure) & group) != 0;
         __syncwarp();   // the row indices are rewritten by the next node
         if (live && sub == 0) {
