@@ -679,7 +679,7 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
     const size_t total = (size_t)(ow * oh);
     // a raster of samples per target image, or (large windows) of coordinates
     // per image
-    const bool sampled = vll::ortho_sampled(H);
+    const bool sampled = vll::ortho_sampled(H, d_ncc != nullptr);
     double2 *ptrs[2 * VLL_MAX_IMAGES] = {};
     for (int ti = sampled ? 1 : 0; ti < P.num_images; ++ti) {
         if (!P.im[ti].selected) continue;

@@ -49,10 +49,10 @@ int derive_level(const vll_level_desc *d, DevLevel *P, std::string *err, bool vl
 cudaError_t launch_ortho_raster(const DevLevel *dP, double2 *const *cd, int64_t ow, int64_t oh,
                                 double im_res, int use_b, cudaStream_t s);
 // The same passes over rasters of samples (window half-sizes ortho_sampled
-// accepts): rasters[ti] = ortho_sample_bytes(ow * oh) bytes per selected
+// takes in that pass): rasters[ti] = ortho_sample_bytes(ow * oh) bytes per selected
 // target image (pointers on the host and on the device), scratch of
 // ortho_sampled_scratch(n_nodes) bytes; ncc_out selects the blunder pass.
-bool ortho_sampled(int H);
+bool ortho_sampled(int H, bool blunder);
 size_t ortho_sample_bytes(int64_t total);
 size_t ortho_sampled_scratch(int64_t n_nodes);
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,

@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kw", [
     dict(seed=11, size=512, nodes=40, res=6.0, template=5, blunder_level=1),
+    dict(seed=11, size=512, nodes=40, res=6.0, template=7, blunder_level=1),
     dict(seed=12, size=512, nodes=40, res=6.0, template=11, blunder_level=1),
     dict(seed=13, size=512, nodes=24, res=9.0, template=15, blunder_level=0),
 ])
