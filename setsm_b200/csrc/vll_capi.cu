@@ -677,13 +677,12 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
     const int64_t oh = (int64_t)((P.boundary[3] - P.boundary[1]) / im_res) + 1;
     if (ow <= 0 || oh <= 0) return fail(ctx, VLL_ERR_INVALID, "empty orthoimage boundary");
     const size_t total = (size_t)(ow * oh);
-    // a raster of samples per target image, or (large windows) of coordinates
-    // per image
+    // a raster per image, of its samples or of its coordinates
     const bool sampled = vll::ortho_sampled(H, d_ncc != nullptr);
+    const size_t bytes = total * sizeof(double2);
     double2 *ptrs[2 * VLL_MAX_IMAGES] = {};
-    for (int ti = sampled ? 1 : 0; ti < P.num_images; ++ti) {
-        if (!P.im[ti].selected) continue;
-        const size_t bytes = sampled ? vll::ortho_sample_bytes((int64_t)total) : total * sizeof(double2);
+    for (int ti = 0; ti < P.num_images; ++ti) {
+        if (!P.im[ti].selected || (sampled && ti == 0 && P.ref != 0)) continue;
         VLL_CUDA(ctx, ensure(ctx->ocd[ti], bytes));
         if (!sampled) VLL_CUDA(ctx, cudaMemsetAsync(ctx->ocd[ti].p, 0, bytes, ctx->stream));
         ptrs[ti] = (double2 *)ctx->ocd[ti].p;
@@ -704,8 +703,7 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
     }
     VLL_CUDA(ctx, cudaEventRecord(ctx->e0, ctx->stream));
     if (sampled) {
-        VLL_CUDA(ctx, vll::launch_ortho_sampled(dP, P, P.n_nodes, (void *const *)ptrs,
-                                                (void *const *)dptr, ow, oh, im_res, H,
+        VLL_CUDA(ctx, vll::launch_ortho_sampled(dP, P, P.n_nodes, ptrs, dptr, ow, oh, im_res, H,
                                                 use_b ? 1 : 0, d_gp3, d_ncc, ctx->tin_scratch.p,
                                                 ctx->stream));
     } else {

@@ -49,14 +49,13 @@ int derive_level(const vll_level_desc *d, DevLevel *P, std::string *err, bool vl
 cudaError_t launch_ortho_raster(const DevLevel *dP, double2 *const *cd, int64_t ow, int64_t oh,
                                 double im_res, int use_b, cudaStream_t s);
 // The same passes over rasters of samples (window half-sizes ortho_sampled
-// takes in that pass): rasters[ti] = ortho_sample_bytes(ow * oh) bytes per selected
-// target image (pointers on the host and on the device), scratch of
+// takes in that pass): rasters[ti] = ow * oh double2 of the reference and each
+// selected target image (pointers on the host and on the device), scratch of
 // ortho_sampled_scratch(n_nodes) bytes; ncc_out selects the blunder pass.
 bool ortho_sampled(int H, bool blunder);
-size_t ortho_sample_bytes(int64_t total);
 size_t ortho_sampled_scratch(int64_t n_nodes);
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,
-                                 void *const *h_rasters, void *const *rasters, int64_t ow,
+                                 double2 *const *h_rasters, double2 *const *rasters, int64_t ow,
                                  int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,
                                  float *ncc_out, void *scratch, cudaStream_t s);
 cudaError_t launch_seeddem(const DevLevel *dP, int64_t n_nodes, double2 *const *cd, int64_t ow,

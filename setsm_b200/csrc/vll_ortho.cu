@@ -170,12 +170,12 @@ __global__ void __launch_bounds__(128) blunder_kernel(const DevLevel *__restrict
 // ---- sampled rasters ------------------------------------------------------------
 // A node's window and its neighbours' overlap (a pixel lies in seven windows
 // when the grid is four pixels apart), and a sample depends on its pixel
-// alone, so the raster holds the samples: {reference intensity, reference
-// magnitude, target intensity, target magnitude} of each pixel and target
-// image, NaN first where SetVecKernelValue would drop the pixel.  The node
-// pass is then one pass of sums over rows of pixels, shifted by the centre
-// pixel's samples; FP64, so its NCC is within 1e-12 of the reference's
-// two-pass one for the same samples.
+// alone, so a raster per image holds its samples: {intensity, magnitude} of
+// each pixel, NaN first where SetVecKernelValue would drop the pixel for this
+// image.  The node pass is then one pass of sums over rows of pixels of the
+// reference's and a target's raster, shifted by the centre pixel's samples;
+// FP64, so its NCC is within 1e-12 of the reference's two-pass one for the
+// same samples.
 //
 // kExact samples at the reference's coordinates.  Otherwise the projection
 // uses CUDA's sin, cos and arctangents (the reference's C library rounds
@@ -194,14 +194,10 @@ constexpr double kExactBand = 1e-9;
 constexpr int kMaxSampledH = 15;   // larger windows take the per-node kernels
 constexpr int kNodeLanes = 4;      // lanes per node: columns c = lane (mod 4)
 
-// A raster: total pixels' {intensity, magnitude} of the reference, then
-// total of the target, so that a node's lanes read whole lines of either.
+// The rasters of a pair of images.
 struct Raster {
     const double2 *ref, *tgt;
 };
-__device__ __forceinline__ Raster raster_of(const double2 *base, int64_t total) {
-    return Raster{base, base + total};
-}
 
 // A fast pyramid coordinate of an image of `size` texels: clamped to [0, vmax]
 // like the reference's, scaled and shifted.  `edge`: too close to the clamp,
@@ -217,9 +213,9 @@ __device__ __forceinline__ double fast_bound(double v, double vmax, double inv, 
     return c;
 }
 
-// The RPCs of the reference and one target image as a kernel parameter: their
-// 160 coefficients per pixel come from the constant bank, not through the
-// load pipe, which they kept 75 % busy.
+// The RPCs of two images (or one) as a kernel parameter: their 160
+// coefficients per pixel come from the constant bank, not through the load
+// pipe, which they kept 75 % busy.
 struct PairRpc {
     double rpc[2][90];
     double adj[2][2];
@@ -318,70 +314,71 @@ __device__ __forceinline__ PatchSrc patch_of(const DevLevel &P, int ti, int use_
                  : PatchSrc{ri.img, ri.mag, tI.img, tI.mag, ri.w, ri.h, tI.w, tI.h};
 }
 
-// Bilinear samples of the pair at fast coordinates (sample4's bounds and
-// positivity rules, fused products); `edge`: an intensity so small that the
-// coordinates' error could decide its sign.
-__device__ __forceinline__ bool fast_samples(const PatchSrc &S, double2 pl, double2 pr, double v[4],
-                                             bool &edge) {
-    if (!(pr.y >= 0 && pr.y + 1.0 < (double)S.rh && pr.x >= 0 && pr.x + 1.0 < (double)S.rw &&
-          pl.y >= 0 && pl.y + 1.0 < (double)S.lh && pl.x >= 0 && pl.x + 1.0 < (double)S.lw))
-        return false;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const double2 p = k ? pr : pl;
-        const uint32_t w = k ? S.rw : S.lw;
-        const int xi = (int)p.x, yi = (int)p.y;
-        const double fx = p.x - (double)xi, fy = p.y - (double)yi;
-        const int64_t at = (int64_t)yi * w + xi;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const uint16_t *I = (k ? (c ? S.rm : S.ri) : (c ? S.lm : S.li)) + at;
-            const int a = I[0], b = I[1], d = I[w], e = I[w + 1];
-            const double u = fma(fx, (double)(b - a), (double)a);
-            const double q = fma(fx, (double)(e - d), (double)d);
-            v[2 * k + c] = fma(fy, q - u, u);
-            if (c == 0 && v[2 * k] < 1e-3 && (a | b | d | e)) edge = true;
-        }
-    }
-    return v[0] > 0 && v[2] > 0;
+// An image's planes at the level the pass samples.
+struct Planes {
+    const uint16_t *img, *mag;
+    uint32_t w, h;
+};
+__device__ __forceinline__ Planes planes_of(const DevImage &im, int use_b) {
+    return use_b ? Planes{im.img_b, im.mag_b, im.wb, im.hb} : Planes{im.img, im.mag, im.w, im.h};
 }
 
-// The samples of raster pixel (row, col) at `lonlat` and height h (an
-// uncovered pixel's coordinates are 0), exact or fast.
+// One image's share of sample4: false where it drops the pixel.
+__device__ __forceinline__ bool exact_sample(const Planes &S, double2 p, double v[2]) {
+    if (!(p.y >= 0 && __dadd_rn(p.y, 1.0) < (double)S.h && p.x >= 0 &&
+          __dadd_rn(p.x, 1.0) < (double)S.w))
+        return false;
+    const uint32_t xi = __double2uint_rz(p.x), yi = __double2uint_rz(p.y);
+    const int64_t at = (int64_t)xi + (int64_t)yi * (int64_t)S.w;
+    const double dx = __dadd_rn(p.x, -u32_to_double(xi)), dy = __dadd_rn(p.y, -u32_to_double(yi));
+    v[0] = interp(S.img, at, S.w, dx, dy);
+    v[1] = interp(S.mag, at, S.w, dx, dy);
+    return v[0] > 0;
+}
+
+// The same at fast coordinates (fused products); `edge`: an intensity so small
+// that the coordinates' error could decide its sign.
+__device__ __forceinline__ bool fast_sample(const Planes &S, double2 p, double v[2], bool &edge) {
+    if (!(p.y >= 0 && p.y + 1.0 < (double)S.h && p.x >= 0 && p.x + 1.0 < (double)S.w)) return false;
+    const int xi = (int)p.x, yi = (int)p.y;
+    const double fx = p.x - (double)xi, fy = p.y - (double)yi;
+    const int64_t at = (int64_t)yi * S.w + xi;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const uint16_t *I = (c ? S.mag : S.img) + at;
+        const int a = I[0], b = I[1], d = I[S.w], e = I[S.w + 1];
+        const double u = fma(fx, (double)(b - a), (double)a);
+        const double q = fma(fx, (double)(e - d), (double)d);
+        v[c] = fma(fy, q - u, u);
+        if (c == 0 && v[0] < 1e-3 && (a | b | d | e)) edge = true;
+    }
+    return v[0] > 0;
+}
+
+// The samples of image im (k: its place in R) at a raster pixel's `lonlat` and
+// height h (an uncovered pixel's coordinates are 0), exact or fast.
 template <bool kExact>
-__device__ __forceinline__ bool raster_sample(const DevLevel &P, const PairRpc &R, int use_b, int ti,
-                                              double v[4], double2 lonlat, bool covered, float h,
-                                              bool &edge) {
-    const PatchSrc S = patch_of(P, ti, use_b);
-    double2 pl = make_double2(0, 0), pr = pl;
+__device__ __forceinline__ bool raster_sample(const DevLevel &P, const DevImage &im, const PairRpc &R,
+                                              int k, int use_b, double v[2], double2 lonlat,
+                                              bool covered, float h, bool &edge) {
+    const Planes S = planes_of(im, use_b);
+    double2 p = make_double2(0, 0);
     if (covered) {
         const int lev = use_b ? P.blunder_level : P.L;
-        constexpr int kUnroll = kExact ? 1 : 2;
-#pragma unroll kUnroll
-        for (int k = 0; k < 2; ++k) {
-            const DevImage &im = P.im[k ? ti : P.ref];
-            const double sx = use_b ? im.sxb : im.sx, sy = use_b ? im.syb : im.sy;
-            double2 q;
-            if constexpr (kExact)
-                q = to_pyramid(rpc_project(R.rpc[k], R.adj[k], lonlat.x, lonlat.y, (double)h), sx,
-                               sy, lev);
-            else
-                q = fast_coord(R.rpc[k], R.adj[k], R.inv_scale[k], lonlat.x, lonlat.y, (double)h,
-                               1.0 / (double)(1 << lev), sx, sy, k ? S.rw : S.lw,
-                               k ? S.rh : S.lh, edge);
-            if (k)
-                pr = q;
-            else
-                pl = q;
-        }
+        const double sx = use_b ? im.sxb : im.sx, sy = use_b ? im.syb : im.sy;
+        if constexpr (kExact)
+            p = to_pyramid(rpc_project(R.rpc[k], R.adj[k], lonlat.x, lonlat.y, (double)h), sx, sy, lev);
+        else
+            p = fast_coord(R.rpc[k], R.adj[k], R.inv_scale[k], lonlat.x, lonlat.y, (double)h,
+                           1.0 / (double)(1 << lev), sx, sy, S.w, S.h, edge);
     }
     if constexpr (kExact)
-        return sample4(S, pl, pr, v);
+        return exact_sample(S, p, v);
     else
-        return fast_samples(S, pl, pr, v, edge);
+        return fast_sample(S, p, v, edge);
 }
 
-// A block's raster tile.  Grid columns and rows (two divisions) are found
+// A block's tile of one or two images' rasters.  Grid columns and rows (two divisions) are found
 // once per tile column and row.  The fast projection is evaluated at 3 x 3
 // points of the tile and interpolated quadratically: its third-order term
 // over the tile is below kTileError pixels wherever the tile lies far enough
@@ -390,10 +387,11 @@ __device__ __forceinline__ bool raster_sample(const DevLevel &P, const PairRpc &
 constexpr int kTileW = 32, kTileH = 8;
 constexpr double kTileError = 1e-8;
 
-template <bool kExact>
+template <bool kExact, int kImages>
 __global__ void __launch_bounds__(kTileW * kTileH, kExact ? 4 : 5) sample_raster_kernel(
-    const DevLevel *__restrict__ Pp, const __grid_constant__ PairRpc R, int ti,
-    double2 *__restrict__ out, int64_t ow, int64_t oh, double im_res, int use_b, int64_t tiles_x) {
+    const DevLevel *__restrict__ Pp, const __grid_constant__ PairRpc R, int image0, int image1,
+    double2 *__restrict__ out0, double2 *__restrict__ out1, int64_t ow, int64_t oh, double im_res,
+    int use_b, int64_t tiles_x) {
     __shared__ int at_col[kTileW], at_row[kTileH];
     __shared__ double2 stencil[9];
     const DevLevel &P = *Pp;
@@ -457,15 +455,18 @@ __global__ void __launch_bounds__(kTileW * kTileH, kExact ? 4 : 5) sample_raster
     // a dropped pixel: NaN first; one the fast coordinates do not decide: NaN
     // twice
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    double o[4];
-    bool edge = false;
-    if (!raster_sample<kExact>(P, R, use_b, ti, o, w, covered, h, edge)) {
-        o[0] = nan;
-        o[1] = o[2] = o[3] = 0.0;
+    constexpr int kUnroll = kExact ? 1 : kImages;
+#pragma unroll kUnroll
+    for (int k = 0; k < kImages; ++k) {
+        double o[2];
+        bool edge = false;
+        if (!raster_sample<kExact>(P, P.im[k ? image1 : image0], R, k, use_b, o, w, covered, h, edge)) {
+            o[0] = nan;
+            o[1] = 0.0;
+        }
+        if (edge) o[0] = o[1] = nan;
+        (k ? out1 : out0)[row * ow + col] = make_double2(o[0], o[1]);
     }
-    if (edge) o[0] = o[1] = nan;
-    out[row * ow + col] = make_double2(o[0], o[1]);
-    out[ow * oh + row * ow + col] = make_double2(o[2], o[3]);
 }
 
 // Whether each node's height is set (the window's pixels of the others are
@@ -580,7 +581,7 @@ __device__ __forceinline__ void ring_join(RingSum &a, const RingSum &b) {
 }
 
 struct SampledArgs {
-    const double2 *const *raster;   // [num_images], see Raster
+    const double2 *const *raster;   // [num_images]: the images' samples
     const uint8_t *set;           // node_set_kernel
     int64_t ow, oh;
     double im_res, band;
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
         bool unsure = false;
         for (int ti = 1; ti < P.num_images; ++ti) {
             if (!P.im[ti].selected) continue;
-            const Raster R = raster_of(A.raster[ti], A.ow * A.oh);
+            const Raster R{A.raster[P.ref], A.raster[ti]};
             RingSum acc[3] = {};
             double sh[4];
             {
@@ -655,24 +656,26 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                 const bool in = a >= 0 && a < A.ow && b >= 0 && b < A.oh;
                 double2 l = in ? R.ref[b * A.ow + a] : make_double2(nan(""), 0);
                 double2 r = in ? R.tgt[b * A.ow + a] : make_double2(0, 0);
-                const bool none = isnan(l.x);
+                const bool none = isnan(l.x) || isnan(r.x);
                 if (none) {
                     // ... else one of the innermost window's (whose sums would
                     // cancel about 0 and list every node beside an empty
                     // area); all of the node's lanes are here
-                    for (int row = -e2; row <= e2 && isnan(l.x); ++row) {
+                    bool mine = false;
+                    for (int row = -e2; row <= e2 && !mine; ++row) {
                         const int2 at_row = rows[row + H];
                         if (at_row.x < 0) continue;
 #pragma unroll
                         for (int j = 0; j < NJ; ++j) {
                             const int c = -H + sub + kNodeLanes * j;
-                            if (!isnan(l.x) || c < -e2 || c > e2 || tc[j] < 0) continue;
+                            if (mine || c < -e2 || c > e2 || tc[j] < 0) continue;
                             const int64_t q = (int64_t)at_row.x * A.ow + tc[j];
                             l = R.ref[q];
                             r = R.tgt[q];
+                            mine = !isnan(l.x) && !isnan(r.x);
                         }
                     }
-                    const unsigned have = __ballot_sync(group, !isnan(l.x));
+                    const unsigned have = __ballot_sync(group, mine);
                     const int src = have ? __ffs(have) - 1 : 0;
                     l.x = __shfl_sync(group, l.x, src);
                     l.y = __shfl_sync(group, l.y, src);
@@ -712,8 +715,8 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                     const int ac = c < 0 ? -c : c;
                     const int r2 = row * row + c * c;
                     if (!use[j]) continue;
-                    if (isnan(lo[j].x)) {
-                        if (isnan(lo[j].y)) unsure = true;
+                    if (isnan(lo[j].x) || isnan(hi[j].x)) {
+                        if (isnan(lo[j].y) || isnan(hi[j].y)) unsure = true;
                         continue;
                     }
                     const double d[4] = {lo[j].x - sh[0], lo[j].y - sh[1], hi[j].x - sh[2],
@@ -805,6 +808,7 @@ __global__ void __launch_bounds__(32, 16) exact_node_kernel(const DevLevel *__re
         node_begin<kBlunder>(P, pt, st);
         for (int ti = 1; ti < P.num_images; ++ti) {
             if (!P.im[ti].selected) continue;
+            const PatchSrc S = patch_of(P, ti, A.use_b);
             for (int k = lane; k < 180; k += 32)
                 R.rpc[k / 90][k % 90] = P.im[k < 90 ? P.ref : ti].rpc[k % 90];
             if (lane < 4) R.adj[lane >> 1][lane & 1] = P.im[lane < 2 ? P.ref : ti].adj[lane & 1];
@@ -830,9 +834,19 @@ __global__ void __launch_bounds__(32, 16) exact_node_kernel(const DevLevel *__re
                         const bool covered = pixel_height(P, rX, rY, h);
                         double2 w = make_double2(0, 0);
                         if (covered) w = ps2wgs_dev(P.param, rX, rY);
+                        double2 p[2] = {make_double2(0, 0), make_double2(0, 0)};
+                        if (covered) {
+                            const int lev = A.use_b ? P.blunder_level : P.L;
+#pragma unroll 1
+                            for (int im = 0; im < 2; ++im) {
+                                const DevImage &I = P.im[im ? ti : P.ref];
+                                p[im] = to_pyramid(
+                                    rpc_project(R.rpc[im], R.adj[im], w.x, w.y, (double)h),
+                                    A.use_b ? I.sxb : I.sx, A.use_b ? I.syb : I.sy, lev);
+                            }
+                        }
                         double v[4];
-                        bool edge = false;
-                        if (raster_sample<true>(P, R, A.use_b, ti, v, w, covered, h, edge)) {
+                        if (sample4(S, p[0], p[1], v)) {
                             f = (unsigned char)(1 + window_depth(H, row, col, r2));
 #pragma unroll
                             for (int c = 0; c < 4; ++c) smp[4 * k + c] = v[c];
@@ -903,7 +917,6 @@ unsigned blocks_for(int64_t n, int threads) {
 // hold 9 and 29, and its raster is the cheaper fast one.
 bool ortho_sampled(int H, bool blunder) { return H >= (blunder ? 3 : 1) && H <= kMaxSampledH; }
 
-size_t ortho_sample_bytes(int64_t total) { return (size_t)total * 2 * sizeof(double2); }
 size_t ortho_sampled_scratch(int64_t n_nodes) {
     return (((size_t)n_nodes + 255) & ~(size_t)255) + 256 + (size_t)n_nodes * 8;
 }
@@ -931,7 +944,7 @@ static cudaError_t launch_nodes(const DevLevel *dP, int64_t n, const SampledArgs
 }
 
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,
-                                 void *const *h_rasters, void *const *rasters, int64_t ow,
+                                 double2 *const *h_rasters, double2 *const *rasters, int64_t ow,
                                  int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,
                                  float *ncc_out, void *scratch, cudaStream_t s) {
     uint8_t *set = (uint8_t *)scratch;
@@ -942,25 +955,30 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
     if (e != cudaSuccess) return e;
     const int64_t tx = (ow + kTileW - 1) / kTileW, ty = (oh + kTileH - 1) / kTileH;
     if (tx * ty > 0x7fffffff) return cudaErrorInvalidValue;
-    for (int ti = 1; ti < hP.num_images; ++ti) {
-        if (!hP.im[ti].selected) continue;
+    // the rasters of images a and b (b < 0: of a alone)
+    auto sample = [&](int a, int b) {
         PairRpc R;
         for (int k = 0; k < 2; ++k) {
-            const DevImage &im = hP.im[k ? ti : hP.ref];
+            const DevImage &im = hP.im[k && b >= 0 ? b : a];
             memcpy(R.rpc[k], im.rpc, sizeof(R.rpc[k]));
             memcpy(R.adj[k], im.adj, sizeof(R.adj[k]));
             for (int i = 0; i < 3; ++i) R.inv_scale[k][i] = 1.0 / im.rpc[7 + i];
         }
-        double2 *raster = (double2 *)h_rasters[ti];
         // the blunder pass returns its NCC as a float: it keeps the reference's
         // coordinates, the seed-DEM pass's rounded NCC does not need them
-        if (ncc_out)
-            sample_raster_kernel<true><<<(unsigned)(tx * ty), dim3(kTileW, kTileH), 0, s>>>(
-                dP, R, ti, raster, ow, oh, im_res, use_b, tx);
-        else
-            sample_raster_kernel<false><<<(unsigned)(tx * ty), dim3(kTileW, kTileH), 0, s>>>(
-                dP, R, ti, raster, ow, oh, im_res, use_b, tx);
-    }
+        auto kernel = ncc_out ? (b >= 0 ? sample_raster_kernel<true, 2> : sample_raster_kernel<true, 1>)
+                              : (b >= 0 ? sample_raster_kernel<false, 2> : sample_raster_kernel<false, 1>);
+        kernel<<<(unsigned)(tx * ty), dim3(kTileW, kTileH), 0, s>>>(
+            dP, R, a, b, h_rasters[a], b >= 0 ? h_rasters[b] : nullptr, ow, oh, im_res, use_b, tx);
+    };
+    // a pixel is projected to longitude and latitude once for the reference and
+    // the first target image together
+    int first = -1;
+    for (int ti = 1; ti < hP.num_images && first < 0; ++ti)
+        if (hP.im[ti].selected && ti != hP.ref) first = ti;
+    sample(hP.ref, first);
+    for (int ti = 1; ti < hP.num_images; ++ti)
+        if (hP.im[ti].selected && ti != hP.ref && ti != first) sample(ti, -1);
     node_set_kernel<<<blocks_for(n_nodes, 256), 256, 0, s>>>(dP, set);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
