@@ -705,7 +705,7 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
     if (sampled) {
         VLL_CUDA(ctx, vll::launch_ortho_sampled(dP, P, P.n_nodes, ptrs, dptr, ow, oh, im_res, H,
                                                 use_b ? 1 : 0, d_gp3, d_ncc, ctx->tin_scratch.p,
-                                                ctx->stream));
+                                                &ctx->launches_total, ctx->stream));
     } else {
         VLL_CUDA(ctx, vll::launch_ortho_raster(dP, dptr, ow, oh, im_res, use_b ? 1 : 0,
                                                ctx->stream));
@@ -717,7 +717,7 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
                                               use_b ? 1 : 0, d_gp3, ctx->stream));
     }
     VLL_CUDA(ctx, cudaEventRecord(ctx->e1, ctx->stream));
-    ctx->launches_total += sampled ? 4 : 2;
+    if (!sampled) ctx->launches_total += 2;
     if (stats) {
         VLL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         float ms = 0;

@@ -57,7 +57,8 @@ size_t ortho_sampled_scratch(int64_t n_nodes);
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,
                                  double2 *const *h_rasters, double2 *const *rasters, int64_t ow,
                                  int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,
-                                 float *ncc_out, void *scratch, cudaStream_t s);
+                                 float *ncc_out, void *scratch, int64_t *launches,
+                                 cudaStream_t s);
 cudaError_t launch_seeddem(const DevLevel *dP, int64_t n_nodes, double2 *const *cd, int64_t ow,
                            int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,
                            cudaStream_t s);

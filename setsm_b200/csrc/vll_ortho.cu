@@ -946,7 +946,8 @@ static cudaError_t launch_nodes(const DevLevel *dP, int64_t n, const SampledArgs
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,
                                  double2 *const *h_rasters, double2 *const *rasters, int64_t ow,
                                  int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,
-                                 float *ncc_out, void *scratch, cudaStream_t s) {
+                                 float *ncc_out, void *scratch, int64_t *launches,
+                                 cudaStream_t s) {
     uint8_t *set = (uint8_t *)scratch;
     unsigned long long *n_todo =
         (unsigned long long *)((char *)scratch + (((size_t)n_nodes + 255) & ~(size_t)255));
@@ -970,6 +971,7 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
                               : (b >= 0 ? sample_raster_kernel<false, 2> : sample_raster_kernel<false, 1>);
         kernel<<<(unsigned)(tx * ty), dim3(kTileW, kTileH), 0, s>>>(
             dP, R, a, b, h_rasters[a], b >= 0 ? h_rasters[b] : nullptr, ow, oh, im_res, use_b, tx);
+        ++*launches;
     };
     // a pixel is projected to longitude and latitude once for the reference and
     // the first target image together
@@ -984,6 +986,7 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
     if (e != cudaSuccess) return e;
     const SampledArgs A{(const double2 *const *)rasters, set, ow, oh, im_res, ncc_out ? kExactBand : kFastBand, H,
                         ncc_out ? (H - 1) * (H - 1) : (H + 1) * (H + 1), use_b};
+    *launches += 3;
     return ncc_out ? launch_nodes<true>(dP, n_nodes, A, gout, ncc_out, todo, n_todo, s)
                    : launch_nodes<false>(dP, n_nodes, A, gout, ncc_out, todo, n_todo, s);
 }

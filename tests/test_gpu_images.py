@@ -38,6 +38,18 @@ def test_each_target_is_its_pair(gpu_ctx, name, ref):
     assert np.array_equal(triple.gridpt3["ortho_ncc"][:, 1], pair.gridpt3["ortho_ncc"][:, 1])
 
 
+@pytest.mark.parametrize("name", sorted(PASSES))
+@pytest.mark.parametrize("images,launches", [(2, 4), (3, 5), (5, 7)])
+def test_launches(gpu_ctx, name, images, launches):
+    """A raster launch for the reference and the first target, one for each
+    further target, the flags, the nodes and the listed nodes."""
+    inp = cases.make_variant_case(seed=28, size=512, nodes=32, res=8.0, n_images=3)
+    ims = [inp.images[k] for k in (0, 1, 2, 1, 2)][:images]
+    before = gpu_ctx.launch_count()
+    PASSES[name](gpu_ctx, fresh(inp, ims))
+    assert gpu_ctx.launch_count() - before == launches
+
+
 def test_raster_bytes():
     """Three images of a 2049 x 2049 raster: 3 x 16 bytes per pixel (and less
     than a quarter of one image's for all else)."""
