@@ -688,7 +688,8 @@ int run_ortho_variant(vll_context *ctx, DevLevel &P, vll_ugrid *d_gp3, int H, do
         ptrs[ti] = (double2 *)ctx->ocd[ti].p;
     }
     if (sampled)
-        VLL_CUDA(ctx, ensure(ctx->tin_scratch, vll::ortho_sampled_scratch(P.n_nodes)));
+        VLL_CUDA(ctx, ensure(ctx->tin_scratch,
+                             vll::ortho_sampled_scratch(P.n_nodes, ow, oh, P.num_images)));
     P.gp3 = d_gp3;
     int rc = upload_level_block(ctx, P);
     if (rc) return rc;

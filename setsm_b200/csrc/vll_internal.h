@@ -51,9 +51,9 @@ cudaError_t launch_ortho_raster(const DevLevel *dP, double2 *const *cd, int64_t 
 // The same passes over rasters of samples (window half-sizes ortho_sampled
 // takes in that pass): rasters[ti] = ow * oh double2 of the reference and each
 // selected target image (pointers on the host and on the device), scratch of
-// ortho_sampled_scratch(n_nodes) bytes; ncc_out selects the blunder pass.
+// ortho_sampled_scratch bytes; ncc_out selects the blunder pass.
 bool ortho_sampled(int H, bool blunder);
-size_t ortho_sampled_scratch(int64_t n_nodes);
+size_t ortho_sampled_scratch(int64_t n_nodes, int64_t ow, int64_t oh, int num_images);
 cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t n_nodes,
                                  double2 *const *h_rasters, double2 *const *rasters, int64_t ow,
                                  int64_t oh, double im_res, int H, int use_b, vll_ugrid *gout,

@@ -7,6 +7,8 @@
 // seed-DEM pass widens or voids the node's height range where that NCC is
 // low, the blunder pass records it (ortho_ncc, Mean_ortho_ncc, one float per
 // node).  FP64 in the reference's operation order (compiled -fmad=false).
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -179,18 +181,21 @@ __global__ void __launch_bounds__(128) blunder_kernel(const DevLevel *__restrict
 //
 // kExact samples at the reference's coordinates.  Otherwise the projection
 // uses CUDA's sin, cos and arctangents (the reference's C library rounds
-// correctly) and fused products: coordinates within 1e-8 pixel, which moves
-// the NCC by far less than kFastBand.  Either way a node whose rounding to
-// 1/1000, thresholds or variance tests lie within the band is listed and
-// evaluated again in the reference's order (exact_node_kernel).
+// correctly) and fused products: a coordinate off by up to `delta` pixel (see
+// coord_error), a sample by 2 delta times the largest step between its texels,
+// an NCC by what that is to the window's spread.  The fast raster therefore
+// comes with the largest step of each of its tiles, and a node's band follows
+// from those its window touches.  (One band for all, 2e-7, missed windows that
+// rest on single texels at a corner's tiny weight.)  Either way a node whose
+// rounding to 1/1000, thresholds or variance tests lie within the band is
+// listed and evaluated again in the reference's order (exact_node_kernel).
 //
 // 1024^2 grid, 4097^2 pixels, 11x11 window: 9.85 ms with the samples formed
-// per node and pass (raster 3.8, nodes 6.0), now 2.05 (raster 0.95, nodes 0.98,
-// exact 0.2): the raster is bound by FP64 issue and latency (585 FP64
+// per node and pass (raster 3.8, nodes 6.0), now 2.11 (2.04 with one band for
+// all nodes; raster about 0.95, nodes 0.95, exact 0.2): the raster is bound by FP64 issue and latency (585 FP64
 // instructions per 32 pixels), the node pass by latency at 16 warps per SM (12
 // warps: 2.37 ms in all, 20: 2.54).
-constexpr double kFastBand = 2e-7;
-constexpr double kExactBand = 1e-9;
+constexpr double kSumBand = 1e-9;   // one-pass against two-pass sums of the same samples
 constexpr int kMaxSampledH = 15;   // larger windows take the per-node kernels
 constexpr int kNodeLanes = 4;      // lanes per node: columns c = lane (mod 4)
 
@@ -199,17 +204,19 @@ struct Raster {
     const double2 *ref, *tgt;
 };
 
-// A fast pyramid coordinate of an image of `size` texels: clamped to [0, vmax]
-// like the reference's, scaled and shifted.  `edge`: too close to the clamp,
-// or (unclamped) to the bounds 0 and size - 1, to be trusted with the
-// reference's tests.
+// A fast pyramid coordinate: clamped to [0, vmax] like the reference's, scaled
+// and shifted.  `edge`: too close to the clamp, or (unclamped) to a texel's
+// position, the image's bounds among them, for its error: the reference may
+// sample the other side, whose texels are not among this one's.  near: four
+// times the error.
 constexpr double kPixelEdge = 1e-6;
 __device__ __forceinline__ double fast_bound(double v, double vmax, double inv, double start,
-                                             uint32_t size, bool &edge) {
+                                             double near, bool &edge) {
+    constexpr double kRint = 6755399441055744.0;   // 1.5 * 2^52
     const bool lo = v < 0, hi = v > vmax;
     const double c = fma(lo ? 0.0 : (hi ? vmax : v), inv, -start);
     if (!(fmin(fabs(v), fabs(v - vmax)) > kPixelEdge)) edge = true;
-    if (!(lo || hi) && !(fmin(fabs(c), fabs((double)size - 1.0 - c)) > kPixelEdge)) edge = true;
+    if (!(lo || hi) && !(fabs(c - __dadd_rn(__dadd_rn(c, kRint), -kRint)) > near)) edge = true;
     return c;
 }
 
@@ -233,11 +240,11 @@ __device__ __forceinline__ double fast_recip(double v, bool &edge) {
 }
 
 // GetObjectToImageRPC_single and OriginalToPyramid_single with fused products
-// (see rpc_project, to_pyramid), for the image level of w x h texels.
+// (see rpc_project, to_pyramid).
 __device__ __forceinline__ double2 fast_coord(const double *rpc, const double *adj,
                                               const double *inv_scale, double lon, double lat,
                                               double h, double inv, double sx, double sy,
-                                              uint32_t w, uint32_t hh, bool &edge) {
+                                              double near, bool &edge) {
     double L = (lon - rpc[2]) * inv_scale[0];
     double P = (lat - rpc[3]) * inv_scale[1];
     const double H = (h - rpc[4]) * inv_scale[2];
@@ -260,8 +267,8 @@ __device__ __forceinline__ double2 fast_coord(const double *rpc, const double *a
     const double y = adj[0] + fma(cf[0] * fast_recip(cf[1], edge), rpc[5], rpc[0]);
     const double x = adj[1] + fma(cf[2] * fast_recip(cf[3], edge), rpc[6], rpc[1]);
     return make_double2(
-        fast_bound(x, __dadd_rn(rpc[1], __dmul_rn(rpc[6], 1.2)), inv, sx, w, edge),
-        fast_bound(y, __dadd_rn(rpc[0], __dmul_rn(rpc[5], 1.2)), inv, sy, hh, edge));
+        fast_bound(x, __dadd_rn(rpc[1], __dmul_rn(rpc[6], 1.2)), inv, sx, near, edge),
+        fast_bound(y, __dadd_rn(rpc[0], __dmul_rn(rpc[5], 1.2)), inv, sy, near, edge));
 }
 
 // ps2wgs_single with CUDA's functions (polar stereographic; UTM grids take
@@ -336,9 +343,11 @@ __device__ __forceinline__ bool exact_sample(const Planes &S, double2 p, double 
     return v[0] > 0;
 }
 
-// The same at fast coordinates (fused products); `edge`: an intensity so small
-// that the coordinates' error could decide its sign.
-__device__ __forceinline__ bool fast_sample(const Planes &S, double2 p, double v[2], bool &edge) {
+// The same at fast coordinates (fused products).  step: the largest step
+// between the texels, of each plane; `edge`: an intensity so small that the
+// coordinates' error (see fast_bound) could decide its sign.
+__device__ __forceinline__ bool fast_sample(const Planes &S, double2 p, double v[2], double near,
+                                            unsigned step[2], bool &edge) {
     if (!(p.y >= 0 && p.y + 1.0 < (double)S.h && p.x >= 0 && p.x + 1.0 < (double)S.w)) return false;
     const int xi = (int)p.x, yi = (int)p.y;
     const double fx = p.x - (double)xi, fy = p.y - (double)yi;
@@ -350,7 +359,8 @@ __device__ __forceinline__ bool fast_sample(const Planes &S, double2 p, double v
         const double u = fma(fx, (double)(b - a), (double)a);
         const double q = fma(fx, (double)(e - d), (double)d);
         v[c] = fma(fy, q - u, u);
-        if (c == 0 && v[0] < 1e-3 && (a | b | d | e)) edge = true;
+        step[c] = max(max(a, b), max(d, e)) - min(min(a, b), min(d, e));
+        if (c == 0 && v[0] < near * (double)step[0]) edge = true;
     }
     return v[0] > 0;
 }
@@ -360,7 +370,8 @@ __device__ __forceinline__ bool fast_sample(const Planes &S, double2 p, double v
 template <bool kExact>
 __device__ __forceinline__ bool raster_sample(const DevLevel &P, const DevImage &im, const PairRpc &R,
                                               int k, int use_b, double v[2], double2 lonlat,
-                                              bool covered, float h, bool &edge) {
+                                              bool covered, float h, double near,
+                                              unsigned step[2], bool &edge) {
     const Planes S = planes_of(im, use_b);
     double2 p = make_double2(0, 0);
     if (covered) {
@@ -370,12 +381,12 @@ __device__ __forceinline__ bool raster_sample(const DevLevel &P, const DevImage 
             p = to_pyramid(rpc_project(R.rpc[k], R.adj[k], lonlat.x, lonlat.y, (double)h), sx, sy, lev);
         else
             p = fast_coord(R.rpc[k], R.adj[k], R.inv_scale[k], lonlat.x, lonlat.y, (double)h,
-                           1.0 / (double)(1 << lev), sx, sy, S.w, S.h, edge);
+                           1.0 / (double)(1 << lev), sx, sy, near, edge);
     }
     if constexpr (kExact)
         return exact_sample(S, p, v);
     else
-        return fast_sample(S, p, v, edge);
+        return fast_sample(S, p, v, near, step, edge);
 }
 
 // A block's tile of one or two images' rasters.  Grid columns and rows (two divisions) are found
@@ -390,10 +401,12 @@ constexpr double kTileError = 1e-8;
 template <bool kExact, int kImages>
 __global__ void __launch_bounds__(kTileW * kTileH, kExact ? 4 : 5) sample_raster_kernel(
     const DevLevel *__restrict__ Pp, const __grid_constant__ PairRpc R, int image0, int image1,
-    double2 *__restrict__ out0, double2 *__restrict__ out1, int64_t ow, int64_t oh, double im_res,
-    int use_b, int64_t tiles_x) {
+    double2 *__restrict__ out0, double2 *__restrict__ out1, ushort2 *__restrict__ steps0,
+    ushort2 *__restrict__ steps1, int64_t ow, int64_t oh, double im_res, int use_b,
+    int64_t tiles_x, double near) {
     __shared__ int at_col[kTileW], at_row[kTileH];
     __shared__ double2 stencil[9];
+    __shared__ unsigned tile_step[kImages][2];
     const DevLevel &P = *Pp;
     const int64_t by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
     const int64_t col = bx * kTileW + threadIdx.x, row = by * kTileH + threadIdx.y;
@@ -417,14 +430,17 @@ __global__ void __launch_bounds__(kTileW * kTileH, kExact ? 4 : 5) sample_raster
         const double rho2 = (x0 + sx) * (x0 + sx) + (y0 + sy) * (y0 + sy);
         tiled = P.param.projection == 1 && half2 * sqrt(half2) < kTileError * im_res * rho2;
         const int t = threadIdx.x + kTileW * threadIdx.y - 32;   // the second warp
+        if (t >= 32 && t < 32 + 2 * kImages) tile_step[(t - 32) >> 1][t & 1] = 0;
         if (tiled && t >= 0 && t < 9)
             stencil[t] = ps2wgs_fast(P.param, x0 + (double)(t % 3) * sx, y0 + (double)(t / 3) * sy);
     }
     __syncthreads();
-    if (col >= ow || row >= oh) return;
+    // (every thread of a fast tile takes part in its largest step)
+    const bool live = col < ow && row < oh;
+    if (kExact && !live) return;
     const int gc = at_col[threadIdx.x], gr = at_row[threadIdx.y];
     float h = 0.f;
-    const bool covered = gc >= 0 && gr >= 0 && cell_height(P, gc, gr, h);
+    const bool covered = live && gc >= 0 && gr >= 0 && cell_height(P, gc, gr, h);
     double2 w = make_double2(0, 0);
     if (covered) {
         if constexpr (kExact) {
@@ -459,23 +475,60 @@ __global__ void __launch_bounds__(kTileW * kTileH, kExact ? 4 : 5) sample_raster
 #pragma unroll kUnroll
     for (int k = 0; k < kImages; ++k) {
         double o[2];
+        unsigned step[2] = {0, 0};
         bool edge = false;
-        if (!raster_sample<kExact>(P, P.im[k ? image1 : image0], R, k, use_b, o, w, covered, h, edge)) {
+        if (!raster_sample<kExact>(P, P.im[k ? image1 : image0], R, k, use_b, o, w, covered, h, near,
+                                   step, edge)) {
             o[0] = nan;
             o[1] = 0.0;
         }
         if (edge) o[0] = o[1] = nan;
-        (k ? out1 : out0)[row * ow + col] = make_double2(o[0], o[1]);
+        if (live) (k ? out1 : out0)[row * ow + col] = make_double2(o[0], o[1]);
+        if constexpr (!kExact) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const unsigned m = __reduce_max_sync(0xffffffffu, step[c]);
+                if (threadIdx.x == 0) atomicMax(&tile_step[k][c], m);
+            }
+        }
+    }
+    if constexpr (!kExact) {
+        __syncthreads();
+        if (threadIdx.y == 0 && threadIdx.x < kImages)
+            (threadIdx.x ? steps1 : steps0)[blockIdx.x] =
+                make_ushort2((unsigned short)tile_step[threadIdx.x][0],
+                             (unsigned short)tile_step[threadIdx.x][1]);
     }
 }
 
 // Whether each node's height is set (the window's pixels of the others are
-// dropped).
-__global__ void node_set_kernel(const DevLevel *__restrict__ Pp, uint8_t *__restrict__ set) {
+// dropped), and over fast rasters the largest steps of the tiles around each
+// node's window, of every image sampled (node_steps: [num_images][n_nodes]).
+// (Looked up by the node pass itself they cost it 6 %.)
+__global__ void node_set_kernel(const DevLevel *__restrict__ Pp, uint8_t *__restrict__ set,
+                                const ushort2 *__restrict__ steps, int64_t tiles_x, int64_t n_tiles,
+                                int64_t ow, int64_t oh, double im_res, int H,
+                                ushort2 *__restrict__ node_steps) {
     const DevLevel &P = *Pp;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n_nodes;
-         i += (int64_t)gridDim.x * blockDim.x)
+         i += (int64_t)gridDim.x * blockDim.x) {
         set[i] = P.gp3[i].Height != -1000;
+        if (!node_steps) continue;
+        const int64_t a = (int64_t)((P.grid_pts[2 * i] - P.boundary[0]) / im_res);
+        const int64_t b = (int64_t)((P.grid_pts[2 * i + 1] - P.boundary[1]) / im_res);
+        const int64_t x0 = max(a - H - 1, (int64_t)0) / kTileW, x1 = min(a + H + 1, ow - 1) / kTileW;
+        const int64_t y0 = max(b - H - 1, (int64_t)0) / kTileH, y1 = min(b + H + 1, oh - 1) / kTileH;
+        for (int im = 0; im < P.num_images; ++im) {
+            if (!P.im[im].selected || (im == 0 && P.ref != 0)) continue;
+            ushort2 m = make_ushort2(0, 0);
+            for (int64_t y = y0; y <= y1; ++y)
+                for (int64_t x = x0; x <= x1; ++x) {
+                    const ushort2 t = steps[im * n_tiles + y * tiles_x + x];
+                    m = make_ushort2(max(m.x, t.x), max(m.y, t.y));
+                }
+            node_steps[im * P.n_nodes + i] = m;
+        }
+    }
 }
 
 // What a variant writes from a node's NCC values (VerticalLineLocus_seeddem,
@@ -584,8 +637,11 @@ struct SampledArgs {
     const double2 *const *raster;   // [num_images]: the images' samples
     const uint8_t *set;           // node_set_kernel
     int64_t ow, oh;
-    double im_res, band;
+    double im_res;
     int H, r2max, use_b;
+    // fast rasters: see node_set_kernel; twice the coordinates' error in texels
+    const ushort2 *node_steps;
+    float delta;
 };
 
 // Four lanes per node, each the window columns congruent to it (NJ of them at
@@ -649,6 +705,11 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
             const Raster R{A.raster[P.ref], A.raster[ti]};
             RingSum acc[3] = {};
             double sh[4];
+            ushort2 step[2];
+            if constexpr (!kBlunder) {
+                step[0] = A.node_steps[P.ref * P.n_nodes + pt];
+                step[1] = A.node_steps[ti * P.n_nodes + pt];
+            }
             {
                 // the shift: the pixel of the node itself, where it has samples
                 const int64_t a = (int64_t)__ddiv_rn(__dadd_rn(gx, -B[0]), A.im_res);
@@ -737,12 +798,14 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
             // nested windows: 2 = ring 2; 1 = rings 1 + 2; 0 = all rings
             ring_join(acc[1], acc[2]);
             ring_join(acc[0], acc[1]);
-            double ncc = 0, cnt = 0;
+            double ncc = 0, cnt = 0, band = kSumBand;
             if (acc[0].n > 0 && acc[1].n > 0 && acc[2].n > 0) {
                 double tot = 0;
+                float err = 0.f;
 #pragma unroll
                 for (int w = 0; w < 3; ++w) {
                     const double inv = 1.0 / acc[w].n;
+                    const float root_n = sqrtf((float)acc[w].n);
 #pragma unroll
                     for (int p = 0; p < 2; ++p) {
                         const double vl = fma(-acc[w].sl[p] * inv, acc[w].sl[p], acc[w].sll[p]);
@@ -756,14 +819,30 @@ __global__ void __launch_bounds__(128, NJ <= 4 ? 4 : 2) node_ncc_kernel(const De
                             (qr > kNone && vr < fma(1e-3, qr, 1e-4)))
                             unsure = true;
                         if (vl > 1e-8 && vr > 1e-8) {
-                            tot += cv / sqrt(vl * vr);
+                            const double rho = cv / sqrt(vl * vr);
+                            tot += rho;
                             cnt += 1.0;
+                            if constexpr (!kBlunder) {
+                                // samples off by `delta` steps turn the vectors
+                                // by at most x in all, the correlation (a
+                                // cosine) by x times its sine and x^2
+                                const float x = A.delta * root_n *
+                                                ((float)(p ? step[0].y : step[0].x) *
+                                                     rsqrtf((float)vl) +
+                                                 (float)(p ? step[1].y : step[1].x) *
+                                                     rsqrtf((float)vr));
+                                const float c = (float)rho;
+                                err += x * (sqrtf(fmaxf(fmaf(-c, c, 1.f), 0.f)) + 2.f * x);
+                            }
                         }
                     }
                 }
-                if (cnt > 0) ncc = tot / cnt;
+                if (cnt > 0) {
+                    ncc = tot / cnt;
+                    if constexpr (!kBlunder) band += (double)err / cnt;
+                }
             }
-            if (near_decision<kBlunder>(ncc, cnt > 0, A.band)) unsure = true;
+            if (near_decision<kBlunder>(ncc, cnt > 0, band)) unsure = true;
             node_image<kBlunder>(P, ti, ncc, (int)acc[0].n, st);
         }
         // (any of the node's lanes)
@@ -917,8 +996,29 @@ unsigned blocks_for(int64_t n, int threads) {
 // hold 9 and 29, and its raster is the cheaper fast one.
 bool ortho_sampled(int H, bool blunder) { return H >= (blunder ? 3 : 1) && H <= kMaxSampledH; }
 
-size_t ortho_sampled_scratch(int64_t n_nodes) {
-    return (((size_t)n_nodes + 255) & ~(size_t)255) + 256 + (size_t)n_nodes * 8;
+static int64_t raster_tiles(int64_t ow, int64_t oh) {
+    return ((ow + kTileW - 1) / kTileW) * ((oh + kTileH - 1) / kTileH);
+}
+size_t ortho_sampled_scratch(int64_t n_nodes, int64_t ow, int64_t oh, int num_images) {
+    return (((size_t)n_nodes + 255) & ~(size_t)255) + 256 + (size_t)n_nodes * 8 +
+           (size_t)num_images * (raster_tiles(ow, oh) + n_nodes) * sizeof(ushort2);
+}
+
+// The fast coordinates' distance from the reference's in texels: the map
+// projection's rounding (5e-9 m; 3.6e-9 m at most over 670 million points to
+// 4000 km from either pole), and the third-order term of a tile's quadratic
+// interpolation, which sample_raster_kernel keeps below kTileError pixels of
+// the raster and which falls with the square of the distance to the pole.
+static double coord_error(const DevLevel &P, double im_res, int use_b) {
+    const double hx = 0.5 * (kTileW - 1) * im_res, hy = 0.5 * (kTileH - 1) * im_res;
+    const double half2 = hx * hx + hy * hy;
+    const double *B = P.boundary;
+    const double dx = std::max(std::max(B[0], -B[2]), 0.0), dy = std::max(std::max(B[1], -B[3]), 0.0);
+    const double rho2 = dx * dx + dy * dy;
+    double tile = kTileError * im_res;
+    if (rho2 > 0) tile = std::min(tile, half2 * sqrt(half2) / rho2);
+    const double texel = P.im_res / (double)(1 << P.L) * (double)(1 << (use_b ? P.blunder_level : P.L));
+    return (5e-9 + tile) / texel;
 }
 
 // The node pass of one variant over its sampled raster.
@@ -954,8 +1054,10 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
     int64_t *todo = (int64_t *)((char *)n_todo + 256);
     cudaError_t e = cudaMemsetAsync(n_todo, 0, 8, s);
     if (e != cudaSuccess) return e;
-    const int64_t tx = (ow + kTileW - 1) / kTileW, ty = (oh + kTileH - 1) / kTileH;
-    if (tx * ty > 0x7fffffff) return cudaErrorInvalidValue;
+    const int64_t tx = (ow + kTileW - 1) / kTileW, tiles = raster_tiles(ow, oh);
+    ushort2 *steps = (ushort2 *)(todo + n_nodes), *node_steps = steps + hP.num_images * tiles;
+    const double delta = coord_error(hP, im_res, use_b);
+    if (tiles > 0x7fffffff) return cudaErrorInvalidValue;
     // the rasters of images a and b (b < 0: of a alone)
     auto sample = [&](int a, int b) {
         PairRpc R;
@@ -969,8 +1071,9 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
         // coordinates, the seed-DEM pass's rounded NCC does not need them
         auto kernel = ncc_out ? (b >= 0 ? sample_raster_kernel<true, 2> : sample_raster_kernel<true, 1>)
                               : (b >= 0 ? sample_raster_kernel<false, 2> : sample_raster_kernel<false, 1>);
-        kernel<<<(unsigned)(tx * ty), dim3(kTileW, kTileH), 0, s>>>(
-            dP, R, a, b, h_rasters[a], b >= 0 ? h_rasters[b] : nullptr, ow, oh, im_res, use_b, tx);
+        kernel<<<(unsigned)tiles, dim3(kTileW, kTileH), 0, s>>>(
+            dP, R, a, b, h_rasters[a], b >= 0 ? h_rasters[b] : nullptr, steps + a * tiles,
+            steps + (b >= 0 ? b : a) * tiles, ow, oh, im_res, use_b, tx, 4.0 * delta);
         ++*launches;
     };
     // a pixel is projected to longitude and latitude once for the reference and
@@ -981,11 +1084,13 @@ cudaError_t launch_ortho_sampled(const DevLevel *dP, const DevLevel &hP, int64_t
     sample(hP.ref, first);
     for (int ti = 1; ti < hP.num_images; ++ti)
         if (hP.im[ti].selected && ti != hP.ref && ti != first) sample(ti, -1);
-    node_set_kernel<<<blocks_for(n_nodes, 256), 256, 0, s>>>(dP, set);
+    node_set_kernel<<<blocks_for(n_nodes, 256), 256, 0, s>>>(
+        dP, set, steps, tx, tiles, ow, oh, im_res, H, ncc_out ? nullptr : node_steps);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const SampledArgs A{(const double2 *const *)rasters, set, ow, oh, im_res, ncc_out ? kExactBand : kFastBand, H,
-                        ncc_out ? (H - 1) * (H - 1) : (H + 1) * (H + 1), use_b};
+    const SampledArgs A{(const double2 *const *)rasters, set, ow, oh, im_res, H,
+                        ncc_out ? (H - 1) * (H - 1) : (H + 1) * (H + 1), use_b, node_steps,
+                        (float)(2.0 * delta)};
     *launches += 3;
     return ncc_out ? launch_nodes<true>(dP, n_nodes, A, gout, ncc_out, todo, n_todo, s)
                    : launch_nodes<false>(dP, n_nodes, A, gout, ncc_out, todo, n_todo, s);
