@@ -155,14 +155,19 @@ struct TriBox {
     bool listed;
 };
 
-// Screened correlations lie within kScreenBand of the exact ones: the
-// coordinates come from FP64 cubics (1e-10 pixel), the plane's height from
-// the triangle's linear form (the reference's plane equation at coordinates
-// of 10^6 m is off by 1e-9 m over the plane's |C|, which is kept above
-// kMinC), the sums from one FP64 pass over samples shifted by the first.
+// A screened correlation comes with a bound on its distance from the exact
+// one.  The coordinates come from FP64 cubics (kCubicError pixel), the plane's
+// height from the triangle's linear form, which the reference's plane equation
+// differs from by its rounding at coordinates of 10^6 m over the plane's |C|
+// (kept above kMinC; see plane_error).  What that is to the correlation follows
+// from the steps between the texels against the samples' spread
+// (ScreenAcc::corr): little for ordinary texture, 1e-5 and more for a steep
+// triangle's few samples beside a bright texel.  kScreenBand covers the rest:
+// one FP64 pass of sums over samples shifted by the first, and the float.
 constexpr double kScreenBand = 1e-6;
 constexpr double kMinC = 1e-2;
-constexpr double kCoordEdge = 1e-6;   // coordinate distance to an image bound left to the exact pass
+constexpr double kCubicError = 2e-9;
+constexpr double kCoordEdge = 1e-6;   // coordinate distance to a clamp left to the exact pass
 
 // 1 / v from an FP32 seed and two Newton steps; `edge` is set where the seed
 // is no finite non-zero float.
@@ -208,14 +213,17 @@ __device__ void screen_poly(const double *rpc, double lon, double lat, int j0, d
 // One pyramid coordinate from the scaled ratio v (clamped to [0, vmax] like
 // the reference's) and whether it lies in an image of `size` texels (0 <= c,
 // c + 1 < size).  `edge`: v lies too close to a clamp, or the unclamped
-// coordinate to a bound, for the cubics to decide (a clamped one is exact).
+// coordinate within `near` (four errors) of a texel's position, the bounds
+// among them, for the cubics to decide (a clamped one is exact).
 __device__ __forceinline__ double screen_bound(double v, double vmax, double inv_s, double start,
-                                               uint32_t size, bool &in, bool &edge) {
+                                               uint32_t size, float near, bool &in,
+                                               bool &edge) {
+    constexpr double kRint = 6755399441055744.0;   // 1.5 * 2^52
     const bool lo = v < 0, hi = v > vmax;
     const double c = fma(lo ? 0.0 : (hi ? vmax : v), inv_s, -start);
     const double last = (double)size - 1.0;
     if (!(fmin(fabs(v), fabs(v - vmax)) > kCoordEdge)) edge = true;
-    if (!(lo || hi) && !(fmin(fabs(c), fabs(last - c)) > kCoordEdge)) edge = true;
+    if (!(lo || hi) && !(fabs(c - __dadd_rn(__dadd_rn(c, kRint), -kRint)) > (double)near)) edge = true;
     in = in && c >= 0 && c < last;
     return c;
 }
@@ -223,7 +231,8 @@ __device__ __forceinline__ double screen_bound(double v, double vmax, double inv
 // Pyramid coordinate of a screened cell at height z.
 __device__ __forceinline__ double2 screen_coord(const double (*a)[4], const DevImage &im,
                                                 const double *adj, double z, double hoff,
-                                                double hinv, double inv_s, bool &in, bool &edge) {
+                                                double hinv, double inv_s, float near, bool &in,
+                                                bool &edge) {
     const double H = (z - hoff) * hinv;
     double v[4];
 #pragma unroll
@@ -232,12 +241,14 @@ __device__ __forceinline__ double2 screen_coord(const double (*a)[4], const DevI
     const double x = adj[1] + fma(v[2] * screen_rcp(v[3], edge), im.rpc[6], im.rpc[1]);
     const double ymax = __dadd_rn(im.rpc[0], __dmul_rn(im.rpc[5], 1.2));
     const double xmax = __dadd_rn(im.rpc[1], __dmul_rn(im.rpc[6], 1.2));
-    return make_double2(screen_bound(x, xmax, inv_s, im.sx, im.w, in, edge),
-                        screen_bound(y, ymax, inv_s, im.sy, im.h, in, edge));
+    return make_double2(screen_bound(x, xmax, inv_s, im.sx, im.w, near, in, edge),
+                        screen_bound(y, ymax, inv_s, im.sy, im.h, near, in, edge));
 }
 
-// Bilinear samples of both planes of an image at (x, y), inside its bounds.
-__device__ __forceinline__ double2 screen_sample(const DevImage &im, double x, double y) {
+// Bilinear samples of both planes of an image at (x, y), inside its bounds;
+// step: raised to the largest step between the texels, of each plane.
+__device__ __forceinline__ double2 screen_sample(const DevImage &im, double x, double y,
+                                                 int (&step)[2]) {
     const int xi = __double2int_rd(x), yi = __double2int_rd(y);
     const double fx = x - (double)xi, fy = y - (double)yi;
     const int64_t p = (int64_t)yi * im.w + xi;
@@ -249,6 +260,7 @@ __device__ __forceinline__ double2 screen_sample(const DevImage &im, double x, d
         const double t = fma(fx, (double)(b - a), (double)a);
         const double u = fma(fx, (double)(d - c), (double)c);
         r[k] = fma(fy, u - t, t);
+        step[k] = max(step[k], max(max(a, b), max(c, d)) - min(min(a, b), min(c, d)));
     }
     return make_double2(r[0], r[1]);
 }
@@ -262,36 +274,65 @@ struct ScreenAcc {
         srr = fma(r, r, srr);
         slr = fma(l, r, slr);
     }
-    // Correlate's value; a variance whose 1e-8 test the sums do not decide
-    // sets `unsure`
-    __device__ double corr(double n, bool &unsure) const {
+    // Correlate's value and in `off` what the coordinates' error can move it by:
+    // samples off by 2 delta steps each (err: that times the root of their
+    // number) turn the vectors by at most x in all, the correlation by x
+    // times its sine and x^2.  A variance whose 1e-8 test the sums do not
+    // decide, and an x that is not small, set `unsure`.
+    __device__ double corr(double n, float err, int step, float &off,
+                           bool &unsure) const {
         const double inv = 1.0 / n;
         const double vl = fma(-sl * inv, sl, sll), vr = fma(-sr * inv, sr, srr);
         const double cv = fma(-sl * inv, sr, slr);
         if ((vl > 1e-11 && vl < 1e-5) || (vr > 1e-11 && vr < 1e-5)) unsure = true;
         if (!(vl > 1e-8 && vr > 1e-8)) return -99.0;
-        return cv / sqrt(vl * vr);
+        const double r = cv / sqrt(vl * vr);
+        const float x = err * (float)step * (rsqrtf((float)vl) + rsqrtf((float)vr));
+        const float c = (float)r;
+        if (!(x < 0.1f)) unsure = true;
+        off = x * (sqrtf(fmaxf(fmaf(-c, c, 1.f), 0.f)) + 2.f * x);
+        return r;
     }
 };
 
+// What the reference's plane equation (exact_height) may differ from the
+// triangle's linear form by, in metres of height: nine roundings of its terms,
+// of the size of the coordinates, over |C|, and of the normal, which a thin
+// triangle magnifies, over the triangle.  len: the normal's length, den: its
+// vertical component.
+__device__ __forceinline__ double plane_error(const P3 &r1, double v12x, double v12y, double v12z,
+                                              double v13x, double v13y, double v13z, double den,
+                                              double len) {
+    const double a = sqrt(v12x * v12x + v12y * v12y + v12z * v12z);
+    const double b = sqrt(v13x * v13x + v13y * v13y + v13z * v13z);
+    return 1e-15 * (fabs(r1.x) + fabs(r1.y) + fabs(r1.z) + (a + b) * (a * b / len)) * len / fabs(den);
+}
+
 // The correlation of the triangle at one height per thread: the mean over the
-// target images and, in *avg, the mean number of samples; NaN where the
-// screen does not decide it.  Every thread of the block takes part.
+// target images, in *band the bound on its error and in *avg the mean number
+// of samples; NaN where the screen does not decide it.  Every thread of the
+// block takes part.
 __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ lonlat,
-                                const TriBox &T, double hgt, bool live, int *avg, CellStage &st) {
+                                const TriBox &T, double hgt, bool live, int *avg, float *band,
+                                CellStage &st) {
     const int lane = threadIdx.x & 31;
     const double v12x = T.r2.x - T.r1.x, v12y = T.r2.y - T.r1.y, v12z = T.r2.z - T.r1.z;
     const double v13x = T.tg.x - T.r1.x, v13y = T.tg.y - T.r1.y, v13z = hgt - T.r1.z;
     const double den = v12x * v13y - v12y * v13x;
     bool unsure = !live;
+    float delta;   // the coordinates' error in texels
     {
         const double nx = v12y * v13z - v12z * v13y, ny = v12z * v13x - v12x * v13z;
         const double len = sqrt(nx * nx + ny * ny + den * den);
-        if (!(fabs(den) > kMinC * len)) unsure = true;
+        // (a metre of height is at most a metre on the ground)
+        const double e = plane_error(T.r1, v12x, v12y, v12z, v13x, v13y, v13z, den, len) / P.im_res;
+        if (!(fabs(den) > kMinC * len) || !(e < 0.25 * kCoordEdge)) unsure = true;
+        delta = (float)(kCubicError + e);
     }
     const double inv_s = 1.0 / (double)(1 << P.L);
     const DevImage &ri = P.im[P.ref];
     double sum_ncc = 0;
+    float sum_off = 0.f;
     int n_img = 0, n_sum = 0;
     for (int ti = 1; ti < P.num_images; ++ti) {
         const DevImage &tI = P.im[ti];
@@ -300,6 +341,7 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
         ScreenAcc acc[2];
         acc[0] = acc[1] = ScreenAcc{0, 0, 0, 0, 0};
         double2 s0 = make_double2(0, 0), s1 = make_double2(0, 0);
+        int step[2] = {0, 0};   // of both images (a pair of registers less)
         int n = 0;
         const int64_t items = T.listed ? T.n_in : T.ncell;
         for (int64_t base = 0; base < items; base += 32) {
@@ -340,13 +382,15 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
                 const ScreenCell &S = st.sc[c];
                 const double z = fma(hgt, S.z1, S.z0);
                 bool in = true, edge = false;
-                const double2 rp = screen_coord(S.c[0], ri, ri.adj, z, ho0, hi0, inv_s, in, edge);
-                const double2 tp = screen_coord(S.c[1], tI, ri.adj, z, ho1, hi1, inv_s, in, edge);
+                const double2 rp = screen_coord(S.c[0], ri, ri.adj, z, ho0, hi0, inv_s,
+                                                4.f * delta, in, edge);
+                const double2 tp = screen_coord(S.c[1], tI, ri.adj, z, ho1, hi1, inv_s,
+                                                4.f * delta, in, edge);
                 if (edge) unsure = true;
                 in = in && !edge;
                 // (a cell outside samples texel 0 and adds nothing)
-                const double2 a = screen_sample(ri, in ? rp.x : 0.0, in ? rp.y : 0.0);
-                const double2 b = screen_sample(tI, in ? tp.x : 0.0, in ? tp.y : 0.0);
+                const double2 a = screen_sample(ri, in ? rp.x : 0.0, in ? rp.y : 0.0, step);
+                const double2 b = screen_sample(tI, in ? tp.x : 0.0, in ? tp.y : 0.0, step);
                 if (n == 0) {
                     s0 = a;
                     s1 = b;
@@ -359,9 +403,13 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
         }
         if (n >= 1) {
             double roh = 0, count = 0;
+            const float err = 2.f * delta * sqrtf((float)n);
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-                const double c = acc[p].corr((double)n, unsure);
+                float off = 0.f;
+                const double c = acc[p].corr((double)n, err, step[p], off, unsure);
+                // (the mean's error is at most the larger one's)
+                sum_off += off;
                 if (c != -99.0) {
                     roh += c;
                     count += 1.0;
@@ -373,6 +421,7 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
         }
     }
     *avg = n_img > 0 ? n_sum / n_img : -1;
+    *band = (float)kScreenBand + 2e-7f + sum_off;
     if (unsure) return __int_as_float(0x7fc00000);
     return n_img > 0 ? (float)(sum_ncc / (double)n_img) : -2.f;
 }
@@ -587,28 +636,29 @@ __device__ SearchOut ortho_search(const DevLevel &P, const double2 *__restrict__
         const int kh = chunk + threadIdx.x;
         const bool live = kh < n_heights;
         int avg;
-        float a = screen_heights(P, lonlat, T, (double)height(live ? kh : chunk), live, &avg, st);
-        float sure = -2.f;   // the best correlation that surely passes
+        float band;
+        float a = screen_heights(P, lonlat, T, (double)height(live ? kh : chunk), live, &avg, &band, st);
+        float sure = -2.f;   // what the best correlation that surely passes is at least
         if (!live) {
             a = -2.f;
         } else if (!isnan(a)) {
             const double th = avg >= th_count ? min_th_sncc : min_th_sncc + 0.2;
             if (avg <= min_th_count && avg < th_count)
                 a = -2.f;
-            else if (!((double)a > th - kScreenBand))
+            else if (!((double)a > th - (double)band))
                 a = -2.f;
-            else if ((double)a > th + kScreenBand)
-                sure = a;
+            else if ((double)a > th + (double)band)
+                sure = a - band;
         }
 #pragma unroll
         for (int d = 16; d; d >>= 1) sure = fmaxf(sure, __shfl_xor_sync(0xffffffffu, sure, d));
         if (lane == 0) st.warp_best[warp] = sure;
         __syncthreads();
         for (int w = 0; w < kSearchWarps; ++w) sure = fmaxf(sure, st.warp_best[w]);
-        // (the screened values are floats: 2e-7 more on each side; a value
-        // that cannot beat the best so far is left out, NaN compares false)
-        const float slack = 2.f * (float)kScreenBand + 4e-7f;
-        const bool can = isnan(a) || (a > -2.f && a >= sure - slack && !(a + slack < (float)f_ncc));
+        // (a value that cannot beat the best so far is left out, NaN compares
+        // false)
+        const bool can =
+            isnan(a) || (a > -2.f && a + band >= sure && !(a + band < (float)f_ncc - 2e-7f));
         const unsigned m = __ballot_sync(0xffffffffu, can);
         if (lane == 0) st.todo[warp] = m;
         __syncthreads();
