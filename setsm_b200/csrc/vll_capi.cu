@@ -1281,9 +1281,9 @@ static int ortho_blunder_run(vll_context *ctx, DevLevel &P, double mpp, vll_poin
                                          d_tris, n_tris, d_gp3, ctx->tin_scratch.p, bytes, &it,
                                          &bad, ctx->stream));
     if (bad) return fail(ctx, VLL_ERR_INVALID, "a triangle vertex lies outside the grid");
-    // own kernels: the node and lon/lat passes, then select / search / records / apply /
-    // anchor per round (the radix sort between them is CUB's)
-    ctx->launches_total += 2 + 5 * (int64_t)it;
+    // own kernels: the node and lon/lat passes, then select / search / few heights /
+    // records / apply / anchor per round (the radix sort between them is CUB's)
+    ctx->launches_total += 2 + 6 * (int64_t)it;
     if (rounds) *rounds = it;
     return VLL_OK;
 }

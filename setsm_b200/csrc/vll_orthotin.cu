@@ -431,6 +431,7 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
 // the images' correlations, their number and the samples' number.  The cells
 // are sampled a thread each; each of Correlate's sums is then formed by one
 // thread in cell order.
+template <int kThreads>
 __device__ void exact_height(const DevLevel &P, const double2 *__restrict__ lonlat,
                              const TriBox &T, float iter_height, CellStage &st, double &sum_ncc,
                              int &count_ncc, int &sum_count_n) {
@@ -474,7 +475,7 @@ __device__ void exact_height(const DevLevel &P, const double2 *__restrict__ lonl
             for (int64_t base = 0; base < n_items; base += kCellCap) {
                 const int chunk = (int)(n_items - base < kCellCap ? n_items - base : kCellCap);
                 if (pass == 0 || !T.listed) {
-                    for (int i = t; i < ((chunk + 31) & ~31); i += kSearchThreads) {
+                    for (int i = t; i < ((chunk + 31) & ~31); i += kThreads) {
                         double v[4] = {0, 0, 0, 0};
                         bool ok = false;
                         if (i < chunk) {
@@ -581,32 +582,51 @@ __device__ bool tri_box(const DevLevel &P, P3 r1, P3 r2, P3 tg, TriBox &T) {
 // reference's exact value.  All heights are screened first, a thread each
 // (FP64 cubics per cell, one pass of FP64 sums), and those whose screened
 // correlation lies within the band of the best, or does not decide, are
-// evaluated exactly, in order: about one in a hundred.  Ortho_blunder on a
-// 700 x 690 grid with 9.7 k points (107 heights of 25 cells per search, 4
+// evaluated exactly, in order: about one in a hundred.  A few heights are all
+// evaluated exactly (few_heights).  Ortho_blunder on a 700 x 690 grid with 9.7 k points (107 heights of 25 cells per search, 4
 // rounds): 27.0 ms of search with every height evaluated exactly by a warp,
 // 2.0 ms; bound by the latency of the FP64 chains (12 warps per SM, FP64 pipe
 // 26 % busy).  Resident blocks 3, 4 or 5 per SM and one or two cells per
 // iteration: 2.9 to 3.1 ms for the whole call.
+// The step of the swept heights, and their number for a target node.
+__device__ __forceinline__ double height_step(const DevLevel &P, double mpp) {
+    if (mpp > 3) mpp = 3;
+    if (mpp < 1) mpp = 1;
+    return __dmul_rn(P.im_res, mpp);
+}
+__device__ __forceinline__ int height_count(const DevLevel &P, double hstep, int64_t target_index) {
+    const int lo = P.gp3[target_index].minHeight, hi = P.gp3[target_index].maxHeight;
+    return (int)__ddiv_rn((double)(hi - lo), hstep) + 1;
+}
+
+// Heights so few that the screen, which costs the same up to 128, costs more
+// than their exact values: seven over a small box, four over a larger one
+// (whole calls on a 700 x 690 grid, all evaluated exactly against all screened:
+// 9.7 k points 3 heights 1.24 and 2.37 ms, 6 heights 1.85 and 2.38; 2.4 k points
+// 2.24 and 2.90, 3.79 and 2.77; 483 points 13.3 and 19.7, 25.9 and 19.6).
+__device__ __forceinline__ bool few_heights(int n_heights, int64_t ncell) {
+    return n_heights <= (ncell < 160 ? 7 : 4);
+}
+
+template <int kThreads>
 __device__ SearchOut ortho_search(const DevLevel &P, const double2 *__restrict__ lonlat,
                                   double mpp, P3 r1, P3 r2, P3 tg, int64_t target_index,
                                   CellStage &st) {
+    constexpr int kWarps = kThreads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SearchOut o{-9999.0, 0.0, 0};
     double f_ncc = -1.0;
     double selected_count = 0;
-    if (mpp > 3) mpp = 3;
-    if (mpp < 1) mpp = 1;
-    const double hstep = __dmul_rn(P.im_res, mpp);
+    const double hstep = height_step(P, mpp);
     const int start_h = P.gp3[target_index].minHeight;
-    const int end_h = P.gp3[target_index].maxHeight;
-    const int n_heights = (int)__ddiv_rn((double)(end_h - start_h), hstep) + 1;
+    const int n_heights = height_count(P, hstep, target_index);
     const int th_count = 10;
     const int min_th_count = P.L < 4 ? 0 : 2;
     const double min_th_sncc = P.L < 4 ? 0.5 : 0.2;
     TriBox T;
     if (!tri_box(P, r1, r2, tg, T)) return o;
     // the inside cells, in cell order
-    for (int64_t base = 0; base < T.ncell; base += kSearchThreads) {
+    for (int64_t base = 0; base < T.ncell; base += kThreads) {
         const int64_t i = base + threadIdx.x;
         const bool in = i < T.ncell &&
                         cell_inside(P, r1, r2, tg, T.row0 + i / T.ncol, T.col0 + i % T.ncol);
@@ -614,7 +634,7 @@ __device__ SearchOut ortho_search(const DevLevel &P, const double2 *__restrict__
         if (lane == 0) st.warp_n[warp] = __popc(m);
         __syncthreads();
         int64_t at = T.n_in + __popc(m & ((1u << lane) - 1u));
-        for (int w = 0; w < kSearchWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             if (w < warp) at += st.warp_n[w];
             T.n_in += st.warp_n[w];
         }
@@ -630,66 +650,77 @@ __device__ SearchOut ortho_search(const DevLevel &P, const double2 *__restrict__
     auto height = [&](int kh) {
         return (float)__dadd_rn((double)start_h, __dmul_rn((double)kh, hstep));
     };
-    for (int chunk = 0; chunk < n_heights; chunk += kSearchThreads) {
-        // screen: a height that cannot pass its threshold is -2, one that the
-        // screen does not decide NaN
+    // the exact value of one height, taken where it is the best so far
+    auto take = [&](int kh) {
+        const float iter_height = height(kh);
+        double sum_ncc;
+        int count_ncc, sum_count_n;
+        exact_height<kThreads>(P, lonlat, T, iter_height, st, sum_ncc, count_ncc, sum_count_n);
+        if (count_ncc <= 0) return;
+        const double sncc = __ddiv_rn(sum_ncc, (double)count_ncc);
+        const double cnt = __ddiv_rn((double)sum_count_n, (double)count_ncc);
+        if (sum_count_n / count_ncc >= th_count) {
+            if (sncc > min_th_sncc && f_ncc < sncc) {
+                f_ncc = sncc;
+                o.f_height = (double)iter_height;
+                selected_count = cnt;
+                o.f_sncc = f_ncc;
+            }
+        } else if (sum_count_n / count_ncc > min_th_count) {
+            if (sncc > __dadd_rn(min_th_sncc, 0.2) && f_ncc < sncc) {
+                f_ncc = sncc;
+                o.f_height = __ddiv_rn(__dadd_rn(r1.z, r2.z), 2.0);
+                selected_count = cnt;
+                o.f_sncc = f_ncc;
+            }
+        }
+    };
+    for (int chunk = 0; chunk < n_heights; chunk += kThreads) {
         const int kh = chunk + threadIdx.x;
         const bool live = kh < n_heights;
-        int avg;
-        float band;
-        float a = screen_heights(P, lonlat, T, (double)height(live ? kh : chunk), live, &avg, &band, st);
-        float sure = -2.f;   // what the best correlation that surely passes is at least
-        if (!live) {
-            a = -2.f;
-        } else if (!isnan(a)) {
-            const double th = avg >= th_count ? min_th_sncc : min_th_sncc + 0.2;
-            if (avg <= min_th_count && avg < th_count)
-                a = -2.f;
-            else if (!((double)a > th - (double)band))
-                a = -2.f;
-            else if ((double)a > th + (double)band)
-                sure = a - band;
-        }
+        bool can = live;
+        if constexpr (kThreads == kSearchThreads) {
+            if (!few_heights(n_heights, T.ncell)) {
+                // screen: a height that cannot pass its threshold is -2, one that
+                // the screen does not decide NaN
+                int avg;
+                float band;
+                float a = screen_heights(P, lonlat, T, (double)height(live ? kh : chunk), live, &avg,
+                                         &band, st);
+                float sure = -2.f;   // what the best that surely passes is at least
+                if (!live) {
+                    a = -2.f;
+                } else if (!isnan(a)) {
+                    const double th = avg >= th_count ? min_th_sncc : min_th_sncc + 0.2;
+                    if (avg <= min_th_count && avg < th_count)
+                        a = -2.f;
+                    else if (!((double)a > th - (double)band))
+                        a = -2.f;
+                    else if ((double)a > th + (double)band)
+                        sure = a - band;
+                }
 #pragma unroll
-        for (int d = 16; d; d >>= 1) sure = fmaxf(sure, __shfl_xor_sync(0xffffffffu, sure, d));
-        if (lane == 0) st.warp_best[warp] = sure;
-        __syncthreads();
-        for (int w = 0; w < kSearchWarps; ++w) sure = fmaxf(sure, st.warp_best[w]);
-        // (a value that cannot beat the best so far is left out, NaN compares
-        // false)
-        const bool can =
-            isnan(a) || (a > -2.f && a + band >= sure && !(a + band < (float)f_ncc - 2e-7f));
+                for (int d = 16; d; d >>= 1)
+                    sure = fmaxf(sure, __shfl_xor_sync(0xffffffffu, sure, d));
+                if (lane == 0) st.warp_best[warp] = sure;
+                __syncthreads();
+                for (int w = 0; w < kWarps; ++w) sure = fmaxf(sure, st.warp_best[w]);
+                // (a value that cannot beat the best so far is left out, NaN
+                // compares false)
+                can = isnan(a) ||
+                      (a > -2.f && a + band >= sure && !(a + band < (float)f_ncc - 2e-7f));
+            }
+        }
         const unsigned m = __ballot_sync(0xffffffffu, can);
         if (lane == 0) st.todo[warp] = m;
         __syncthreads();
         // exact: the heights that can be the first of the largest correlation
-        for (int w = 0; w < kSearchWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             unsigned todo = st.todo[w];
             while (todo) {
                 const int b = __ffs(todo) - 1;
                 todo &= todo - 1;
-                const float iter_height = height(chunk + 32 * w + b);
-                double sum_ncc;
-                int count_ncc, sum_count_n;
-                exact_height(P, lonlat, T, iter_height, st, sum_ncc, count_ncc, sum_count_n);
-                if (count_ncc <= 0) continue;
-                const double sncc = __ddiv_rn(sum_ncc, (double)count_ncc);
-                const double cnt = __ddiv_rn((double)sum_count_n, (double)count_ncc);
-                if (sum_count_n / count_ncc >= th_count) {
-                    if (sncc > min_th_sncc && f_ncc < sncc) {
-                        f_ncc = sncc;
-                        o.f_height = (double)iter_height;
-                        selected_count = cnt;
-                        o.f_sncc = f_ncc;
-                    }
-                } else if (sum_count_n / count_ncc > min_th_count) {
-                    if (sncc > __dadd_rn(min_th_sncc, 0.2) && f_ncc < sncc) {
-                        f_ncc = sncc;
-                        o.f_height = __ddiv_rn(__dadd_rn(r1.z, r2.z), 2.0);
-                        selected_count = cnt;
-                        o.f_sncc = f_ncc;
-                    }
-                }
+                take(chunk + 32 * w + b);
             }
         }
         __syncthreads();   // the masks are rewritten by the next chunk
@@ -713,7 +744,7 @@ __global__ void __launch_bounds__(kSearchThreads) ortho_search_kernel(
     double *out) {
     const DevLevel &P = *Pp;
     __shared__ CellStage st;
-    const SearchOut o = ortho_search(P, nullptr, mpp, P3{pts3[0].x, pts3[0].y, pts3[0].z},
+    const SearchOut o = ortho_search<kSearchThreads>(P, nullptr, mpp, P3{pts3[0].x, pts3[0].y, pts3[0].z},
                                      P3{pts3[1].x, pts3[1].y, pts3[1].z},
                                      P3{pts3[2].x, pts3[2].y, pts3[2].z}, target_index, st);
     if (threadIdx.x == 0) {
@@ -746,17 +777,19 @@ __device__ SearchTri search_tri(const DevLevel &P, const vll_point3 *pts, const 
 constexpr int64_t kLargeBox = 512;
 
 // The triangles to search this round, listed in any order: those with a
-// large box from the front, the others from the back; n_list: their counts.
-__global__ void tri_select_kernel(const DevLevel *__restrict__ Pp, const vll_point3 *pts,
+// large box from the front, the others from the back, and in `few` those of
+// few heights and a box that is not large; n_list: their counts (others,
+// large, [3] few).
+__global__ void tri_select_kernel(const DevLevel *__restrict__ Pp, double mpp, const vll_point3 *pts,
                                   int64_t n_pts, const vll_tri *tris, int64_t n_tris,
                                   const int64_t *tri_nodes, uint8_t *tris_check,
-                                  uint32_t *sort_key, int32_t *list, int *n_list) {
+                                  uint32_t *sort_key, int32_t *list, int32_t *few, int *n_list) {
     const DevLevel &P = *Pp;
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t n_round = (n_tris + 31) & ~(int64_t)31;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_round; t += stride) {
-        int kind = 0;   // 1 search, 2 search early
+        int kind = 0;   // 1 search, 2 search early, 3 few heights
         if (t < n_tris) {
             sort_key[t] = (uint32_t)n_pts;
             const vll_tri tr = tris[t];
@@ -769,18 +802,26 @@ __global__ void tri_select_kernel(const DevLevel *__restrict__ Pp, const vll_poi
                 } else if (nf == 2) {
                     const SearchTri q = search_tri(P, pts, tr, tri_nodes + 3 * t);
                     TriBox T;
-                    if (tri_box(P, q.r1, q.r2, q.tg, T)) kind = T.ncell >= kLargeBox ? 2 : 1;
+                    if (tri_box(P, q.r1, q.r2, q.tg, T))
+                        kind = T.ncell >= kLargeBox ? 2
+                               : few_heights(height_count(P, height_step(P, mpp), q.node), T.ncell) ? 3
+                                                                                                   : 1;
                 }
             }
         }
 #pragma unroll
-        for (int k = 1; k <= 2; ++k) {
+        for (int k = 1; k <= 3; ++k) {
             const unsigned m = __ballot_sync(0xffffffffu, kind == k);
             if (!m) continue;
             int at = 0;
-            if (lane == __ffs(m) - 1) at = atomicAdd(n_list + (k - 1), __popc(m));
+            if (lane == __ffs(m) - 1) at = atomicAdd(n_list + (k == 3 ? 3 : k - 1), __popc(m));
             at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
-            if (kind == k) list[k == 2 ? at : (int)n_tris - 1 - at] = (int32_t)t;
+            if (kind == k) {
+                if (k == 3)
+                    few[at] = (int32_t)t;
+                else
+                    list[k == 2 ? at : (int)n_tris - 1 - at] = (int32_t)t;
+            }
         }
     }
 }
@@ -802,13 +843,40 @@ __global__ void __launch_bounds__(kSearchThreads, 3) tri_search_kernel(
         if (i >= n_small + n_large) return;
         const int64_t t = i < n_large ? list[i] : list[(int)n_tris - 1 - (i - n_large)];
         const SearchTri q = search_tri(P, pts, tris[t], tri_nodes + 3 * t);
-        const SearchOut o = ortho_search(P, lonlat, mpp, q.r1, q.r2, q.tg, q.node, st);
+        const SearchOut o = ortho_search<kSearchThreads>(P, lonlat, mpp, q.r1, q.r2, q.tg, q.node, st);
         if (threadIdx.x == 0 && o.f_height != -9999.0) {
             hgt[t] = o.f_height;
             cnt[t] = o.selected;
             sort_key[t] = q.point;
         }
         __syncthreads();   // the staging is rewritten by the next triangle
+    }
+}
+
+// The listed triangles of few heights, a warp each, from a queue: a block's
+// other warps would wait for most of an exact evaluation (700 x 690 grid, 145 k
+// points, 3 heights each: 10.1 ms screened by blocks, 3.6 here).
+__global__ void __launch_bounds__(32, 12) tri_few_kernel(
+    const DevLevel *__restrict__ Pp, double mpp, const vll_point3 *pts, const vll_tri *tris,
+    const int64_t *tri_nodes, double *hgt, int32_t *cnt, uint32_t *sort_key, const int32_t *few,
+    int *n_list, const double2 *__restrict__ lonlat) {
+    const DevLevel &P = *Pp;
+    __shared__ CellStage st;
+    const int n = n_list[3];
+    for (;;) {
+        int i = 0;
+        if (threadIdx.x == 0) i = atomicAdd(n_list + 4, 1);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= n) return;
+        const int64_t t = few[i];
+        const SearchTri q = search_tri(P, pts, tris[t], tri_nodes + 3 * t);
+        const SearchOut o = ortho_search<32>(P, lonlat, mpp, q.r1, q.r2, q.tg, q.node, st);
+        if (threadIdx.x == 0 && o.f_height != -9999.0) {
+            hgt[t] = o.f_height;
+            cnt[t] = o.selected;
+            sort_key[t] = q.point;
+        }
+        __syncwarp();   // the staging is rewritten by the next triangle
     }
 }
 
@@ -987,8 +1055,8 @@ cudaError_t run_ortho_blunder(const DevLevel *dP, const DevLevel &hP, double mpp
     int32_t *sval = (int32_t *)take(n_tris * 4);
     int32_t *list = (int32_t *)take(n_tris * 4);
     unsigned long long *first_anchor = (unsigned long long *)take(hP.n_nodes * 8);
-    // [0] any record, [1] bad input, [2..4] listed triangles (small, large box)
-    // and the search's queue
+    // [0] any record, [1] bad input, [2..6] listed triangles: others, large
+    // box, the search's queue, few heights, their queue
     int *flags = (int *)take(32);
     double2 *lonlat = (double2 *)take(hP.n_nodes * 16);
     if ((size_t)(p - (char *)scratch) > scratch_bytes) return cudaErrorInvalidValue;
@@ -1015,13 +1083,20 @@ cudaError_t run_ortho_blunder(const DevLevel *dP, const DevLevel &hP, double mpp
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri_search_kernel, kSearchThreads, 0);
     const unsigned search_blocks =
         (unsigned)std::min<int64_t>(n_tris, (int64_t)sms * std::max(per_sm, 1));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri_few_kernel, 32, 0);
+    const unsigned few_blocks =
+        (unsigned)std::min<int64_t>(n_tris, (int64_t)sms * std::max(per_sm, 1));
+    // (the sort's output is free until the sort)
+    int32_t *few = sval;
     for (int it = 0; it < 200; ++it) {
         *iterations = it + 1;
         if ((e = cudaMemsetAsync(flags, 0, 32, s))) return e;
         tri_select_kernel<<<blocks_for(n_tris, 256), 256, 0, s>>>(
-            dP, pts, n_pts, tris, n_tris, tri_nodes, tris_check, key, list, flags + 2);
+            dP, mpp, pts, n_pts, tris, n_tris, tri_nodes, tris_check, key, list, few, flags + 2);
         tri_search_kernel<<<search_blocks, kSearchThreads, 0, s>>>(
             dP, mpp, pts, tris, n_tris, tri_nodes, hgt, cnt, key, list, flags + 2, lonlat);
+        tri_few_kernel<<<few_blocks, 32, 0, s>>>(dP, mpp, pts, tris, tri_nodes, hgt, cnt, key, few,
+                                                 flags + 2, lonlat);
         if ((e = cudaGetLastError())) return e;
         if ((e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, skey, val, sval, (int)n_tris,
                                                  0, end_bit, s)))

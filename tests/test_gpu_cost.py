@@ -71,3 +71,24 @@ def test_blunder_beside_empty_areas(gpu_ctx):
             lambda g: gpu_ctx.blunder_device(d, g.data_ptr(), 1, False, out.data_ptr()),
             lambda: (first.clone(),))
     assert times[True] < 1.7 * times[False], times
+
+
+def test_search_of_few_heights(gpu_ctx):
+    """Three heights per triangle against 41 on the same triangles: at most
+    0.65 of the time (0.48 as measured; 0.76 when three were screened too)."""
+    import torch
+    times = {}
+    for half in (1, 20):
+        inp, pts, tris = cases.make_tin_case(seed=9, size=1024, nodes=240, res=2.0, point_frac=0.2)
+        inp.resolution = 1.0    # of the heights' step
+        g = inp.gridpt3
+        mid = (g["minHeight"].astype(int) + g["maxHeight"]) // 2
+        g["minHeight"], g["maxHeight"] = mid - half, mid + half
+        d, gp3, keep = on_device(inp)
+        dev = lambda a: torch.from_numpy(a.view(np.uint8).copy()).cuda()
+        p0, t = dev(pts), dev(tris)
+        times[half] = median_time(
+            lambda g, p: gpu_ctx.ortho_blunder_device(d, 1.0, p.data_ptr(), len(pts), t.data_ptr(),
+                                                      len(tris), g.data_ptr()),
+            lambda: (gp3.clone(), p0.clone()))
+    assert times[1] < 0.65 * times[20], times
