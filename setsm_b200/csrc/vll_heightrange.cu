@@ -8,9 +8,9 @@
 // the iteration, the triangle's slope (SetNormalAngle, :2997-3012) and the
 // node's orthoimage NCC; nodes in no triangle take the union of their matched
 // neighbours' ranges.  The reference walks the triangles in order and a node
-// is set by the first triangle that contains it; here one warp per triangle
-// marks, per node, the smallest containing triangle index (atomicMin), and a
-// pass over the nodes then applies that triangle's update -- the same result.
+// is set by the first triangle that contains it; here a triangle's lanes (one
+// to a block's) mark, per node, the smallest containing triangle index (atomicMin),
+// and a pass over the nodes then applies that triangle's update -- the same result.
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -156,10 +156,13 @@ __device__ __forceinline__ void cover_cells(const DevLevel &P, const Tri3 &T, co
 
 // The extent of the triangles' vertex heights and, per node inside a
 // triangle, the smallest containing triangle index.  A triangle per kLanes
-// lanes: one where the triangles fill the chip, up to eight where they do not
-// and a lane's chain of FP64 cell tests would set the time (27 k triangles: the
-// points' calls 313 -> 273 us);
-// the extent is reduced per warp before its two atomics (one pair per
+// lanes: one where the triangles fill the chip, 4 to 128 where they do not and
+// a lane's chain of FP64 cell tests would set the time.  The fewer the
+// triangles, the larger their boxes: the call on 700 x 690 nodes with 131
+// triangles took 948 us with eight lanes each (large boxes swept by a warp, one
+// after the other) and 433 with a warp each, now 230; with 1.9 k 217, 185 and
+// 163; with 9.4 k 174, 162 and 165.
+// The extent is reduced per warp before its two atomics (one pair per
 // triangle, all on the same words, took 0.78 of the kernel's 0.87 ms for the
 // 650 k triangles of a 600 x 600 grid, which now takes 0.12).
 template <int kLanes>
@@ -170,13 +173,14 @@ __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__
                                                     unsigned long long *zext) {
     const DevLevel &P = *Pp;
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    // a warp's step is kPer triangles (kLanes = 128: a block's is one)
+    constexpr int kUnit = kLanes > 32 ? kLanes : 32, kPer = kLanes > 32 ? 1 : 32 / kLanes;
+    const int64_t unit = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kUnit;
+    const int64_t n_units = (int64_t)gridDim.x * blockDim.x / kUnit;
     unsigned long long zmin = ~0ull, zmax = 0;
     bool any = false;
-    constexpr int kPer = 32 / kLanes;   // triangles of a warp's step
-    for (int64_t t0 = warp * kPer; t0 < n_tris; t0 += n_warps * kPer) {
-        const int64_t t = t0 + lane / kLanes;
+    for (int64_t t0 = unit * kPer; t0 < n_tris; t0 += n_units * kPer) {
+        const int64_t t = t0 + (kLanes > 32 ? 0 : lane / kLanes);
         Tri3 T;
         BBox b{0, 0, -1, -1};
         if (t < n_tris) {
@@ -192,11 +196,12 @@ __global__ void __launch_bounds__(128) cover_kernel(const DevLevel *__restrict__
             }
         }
         const bool box = b.x1 >= b.x0 && b.y1 >= b.y0;
-        const bool large =
-            box && (int64_t)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1) > kLaneBox * kLanes;
+        // (a whole warp sweeps any box)
+        const bool large = kLanes < 32 && box &&
+                           (int64_t)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1) > kLaneBox * kLanes;
         if (box && !large)
-            cover_cells(P, T, b, (unsigned int)t, lane % kLanes, kLanes, winner);
-        unsigned m = __ballot_sync(0xffffffffu, large && lane % kLanes == 0);
+            cover_cells(P, T, b, (unsigned int)t, threadIdx.x % kLanes, kLanes, winner);
+        unsigned m = kLanes < 32 ? __ballot_sync(0xffffffffu, large && lane % kLanes == 0) : 0;
         while (m) {
             // the warp sweeps the box of lane l's triangle
             const int l = (__ffs(m) - 1) / kLanes;
@@ -486,13 +491,22 @@ cudaError_t run_height_range(const DevLevel *dP, const DevLevel &hP, const vll_p
     if ((e = cudaMemsetAsync(out, 0, N * sizeof(vll_ugrid), s))) return e;
     const RangeArgs a{buffer, th_hg, iteration};
     if (n_tris > 0) {
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         // (few enough warps that their extent atomics do not count)
-        constexpr int64_t kResident = 148 * 2048;   // threads
-        const int lanes = n_tris * 8 <= kResident ? 8 : n_tris * 4 <= kResident ? 4 : 1;
-        const unsigned blocks = std::min(blocks_for(n_tris * lanes, 128), 148u * 16u);
-        (lanes == 8   ? cover_kernel<8>
-         : lanes == 4 ? cover_kernel<4>
-                      : cover_kernel<1>)<<<blocks, 128, 0, s>>>(dP, pts, n_pts, tris, n_tris, winner,
+        const int64_t resident = (int64_t)sms * 2048;   // threads
+        const int lanes = n_tris * 48 <= resident   ? 128
+                          : n_tris * 32 <= resident ? 32
+                          : n_tris * 8 <= resident  ? 8
+                          : n_tris * 4 <= resident  ? 4
+                                                    : 1;
+        const unsigned blocks = std::min(blocks_for(n_tris * lanes, 128), (unsigned)sms * 16u);
+        (lanes == 128  ? cover_kernel<128>
+         : lanes == 32 ? cover_kernel<32>
+         : lanes == 8  ? cover_kernel<8>
+         : lanes == 4  ? cover_kernel<4>
+                       : cover_kernel<1>)<<<blocks, 128, 0, s>>>(dP, pts, n_pts, tris, n_tris, winner,
                                                                 zkey);
     }
     zext_kernel<<<1, 1, 0, s>>>(zkey, zext);

@@ -92,3 +92,21 @@ def test_search_of_few_heights(gpu_ctx):
                                                       len(tris), g.data_ptr()),
             lambda: (gp3.clone(), p0.clone()))
     assert times[1] < 0.65 * times[20], times
+
+
+def test_height_range_of_few_triangles(gpu_ctx):
+    """Some 130 triangles over a grid against 9 k: at most 2.5 times the time
+    (1.2 as measured; 4.0 with eight lanes per triangle)."""
+    import torch
+    times = {}
+    for frac in (0.0003, 0.02):
+        inp, pts, tris = cases.make_range_case(seed=9, size=1024, nodes=480, res=1.0, point_frac=frac)
+        d, gp3, keep = on_device(inp)
+        p, t = (torch.from_numpy(a.view(np.uint8).copy()).cuda() for a in (pts, tris))
+        out = torch.zeros(inp.n * 20, dtype=torch.uint8, device="cuda")
+        times[frac] = median_time(
+            lambda g: gpu_ctx.set_height_range_device(d, p.data_ptr(), len(pts), t.data_ptr(),
+                                                      len(tris), g.data_ptr(), out.data_ptr(), 2, 1.5,
+                                                      False),
+            lambda: (gp3.clone(),))
+    assert times[0.0003] < 2.5 * times[0.02], times
