@@ -309,7 +309,7 @@ __device__ __forceinline__ bool combined_level(const uint16_t *const img[2],
     const float4 *qr = boxes + (riy - H - ry0) * rs + (rix - H - rx0);
     const uint32_t tcen =
         box_off + (uint32_t)(rs * rh + (tiy - ty0) * ts + (tix - tx0)) * 16u;
-    window_any(H, qr, rs, (float)(rp.x - (double)rix), (float)(rp.y - (double)riy),
+    window_any<true>(H, qr, rs, (float)(rp.x - (double)rix), (float)(rp.y - (double)riy),
                tgt_box(smem, tcen, (uint32_t)ts * 16u), (float)(tp.x - (double)tix),
                (float)(tp.y - (double)tiy), cf, sf, incc, unsure);
     return true;
@@ -456,8 +456,9 @@ __global__ void __launch_bounds__(kWinWarps * 32, VLL_WIN_MINB) combined_kernel(
                 }
                 evals++;
             }
-            scan_group(N, scan, K, N.flags, k, k0, status, rho_v, incc_v, all_pos, deferred, wv,
-                       fix_list, fix_cap, ctl, lane);
+            // (the debug values of undecided slots are the exact pass's)
+            scan_group(N, scan, K, N.flags, k, k0, status, rho_v, incc_v, all_pos,
+                       deferred || unsure, wv, fix_list, fix_cap, ctl, lane);
         }
         finish_node(N, scan, K, N.flags, wv, pend_vals, pend_cap, pend_node, pend_off, ctl, lane);
     }

@@ -270,16 +270,18 @@ __host__ __device__ constexpr size_t win_raw_offset(int warp_quads) {
 
 // FP32 window statistics of one slot for the level's window half-size
 // (the window code is unrolled per half-size; a batch may mix them).
+// kStrict: see kCentreFloor.
+template <bool kStrict = false>
 __device__ __forceinline__ void window_any(int H, const float4 *qr, int rbw, float rfx, float rfy,
                                            const TgtBox &tb, float tfx, float tfy, float c,
                                            float s, float &incc, bool &unsure) {
     switch (H) {
-        case 2: window_fp32<2>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 3: window_fp32<3>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 4: window_fp32<4>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 5: window_fp32<5>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        case 6: window_fp32<6>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
-        default: window_fp32<7>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        case 2: window_fp32<2, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        case 3: window_fp32<3, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        case 4: window_fp32<4, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        case 5: window_fp32<5, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        case 6: window_fp32<6, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
+        default: window_fp32<7, kStrict>(qr, rbw, rfx, rfy, tb, tfx, tfy, c, s, incc, unsure); break;
     }
 }
 

@@ -32,10 +32,21 @@ struct Acc {
     float sl, sr, sll, srr, slr;
 };
 
+// A sample is formed from texels less their box's shift and then taken about
+// its window's centre sample: where the window lies far from the shift, c, the
+// samples carry roundings of c, some 3 * 2^-24 |c|, which must stay below 2e-6
+// (half the error band) of the root of the window's sum of squares.  Nearly
+// constant windows beside texture fail that: images with saturated or constant
+// areas had rho off by up to 4.5e-6 in combined levels, whose windows alone
+// take this test (the slot goes to the exact pass).
+constexpr float kCentreFloor = 0.008f;   // (3 * 2^-24 / 2e-6)^2
+
 // Pearson rho from shifted sums; returns -99 when a variance is below the
 // reference's 1e-8 threshold and flags results whose variance is too small
 // for FP32 to decide that threshold safely.
-__device__ __forceinline__ float corr_from(const Acc &a, float n, bool &unsure) {
+// kStrict: the same of a variance below fl (left) or fr (right).
+template <bool kStrict>
+__device__ __forceinline__ float corr_from(const Acc &a, float n, bool &unsure, float fl, float fr) {
     const float inv = 1.0f / n;
     const float vl = a.sll - a.sl * a.sl * inv;
     const float vr = a.srr - a.sr * a.sr * inv;
@@ -43,6 +54,7 @@ __device__ __forceinline__ float corr_from(const Acc &a, float n, bool &unsure) 
     // FP32 relative error of vl is ~n * 6e-8 * (sll / vl); treat anything
     // within a factor of the threshold, or heavily cancelled, as uncertain.
     if (vl < 1e-3f * a.sll + 1e-4f || vr < 1e-3f * a.srr + 1e-4f) unsure = true;
+    if (kStrict && (vl < fl || vr < fr)) unsure = true;
     if (!(vl > 1e-8f && vr > 1e-8f)) return -99.0f;
     return cv * rsqrtf(vl * vr);
 }
@@ -251,7 +263,7 @@ __device__ __forceinline__ Acc plane(const Acc2 &a, int p) {
 // target box addressed from the window centre's texel; (rfx, rfy), (tfx,
 // tfy): the fractional positions.  Sums are shifted by each window's centre
 // sample.
-template <int H>
+template <int H, bool kStrict>
 __device__ __forceinline__ void window_fp32(const float4 *__restrict__ qr, int rbw, float rfx,
                                             float rfy, const TgtBox &tb, float tfx, float tfy,
                                             float c, float s, float &incc_avg, bool &unsure) {
@@ -284,9 +296,12 @@ __device__ __forceinline__ void window_fp32(const float4 *__restrict__ qr, int r
     int nv = 0;
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-        const float r2 = corr_from(plane(acc[2], p), (float)n2, unsure);
-        const float r1 = corr_from(plane(acc[1], p), (float)n1, unsure);
-        const float r0 = corr_from(plane(acc[0], p), (float)n0, unsure);
+        float fl = p ? x.ncl.y : x.ncl.x, fr = p ? x.ntc.y : x.ntc.x;
+        fl *= kCentreFloor * fl;
+        fr *= kCentreFloor * fr;
+        const float r2 = corr_from<kStrict>(plane(acc[2], p), (float)n2, unsure, fl, fr);
+        const float r1 = corr_from<kStrict>(plane(acc[1], p), (float)n1, unsure, fl, fr);
+        const float r0 = corr_from<kStrict>(plane(acc[0], p), (float)n0, unsure, fl, fr);
         if (r0 != -99.0f) { tot += r0; ++nv; }
         if (r1 != -99.0f) { tot += r1; ++nv; }
         if (r2 != -99.0f) { tot += r2; ++nv; }
