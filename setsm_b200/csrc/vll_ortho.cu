@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(128) blunder_kernel(const DevLevel *__restrict
 //
 // 1024^2 grid, 4097^2 pixels, 11x11 window: 9.85 ms with the samples formed
 // per node and pass (raster 3.8, nodes 6.0), now 2.11 (2.04 with one band for
-// all nodes; raster about 0.95, nodes 0.95, exact 0.2): the raster is bound by FP64 issue and latency (585 FP64
-// instructions per 32 pixels), the node pass by latency at 16 warps per SM (12
-// warps: 2.37 ms in all, 20: 2.54).
+// all nodes; raster about 0.95, nodes 0.95, exact 0.2): the raster is bound by
+// FP64 issue and latency (585 FP64 instructions per 32 pixels), the node pass by
+// latency at 16 warps per SM (12 warps: 2.37 ms in all, 20: 2.54).
 constexpr double kSumBand = 1e-9;   // one-pass against two-pass sums of the same samples
 constexpr int kMaxSampledH = 15;   // larger windows take the per-node kernels
 constexpr int kNodeLanes = 4;      // lanes per node: columns c = lane (mod 4)
@@ -1028,6 +1028,8 @@ static cudaError_t launch_nodes(const DevLevel *dP, int64_t n, const SampledArgs
                                 cudaStream_t s) {
     const unsigned blocks = blocks_for(n * kNodeLanes, 128);
     const int nj = (2 * A.H + 1 + kNodeLanes - 1) / kNodeLanes;
+    // (300 x 280 nodes, H = 8 and 15: seed DEM 0.54 and 1.03 ms, blunder 0.48 and
+    // 0.91; by the per-node kernels 1.95 and 5.36, 0.99 and 3.42)
     if (nj <= 3)
         node_ncc_kernel<kBlunder, 3><<<blocks, 128, 0, s>>>(dP, A, gout, ncc_out, todo, n_todo);
     else if (nj <= 4)

@@ -377,7 +377,9 @@ __device__ unsigned long long g_phase_cycles[16];
 #endif
 
 // Image coordinate (pyramid level) of one slot of node N in image im from
-// the node's cubics (fast_coord's arithmetic on the node context).
+// the node's cubics.  Sets `edge` when a coordinate is too close to an
+// integer, or to a clamp, for the cubics' rounding to be trusted with the
+// reference's integer tests.
 __device__ __forceinline__ double2 node_coord(const NodeCtx &N, int im, double hgt, bool &edge) {
     const double H = (hgt - N.hnorm[im][0]) * N.hnorm[im][1];
     double v[4];

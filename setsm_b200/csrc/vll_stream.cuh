@@ -10,9 +10,12 @@
 namespace vll {
 
 // Half-width of the FP32 error band of rho: decisions whose FP32 inputs lie
-// closer than this to their boundary are settled in FP64.  The FP32-vs-FP64
-// error of rho measured over 4.2 M slots of 7x7 and 11x11 windows stays below
-// 6.8e-7 (tests/test_gpu_accuracy.py asserts < kBand / 2), a margin of ~3x.
+// closer than this to their boundary are settled in FP64, which holds while
+// the FP32 error of rho stays below half of it.  Over textured scenes it stays
+// below 4.4e-7 (4.4 M slots of 7x7 and 11x11 windows, tests/test_gpu_accuracy.py;
+// combined levels 2.8e-7 over 0.9 M).  Combined levels of images with
+// saturated, constant or quantised areas: 2.5e-6 at one of 8 M slots, 2e-6 at
+// no other (see kCentreFloor).
 constexpr float kBand = 4e-6f;
 constexpr double kEdge = 1e-7;          // coordinate distance to an integer / clamp
 constexpr int kSlotCap = 512;           // slots per node the peak kernel holds in shared memory
@@ -91,29 +94,6 @@ __device__ __forceinline__ double fast_rcp(double v, bool &edge) {
     return r;
 }
 
-// Image coordinate (pyramid level) of one slot from the per-node cubics.
-// Sets `edge` when a coordinate is too close to an integer, or to a clamp,
-// for the Horner rounding to be trusted with the reference's integer tests.
-__device__ __forceinline__ double2 fast_coord(const double (*a)[4], const double *hn,
-                                              const DevImage &im, double hgt, double inv_s,
-                                              bool &edge) {
-    const double H = (hgt - hn[0]) * hn[1];   // hn[1]: reciprocal of the height scale
-    double v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = fma(fma(fma(a[j][3], H, a[j][2]), H, a[j][1]), H, a[j][0]);
-    double y = im.adj[0] + ((v[0] * fast_rcp(v[1], edge)) * im.rpc[5] + im.rpc[0]);
-    double x = im.adj[1] + ((v[2] * fast_rcp(v[3], edge)) * im.rpc[6] + im.rpc[1]);
-    const double ymax = im.rpc[0] + im.rpc[5] * 1.2, xmax = im.rpc[1] + im.rpc[6] * 1.2;
-    if (fabs(y) < kEdge || fabs(y - ymax) < kEdge || fabs(x) < kEdge || fabs(x - xmax) < kEdge)
-        edge = true;
-    y = y < 0 ? 0 : (y > ymax ? ymax : y);
-    x = x < 0 ? 0 : (x > xmax ? xmax : x);
-    const double px = x * inv_s - im.sx, py = y * inv_s - im.sy;   // inv_s = 2^-L (exact)
-    const double fx = px - floor(px), fy = py - floor(py);
-    if (fx < kEdge || fx > 1.0 - kEdge || fy < kEdge || fy > 1.0 - kEdge) edge = true;
-    return make_double2(px, py);
-}
-
 __device__ __forceinline__ bool near_round(double v) {
     const double x = v * 1000.0;
     return fabs(x - floor(x) - 0.5) < (double)kBand * 1000.0;
@@ -122,8 +102,6 @@ __device__ __forceinline__ bool near_trunc(double v) {
     const double x = v * 1000.0;
     return fabs(x - rint(x)) < (double)kBand * 1000.0;
 }
-
-
 
 __device__ __forceinline__ bool bit(const uint32_t *m, int k) { return (m[k >> 5] >> (k & 31)) & 1u; }
 __device__ __forceinline__ void set_bit(uint32_t *m, int k) { atomicOr(&m[k >> 5], 1u << (k & 31)); }

@@ -16,9 +16,9 @@
 // threshold is then known to lie in a band; a point pass in which some
 // comparison falls inside the band is undone and run again with the sums in
 // the reference's order), the per-point triangle lists by counting and a
-// fill, the point pass one warp per point (lane k takes the point's k-th
-// triangle in triangle order, after a warp sort) with the same
-// compare-and-swap marking, and the closing pass with warp-aggregated atomics
+// fill, the point pass eight lanes per point, a warp where it has more
+// triangles (lane k takes the point's k-th triangle in triangle order, after a
+// sort across the lanes), with the same compare-and-swap marking, and the closing pass with warp-aggregated atomics
 // (order-free counts, min / max).
 #include <cmath>
 #include <cstdint>

@@ -460,12 +460,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
     }
 }
 
-// Orders this thread's earlier generic shared-memory accesses before later
-// asynchronous-proxy (TMA) writes to the same memory.
-__device__ __forceinline__ void fence_async_shared() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // 2-D tile of a tensor map (TMA, no multicast) into this CTA's shared memory
 // at `dst` (128-byte aligned): x (innermost, a multiple of 16 bytes) and y
 // are the tile's first texel; completes the tile's bytes on `bar`.
