@@ -165,9 +165,9 @@ struct TriBox {
 // triangle's few samples beside a bright texel.  kScreenBand covers the rest:
 // one FP64 pass of sums over samples shifted by the first, and the float.
 constexpr double kScreenBand = 1e-6;
-constexpr double kMinC = 1e-2;
-constexpr double kCubicError = 2e-9;
-constexpr double kCoordEdge = 1e-6;   // coordinate distance to a clamp left to the exact pass
+constexpr float kMinC = 1e-2f;
+constexpr float kCubicError = 2e-9f;
+constexpr float kMaxError = 1e-6f;   // larger plane errors, in texels: the exact pass
 
 // 1 / v from an FP32 seed and two Newton steps; `edge` is set where the seed
 // is no finite non-zero float.
@@ -212,9 +212,9 @@ __device__ void screen_poly(const double *rpc, double lon, double lat, int j0, d
 
 // One pyramid coordinate from the scaled ratio v (clamped to [0, vmax] like
 // the reference's) and whether it lies in an image of `size` texels (0 <= c,
-// c + 1 < size).  `edge`: v lies too close to a clamp, or the unclamped
-// coordinate within `near` (four errors) of a texel's position, the bounds
-// among them, for the cubics to decide (a clamped one is exact).
+// c + 1 < size).  `edge`: the coordinate lies within `near` (four errors) of a
+// clamp or, unclamped, of a texel's position, the bounds among them, for the
+// cubics to decide (a clamped one is exact).
 __device__ __forceinline__ double screen_bound(double v, double vmax, double inv_s, double start,
                                                uint32_t size, float near, bool &in,
                                                bool &edge) {
@@ -222,7 +222,7 @@ __device__ __forceinline__ double screen_bound(double v, double vmax, double inv
     const bool lo = v < 0, hi = v > vmax;
     const double c = fma(lo ? 0.0 : (hi ? vmax : v), inv_s, -start);
     const double last = (double)size - 1.0;
-    if (!(fmin(fabs(v), fabs(v - vmax)) > kCoordEdge)) edge = true;
+    if (!(fmin(fabs(v), fabs(v - vmax)) * inv_s > (double)near)) edge = true;
     if (!(lo || hi) && !(fabs(c - __dadd_rn(__dadd_rn(c, kRint), -kRint)) > (double)near)) edge = true;
     in = in && c >= 0 && c < last;
     return c;
@@ -297,15 +297,14 @@ struct ScreenAcc {
 
 // What the reference's plane equation (exact_height) may differ from the
 // triangle's linear form by, in metres of height: nine roundings of its terms,
-// of the size of the coordinates, over |C|, and of the normal, which a thin
-// triangle magnifies, over the triangle.  len: the normal's length, den: its
-// vertical component.
-__device__ __forceinline__ double plane_error(const P3 &r1, double v12x, double v12y, double v12z,
-                                              double v13x, double v13y, double v13z, double den,
-                                              double len) {
-    const double a = sqrt(v12x * v12x + v12y * v12y + v12z * v12z);
-    const double b = sqrt(v13x * v13x + v13y * v13y + v13z * v13z);
-    return 1e-15 * (fabs(r1.x) + fabs(r1.y) + fabs(r1.z) + (a + b) * (a * b / len)) * len / fabs(den);
+// of the size `m` of the coordinates, over |C|, and of the normal, which a thin
+// triangle magnifies, over the triangle.  v12, v13: its edges, len: the normal's
+// length, den: its vertical component.  (A bound: FP32, whose own error the
+// tenth of a rounding more covers.)
+__device__ __forceinline__ float plane_error(float m, float3 v12, float3 v13, float den, float len) {
+    const float a = sqrtf(v12.x * v12.x + v12.y * v12.y + v12.z * v12.z);
+    const float b = sqrtf(v13.x * v13.x + v13.y * v13.y + v13.z * v13.z);
+    return 1.01e-15f * (m + (a + b) * (a * b / len)) * len / fabsf(den);
 }
 
 // The correlation of the triangle at one height per thread: the mean over the
@@ -322,12 +321,15 @@ __device__ float screen_heights(const DevLevel &P, const double2 *__restrict__ l
     bool unsure = !live;
     float delta;   // the coordinates' error in texels
     {
-        const double nx = v12y * v13z - v12z * v13y, ny = v12z * v13x - v12x * v13z;
-        const double len = sqrt(nx * nx + ny * ny + den * den);
+        const float3 v12 = make_float3((float)v12x, (float)v12y, (float)v12z);
+        const float3 v13 = make_float3((float)v13x, (float)v13y, (float)v13z);
+        const float nx = v12.y * v13.z - v12.z * v13.y, ny = v12.z * v13.x - v12.x * v13.z;
+        const float nz = (float)den, len = sqrtf(nx * nx + ny * ny + nz * nz);
         // (a metre of height is at most a metre on the ground)
-        const double e = plane_error(T.r1, v12x, v12y, v12z, v13x, v13y, v13z, den, len) / P.im_res;
-        if (!(fabs(den) > kMinC * len) || !(e < 0.25 * kCoordEdge)) unsure = true;
-        delta = (float)(kCubicError + e);
+        const float m = (float)(fabs(T.r1.x) + fabs(T.r1.y) + fabs(T.r1.z));
+        const float e = plane_error(m, v12, v13, nz, len) / (float)P.im_res;
+        if (!(fabsf(nz) > kMinC * len) || !(e < kMaxError)) unsure = true;
+        delta = kCubicError + e;
     }
     const double inv_s = 1.0 / (double)(1 << P.L);
     const DevImage &ri = P.im[P.ref];
