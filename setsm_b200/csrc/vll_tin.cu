@@ -50,8 +50,10 @@ constexpr int kThreadedCutoff = 100;
 // block in shared memory; larger ones a depth at a time over all points.
 constexpr int kBlockPoints = 1024;
 // Up to this many points the three orders are made by counting: three library
-// sorts of so few keys are some forty dependent passes (7500 points: the call
-// 1288 -> 1100 us, 48 points: 280 -> 241 us; the counting grows with the square).
+// sorts of so few keys are some forty dependent passes.  Calls of 48, 1000, 4000
+// and 8192 points: 306, 635, 1186 and 1443 us sorted, 265, 593, 939 and 1275
+// counted; the counting grows with the square (12000: 1681 and 1598, 16000: 1719
+// and 1810), so the line lies well below the crossing.
 constexpr int kRankPoints = 8192;
 constexpr int kRankLanes = 8, kRankTile = 1024;
 
